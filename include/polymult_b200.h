@@ -49,7 +49,8 @@ enum pm_gemm_form {
 typedef struct pm_info {
     uint32_t N, W, L;
     int32_t K;             /* RNS primes */
-    int32_t logN, w1, w2;  /* 4-step split: nrows = 2^w1, ncols = 2^w2 */
+    int32_t logN, w1, w2;  /* 4-step split: nrows = 2^w1, ncols = 2^w2 (w1 = 4 where the column stages run
+                              inside the GEMM kernels: tensor form, K <= 128, 2^9 <= N <= 2^16) */
     int32_t gemm_form;     /* resolved form: PM_GEMM_PLAIN, PM_GEMM_TENSOR or PM_GEMM_MIXED */
     int32_t device;
     uint64_t delta;        /* 2^W - q */
@@ -74,7 +75,11 @@ int pm_run(pm_context* ctx, const uint32_t* a, const uint32_t* b, uint32_t* c);
 int pm_run_device(pm_context* ctx, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c, uint32_t count,
                   void* stream);
 
-/* Kernels of one device-resident multiply group, in launch order (pm_time_stages). */
+/* Kernels of one device-resident multiply group, in launch order (pm_time_stages).  Where the column
+ * stages run inside the GEMM kernels (pm_info.w1 = 4), PM_STAGE_DEC_A is the one kernel that takes
+ * both operands through decomposition and column pass and PM_STAGE_CRT the inverse column pass and
+ * CRT; PM_STAGE_COLS_A, _DEC_B, _COLS_B and _COLS_INV then read as the bare time between two event
+ * records. */
 #define PM_STAGE_COUNT 8
 enum pm_stage {
     PM_STAGE_DEC_A = 0,    /* RNS decomposition of a */
@@ -153,7 +158,8 @@ typedef struct pm_batch_info {
 } pm_batch_info;
 
 typedef struct pm_batch_class_info {
-    int32_t K, w1, w2;
+    int32_t K, w1, w2;  /* split of separate column and row passes (a class whose column stages run
+                           inside the GEMM kernels: the square split's) */
     int32_t gemm_form;  /* PM_GEMM_PLAIN or PM_GEMM_TENSOR */
     double tuned_ms;    /* measured ms of the chosen configuration; 0 untuned, -1 from the cache */
     int32_t col_tma;    /* 1: column passes by the TMA-pipelined kernel (256-row lines), 0: one tile per CTA */

@@ -16,11 +16,7 @@
 //     them with compile-time indexing.  Between phases the elements are exchanged through
 //     shared memory once (a 256-point row: load -> 4 stages -> exchange -> 4 stages -> store),
 //     where the previous design went through shared memory at every radix-8 pass.
-//
-// Phase k of an NB-bit line covers stage bits NB-1-4k down to b0_k = max(0, NB - 4(k+1));
-// its registers hold index bits [b0_k, b0_k + 4) and the thread's position supplies the
-// rest (low bits below b0_k, high bits above).  The last phase of a line whose length is
-// not a power of 16 re-uses bits [0, 4) and skips the stages an earlier phase has done.
+// The networks and the phase layout are in pm_ntt.cuh.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -29,141 +25,18 @@
 
 #include "pm_async.cuh"
 #include "pm_kernels.cuh"
+#include "pm_ntt.cuh"
 
 namespace pm {
 namespace {
 
-template <int NB>
-struct LineCfg {
-    static constexpr int RB = NB < 4 ? NB : 4;      // index bits held in registers
-    static constexpr int E = 1 << RB;               // elements per thread
-    static constexpr int NPH = RB == 0 ? 0 : (NB + RB - 1) / RB;  // phases (none for a 1-point line)
-    __host__ __device__ static constexpr int b0(int k) { return NB - RB * (k + 1) > 0 ? NB - RB * (k + 1) : 0; }
-    // first local stage of phase k (local stage t pairs register bit RB-1-t)
-    __host__ __device__ static constexpr int t0(int k) { return b0(k) + RB - 1 - (NB - 1 - RB * k); }
-    // global stage index of local stage t of phase k: ls = NB - 1 - (b0 + RB - 1 - t)
-    __host__ __device__ static constexpr int ls(int k, int t) { return NB - b0(k) - RB + t; }
-};
-
-// Forward (CT) radix network on v[] over local stages t0..RB-1 of one phase.  stw(t) returns
-// the stage's twiddle source: w[m] is the Shoup-form Tw2 {w, floor(w 2^32 / p)} of group m
-// (gi = (hi << t) | m; hi is folded in by stw).
-template <int RB, int T0, class StwF>
-__device__ __forceinline__ void radix_fwd(uint32_t (&v)[1 << RB], const StwF& stw, uint32_t p) {
-#pragma unroll
-    for (int t = T0; t < RB; ++t) {
-        const int h = (1 << RB) >> (t + 1);
-        const auto w = stw(t);
-#pragma unroll
-        for (int m = 0; m < (1 << t); ++m) {
-            const Tw2 wm = w[m];
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-                bfly_ct_sh(v[m * 2 * h + i], v[m * 2 * h + i + h], wm, p);
-            }
-        }
-    }
-}
-
-// The forward network on two operands' lines that share their twiddles (the same prime and
-// row): each twiddle is read once for both butterflies.
-template <int RB, int T0, class StwF>
-__device__ __forceinline__ void radix_fwd2(uint32_t (&v)[1 << RB], uint32_t (&u)[1 << RB], const StwF& stw,
-                                           uint32_t p) {
-#pragma unroll
-    for (int t = T0; t < RB; ++t) {
-        const int h = (1 << RB) >> (t + 1);
-        const auto w = stw(t);
-#pragma unroll
-        for (int m = 0; m < (1 << t); ++m) {
-            const Tw2 wm = w[m];
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-                bfly_ct_sh(v[m * 2 * h + i], v[m * 2 * h + i + h], wm, p);
-                bfly_ct_sh(u[m * 2 * h + i], u[m * 2 * h + i + h], wm, p);
-            }
-        }
-    }
-}
-
-// Inverse (GS) network, local stages RB-1 down to T0, mirrored twiddles from stw(t).
-template <int RB, int T0, class StwF>
-__device__ __forceinline__ void radix_inv(uint32_t (&v)[1 << RB], const StwF& stw, uint32_t p) {
-#pragma unroll
-    for (int t = RB - 1; t >= T0; --t) {
-        const int h = (1 << RB) >> (t + 1);
-        const auto w = stw(t);
-#pragma unroll
-        for (int m = 0; m < (1 << t); ++m) {
-            const Tw2 wm = w[m];
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-                bfly_gs_sh(v[m * 2 * h + i], v[m * 2 * h + i + h], wm, p);
-            }
-        }
-    }
-}
-
-// The inverse network on two lines that share their twiddles.
-template <int RB, int T0, class StwF>
-__device__ __forceinline__ void radix_inv2(uint32_t (&v)[1 << RB], uint32_t (&u)[1 << RB], const StwF& stw,
-                                           uint32_t p) {
-#pragma unroll
-    for (int t = RB - 1; t >= T0; --t) {
-        const int h = (1 << RB) >> (t + 1);
-        const auto w = stw(t);
-#pragma unroll
-        for (int m = 0; m < (1 << t); ++m) {
-            const Tw2 wm = w[m];
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-                bfly_gs_sh(v[m * 2 * h + i], v[m * 2 * h + i + h], wm, p);
-                bfly_gs_sh(u[m * 2 * h + i], u[m * 2 * h + i + h], wm, p);
-            }
-        }
-    }
-}
-
-// A stage's run of 2^t consecutive Shoup-form twiddles {w, floor(w 2^32 / p)} starting at
-// `src`, aligned to 2^t entries.  w[m] is entry m (REV: entry 2^t - 1 - m), read at use as
-// half of a 16-byte pair (the two entries of a pair come from one load), so that no more of
-// the run than the current butterflies need is held in registers.
-template <bool REV>
-struct RunTw {
-    const uint2* src;
-    int n;
-    __device__ __forceinline__ Tw2 operator[](int m) const {
-        const int e = REV ? n - 1 - m : m;
-        if (n == 1) {
-            const uint2 u = __ldg(src);
-            return Tw2{u.x, u.y};
-        }
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + (e >> 1));
-        return (e & 1) ? Tw2{u.z, u.w} : Tw2{u.x, u.y};
-    }
-};
-
-// A column stage's run of 2^t Shoup twiddles in shared memory, starting at `start` (aligned to
-// 2^t entries): w[m] is entry m (REV: entry 2^t - 1 - m), read as half of a 16-byte pair.
-template <bool REV>
-struct SmemRun {
-    const Tw2* start;
-    int n;
-    __device__ __forceinline__ Tw2 operator[](int m) const {
-        const int e = REV ? n - 1 - m : m;
-        if (n == 1) return start[0];
-        const uint4 u = reinterpret_cast<const uint4*>(start)[e >> 1];
-        return (e & 1) ? Tw2{u.z, u.w} : Tw2{u.x, u.y};
-    }
-};
-
 // ---------------------------------------------------------------------------------------
 // Row pass layout.  LPR = 2^(NB-RB) threads share a row; a shared-memory region serves
-// GRP = max(32, LPR) threads (one warp, or the two warps of a 1024-point row) and holds
+// GRP = max(32, LPR) threads (one warp, or the 2 to 8 warps of a row of 1024 to 4096 points) and holds
 // RPG = GRP / LPR rows.  Inside a region an element has the index X = (row << NB) | x; it
 // is stored at X ^ G(X >> 5), an XOR swizzle chosen (by exhaustive search over linear maps)
 // so that every exchange of the phase layouts below is free of bank conflicts -- with
-// 16-byte vector access in the last phase for NB = 6, 7, 8.
+// 16-byte vector access in the last phase for NB = 6, 7, 8 and 10, 11, 12.
 // ---------------------------------------------------------------------------------------
 template <int NB>
 struct RowCfg : LineCfg<NB> {
@@ -171,8 +44,9 @@ struct RowCfg : LineCfg<NB> {
     static constexpr int LPR = 1 << (NB - B::RB);
     static constexpr int GRP = LPR > 32 ? LPR : 32;
     static constexpr int RPG = GRP / LPR;             // rows per shared-memory region
-    static constexpr int ROWS_PER_CTA = 128 / LPR;   // 128 threads per CTA
-    static constexpr bool VEC = NB >= 6 && NB <= 8;   // swizzle keeps runs of 4 contiguous
+    static constexpr int THREADS = LPR > 128 ? LPR : 128;  // per CTA
+    static constexpr int ROWS_PER_CTA = THREADS / LPR;
+    static constexpr bool VEC = NB >= 6 && NB != 9;   // swizzle keeps runs of 4 contiguous
     static constexpr int REGION = GRP * B::E;         // words per region
     __host__ __device__ static constexpr uint32_t g(int i) {
         // G(input bit i of X >> 5) for each NB; NB <= 4 has a single phase and no exchange
@@ -180,7 +54,9 @@ struct RowCfg : LineCfg<NB> {
              : NB == 6           ? (i == 0 ? 4u : i == 1 ? 8u : i == 2 ? 4u : i == 3 ? 16u : 0u)
              : NB == 7           ? (i == 0 ? 4u : i == 1 ? 8u : i == 2 ? 8u : i == 3 ? 16u : 0u)
              : NB == 8           ? (i == 0 ? 4u : i == 1 ? 8u : i == 2 ? 0u : i == 3 ? 16u : 0u)
-             : NB == 10          ? (i == 0 ? 1u : i == 1 ? 18u : i == 2 ? 4u : i == 3 ? 8u : 0u)
+             : NB == 10          ? (i == 0 ? 4u : i == 1 ? 8u : i == 2 ? 4u : i == 3 ? 16u : 0u)
+             : NB == 11          ? (i == 0 ? 4u : i == 1 ? 8u : i == 2 ? 8u : i == 3 ? 16u : 0u)
+             : NB == 12          ? (i == 0 ? 4u : i == 1 ? 8u : i == 3 ? 16u : 0u)
                                  : 0u;
     }
     // X ^ G(X >> 5) is linear over XOR: swz(a ^ b) = swz(a) ^ swz(b), so an element's address
@@ -235,8 +111,9 @@ __device__ __forceinline__ void row_xchg(uint32_t (&v)[RowCfg<NB>::E], uint32_t*
     }
 }
 
-// global <-> registers in the layout of phase K (rows of nc consecutive words)
-template <int NB, int K, bool LOAD>
+// global <-> registers in the layout of phase K: rows of consecutive words, or (QUAD) a row of the
+// quad layout, whose element x lies at residue_off(x)
+template <int NB, int K, bool LOAD, bool QUAD>
 __device__ __forceinline__ void row_global(uint32_t (&v)[RowCfg<NB>::E], uint32_t* row, int r, bool active) {
     using C = RowCfg<NB>;
     if (!active) {
@@ -245,34 +122,60 @@ __device__ __forceinline__ void row_global(uint32_t (&v)[RowCfg<NB>::E], uint32_
             for (int e = 0; e < C::E; ++e) v[e] = 0;
         return;
     }
-    if constexpr (C::b0(K) == 0 && C::E >= 4) {  // E consecutive words, 16-byte aligned
-        uint4* g = reinterpret_cast<uint4*>(row + row_x<NB, K>(r, 0));
+    // the register bits of x are zero in the base, and residue_off is additive over disjoint bits
+    const uint32_t x0 = (uint32_t)row_x<NB, K>(r, 0);
+    uint32_t* g0 = row + (QUAD ? residue_off(x0) : x0);
+    if constexpr (C::b0(K) == 0 && C::E >= 4) {  // runs of 4 words (at least), 16-byte aligned
 #pragma unroll
         for (int q = 0; q < C::E / 4; ++q) {
+            uint4* g = reinterpret_cast<uint4*>(g0 + (QUAD ? residue_off(4 * q) : 4 * q));
             if (LOAD) {
-                const uint4 u = g[q];
+                const uint4 u = *g;
                 v[4 * q] = u.x;
                 v[4 * q + 1] = u.y;
                 v[4 * q + 2] = u.z;
                 v[4 * q + 3] = u.w;
             } else {
-                g[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                *g = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
         }
     } else {
 #pragma unroll
         for (int e = 0; e < C::E; ++e) {
-            if (LOAD) v[e] = row[row_x<NB, K>(r, e)];
-            else row[row_x<NB, K>(r, e)] = v[e];
+            constexpr int b0 = C::b0(K);
+            uint32_t* g = g0 + (QUAD ? residue_off((uint32_t)e << b0) : (uint32_t)e << b0);
+            if (LOAD) v[e] = *g;
+            else *g = v[e];
         }
     }
 }
 
+// Last-phase twiddles of a row of the 16-row split, from a copy of the table laid out by thread
+// (build_row_twiddles): a stage's 2^t twiddles of thread r are 16-byte pairs at [pair][r], so that
+// a warp reads consecutive pairs, 4 lines a load -- the table's own runs of 2^t entries per thread
+// take up to 16 lines a load.  w[m]: entry m of thread `r` (REV: 2^t - 1 - m).
+template <int LPR, bool REV>
+struct RowTw {
+    const uint4* base;  // the row's [7][LPR] pairs (stages t = 1, 2, 3), then [LPR] entries of t = 0
+    int r, n;
+    __device__ __forceinline__ Tw2 operator[](int m) const {
+        if (n == 1) {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(base + 7 * LPR) + r);
+            return Tw2{u.x, u.y};
+        }
+        const int e = REV ? n - 1 - m : m;
+        const uint4 u = __ldg(base + (n / 2 - 1 + (e >> 1)) * LPR + r);
+        return (e & 1) ? Tw2{u.z, u.w} : Tw2{u.x, u.y};
+    }
+};
+// uint4 words of a row's table
+__host__ __device__ constexpr int row_tw_stride(int lpr) { return 7 * lpr + lpr / 2; }
+
 // Forward phases K..NPH-1 of a row (registers in the layout of phase K on entry, of phase
 // NPH-1 on exit).  Stage ls of row hi, group gi uses tw[2^(w1+ls) + hi 2^ls + gi].
-template <int NB, int K>
+template <int NB, int K, bool QUAD>
 __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
-                                            const uint2* twj, int w1, uint32_t hi, uint32_t p) {
+                                            const uint2* twj, const uint4* twl, int w1, uint32_t hi, uint32_t p) {
     using C = RowCfg<NB>;
     if constexpr (K < C::NPH) {
         constexpr int b0 = C::b0(K);
@@ -283,23 +186,28 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        radix_fwd<C::RB, C::t0(K)>(v, stw, p);
+        if constexpr (QUAD && K == C::NPH - 1) {
+            auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
+            radix_fwd<C::RB, C::t0(K)>(v, ltw, p);
+        } else {
+            radix_fwd<C::RB, C::t0(K)>(v, stw, p);
+        }
         if constexpr (K + 1 < C::NPH) {
             row_xchg<NB, K, true>(v, region, rho, r);
             region_sync<NB>();
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             region_sync<NB>();
-            row_forward<NB, K + 1>(v, region, rho, r, twj, w1, hi, p);
+            row_forward<NB, K + 1, QUAD>(v, region, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
 
 // row_forward on two operands' rows of the same prime and row index (b in v, a in u), each in
 // its own shared-memory region for the exchanges.
-template <int NB, int K>
+template <int NB, int K, bool QUAD>
 __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint32_t (&u)[RowCfg<NB>::E],
                                              uint32_t* region, uint32_t* region_u, int rho, int r, const uint2* twj,
-                                             int w1, uint32_t hi, uint32_t p) {
+                                             const uint4* twl, int w1, uint32_t hi, uint32_t p) {
     using C = RowCfg<NB>;
     if constexpr (K < C::NPH) {
         constexpr int b0 = C::b0(K);
@@ -308,7 +216,12 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        radix_fwd2<C::RB, C::t0(K)>(v, u, stw, p);
+        if constexpr (QUAD && K == C::NPH - 1) {
+            auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
+            radix_fwd2<C::RB, C::t0(K)>(v, u, ltw, p);
+        } else {
+            radix_fwd2<C::RB, C::t0(K)>(v, u, stw, p);
+        }
         if constexpr (K + 1 < C::NPH) {
             row_xchg<NB, K, true>(v, region, rho, r);
             row_xchg<NB, K, true>(u, region_u, rho, r);
@@ -316,7 +229,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             row_xchg<NB, K + 1, false>(u, region_u, rho, r);
             region_sync<NB>();
-            row_forward2<NB, K + 1>(v, u, region, region_u, rho, r, twj, w1, hi, p);
+            row_forward2<NB, K + 1, QUAD>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
@@ -324,9 +237,9 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
 // Inverse phases K down to 0 (registers in the layout of phase K on entry, phase 0 on exit).
 // The inverse twiddle of (ls, hi, gi) is the forward entry of the mirrored row nrows-1-hi at
 // 2^ls - 1 - gi.
-template <int NB, int K>
+template <int NB, int K, bool QUAD>
 __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
-                                            const uint2* twj, int w1, uint32_t hi_m, uint32_t p) {
+                                            const uint2* twj, const uint4* twl, int w1, uint32_t hi_m, uint32_t p) {
     using C = RowCfg<NB>;
     if constexpr (K >= 0) {
         constexpr int b0 = C::b0(K);
@@ -337,13 +250,20 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<true>{twj + (1u << (w1 + ls)) + (hi_m << ls) + (1u << ls) - ((hip + 1u) << t), 1 << t};
         };
-        radix_inv<C::RB, C::t0(K)>(v, stw, p);
+        if constexpr (QUAD && K == C::NPH - 1) {  // thread LPR - 1 - r's entries of the mirrored row, reversed
+            auto ltw = [&](int t) {
+                return RowTw<C::LPR, true>{twl + (size_t)hi_m * row_tw_stride(C::LPR), C::LPR - 1 - r, 1 << t};
+            };
+            radix_inv<C::RB, C::t0(K)>(v, ltw, p);
+        } else {
+            radix_inv<C::RB, C::t0(K)>(v, stw, p);
+        }
         if constexpr (K > 0) {
             row_xchg<NB, K, true>(v, region, rho, r);
             region_sync<NB>();
             row_xchg<NB, K - 1, false>(v, region, rho, r);
             region_sync<NB>();
-            row_inverse<NB, K - 1>(v, region, rho, r, twj, w1, hi_m, p);
+            row_inverse<NB, K - 1, QUAD>(v, region, rho, r, twj, twl, w1, hi_m, p);
         }
     }
 }
@@ -367,6 +287,8 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
 // fused form (host pipeline, server) keeps a 4-byte stack slot at 7 (8 bytes at 6).
 enum : int { ROWS_FWD = 0, ROWS_FUSED = 1, ROWS_BOTH = 2 };
 __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
+    if (nb == 12) return 3;                      // 256 threads, 80 registers
+    if (nb >= 10) return 6;                      // 80 registers
     return nb >= 9 ? (mode == ROWS_FWD ? 5 : 4) : (mode == ROWS_FWD ? 8 : 7);
 }
 // POLYMULT_ROW_STATIC: the row kernels take the column-stage count w1 (and with it nrows and N)
@@ -377,15 +299,16 @@ __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
 #ifndef POLYMULT_ROW_STATIC
 #define POLYMULT_ROW_STATIC 1
 #endif
-template <int NB, int MODE, int W1>
-__global__ void __launch_bounds__(128, rows_min_blocks(NB, MODE)) k_ntt_rows(DevPlan P, uint32_t* __restrict__ R,
+// QUAD: the residues lie in the quad layout (the 16-row split).
+template <int NB, int MODE, int W1, bool QUAD>
+__global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)) k_ntt_rows(DevPlan P, uint32_t* __restrict__ R,
                                                                            const uint32_t* __restrict__ RA,
                                                                            const uint32_t* __restrict__ ra_sel) {
     using C = RowCfg<NB>;
     const int w1 = W1 >= 0 ? W1 : P.w1;
     const uint32_t nrows = W1 >= 0 ? (1u << (W1 >= 0 ? W1 : 0)) : P.nrows;
     const uint32_t Nn = W1 >= 0 ? (1u << ((W1 >= 0 ? W1 : 0) + NB)) : P.N;  // N <= 2^20
-    constexpr int REGION_WORDS = C::NPH > 1 ? (128 / C::GRP) * C::REGION : 4;  // one operand's regions
+    constexpr int REGION_WORDS = C::NPH > 1 ? (C::THREADS / C::GRP) * C::REGION : 4;  // one operand's regions
     __shared__ __align__(16) uint32_t sh[MODE == ROWS_BOTH ? 2 * REGION_WORDS : REGION_WORDS];
     const int tid = threadIdx.x;
     const int li = tid % C::GRP;                 // thread within the shared-memory region
@@ -410,35 +333,40 @@ __global__ void __launch_bounds__(128, rows_min_blocks(NB, MODE)) k_ntt_rows(Dev
     const bool active = hi < nrows;
     const uint32_t hic = active ? hi : nrows - 1;  // keeps twiddle reads in range
     const uint32_t p = P.p[j], pinv = P.pinv[j];
-    const size_t off = ((size_t)zb * P.K + j) * Nn + (size_t)hic * (1u << NB);
+    auto row_off = [&](uint32_t z) {
+        return QUAD ? residue_base(z, P.KP, j, Nn) + (size_t)hic * (4u << NB)
+                    : ((size_t)z * P.K + j) * Nn + (size_t)hic * (1u << NB);
+    };
+    const size_t off = row_off(zb);
     uint32_t* row = R + off;
     const uint2* twj = P.tw + (size_t)j * Nn;
+    const uint4* twl = QUAD ? P.twl + (size_t)j * nrows * row_tw_stride(C::LPR) : nullptr;
 
     uint32_t v[C::E];
     pdl_trigger();
     pdl_wait();
-    row_global<NB, 0, true>(v, row, r, active);
+    row_global<NB, 0, true, QUAD>(v, row, r, active);
     if constexpr (MODE == ROWS_BOTH) {
         uint32_t a[C::E];
-        row_global<NB, 0, true>(a, const_cast<uint32_t*>(RA + off), r, active);
-        row_forward2<NB, 0>(v, a, region, region + REGION_WORDS, rho, r, twj, w1, hic, p);
+        row_global<NB, 0, true, QUAD>(a, const_cast<uint32_t*>(RA + off), r, active);
+        row_forward2<NB, 0, QUAD>(v, a, region, region + REGION_WORDS, rho, r, twj, twl, w1, hic, p);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1>(v, region, rho, r, twj, w1, nrows - 1 - hic, p);
-        row_global<NB, 0, false>(v, row, r, active);
+        row_inverse<NB, C::NPH - 1, QUAD>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_global<NB, 0, false, QUAD>(v, row, r, active);
     } else if constexpr (MODE == ROWS_FUSED) {
-        row_forward<NB, 0>(v, region, rho, r, twj, w1, hic, p);
+        row_forward<NB, 0, QUAD>(v, region, rho, r, twj, twl, w1, hic, p);
         uint32_t a[C::E];
         const size_t za = ra_sel ? (size_t)__ldg(ra_sel + zb) : (size_t)zb;
-        const size_t offa = (za * P.K + j) * Nn + (size_t)hic * (1u << NB);
-        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true>(a, const_cast<uint32_t*>(RA + offa), r, active);
+        const size_t offa = row_off((uint32_t)za);
+        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true, QUAD>(a, const_cast<uint32_t*>(RA + offa), r, active);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1>(v, region, rho, r, twj, w1, nrows - 1 - hic, p);
-        row_global<NB, 0, false>(v, row, r, active);
+        row_inverse<NB, C::NPH - 1, QUAD>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_global<NB, 0, false, QUAD>(v, row, r, active);
     } else {
-        row_forward<NB, 0>(v, region, rho, r, twj, w1, hic, p);
-        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), false>(v, row, r, active);
+        row_forward<NB, 0, QUAD>(v, region, rho, r, twj, twl, w1, hic, p);
+        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), false, QUAD>(v, row, r, active);
     }
 }
 
@@ -762,6 +690,36 @@ __global__ void __launch_bounds__(ColtCfg<NB>::THREADS, ColtCfg<NB>::MIN_BLOCKS)
     if (threadIdx.x == 0 && *abort_f) flag_error(P.status, DEV_ERR_WAIT);
 }
 
+// Lines of 16 rows: one radix-16 network between registers, two adjacent columns per thread, no
+// shared memory; bound by HBM (10 us against 44 of k_ntt_cols<4> per multiply at N = 65536,
+// W = 1747).  An explicit split of 16 rows, and column chunks narrower than the fused kernels' tiles.
+template <bool INV>
+__global__ void __launch_bounds__(256, 3) k_ntt_cols16(DevPlan P, uint32_t* __restrict__ R, uint32_t col0,
+                                                        uint32_t pairs) {
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = (int)blockIdx.y;
+    const uint32_t p = P.p[j];
+    const uint2* tw = P.tw + (size_t)j * P.N;
+    const size_t step = P.ncols / 2;
+    uint2* g = reinterpret_cast<uint2*>(R + ((size_t)blockIdx.z * P.K + j) * P.N + col0) + x;
+    pdl_trigger();
+    pdl_wait();
+    if (x >= pairs) return;
+    uint32_t v[16], u[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const uint2 w = g[e * step];
+        v[e] = w.x;
+        u[e] = w.y;
+    }
+    // stage t's 2^t twiddles: entries 2^t .. 2^(t+1) - 1, mirrored in the inverse
+    auto stw = [&](int t) { return RunTw<INV>{tw + (1 << t), 1 << t}; };
+    if (!INV) radix_fwd2<4, 0>(v, u, stw, p);
+    else radix_inv2<4, 0>(v, u, stw, p);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) g[e * step] = make_uint2(v[e], u[e]);
+}
+
 template <int NB, bool INV>
 __global__ void __launch_bounds__(256, NB >= 5 ? 4 : 1) k_ntt_cols(DevPlan P, uint32_t* __restrict__ R, uint32_t col0, int ltc) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -781,6 +739,32 @@ __global__ void __launch_bounds__(256, NB >= 5 ? 4 : 1) k_ntt_cols(DevPlan P, ui
     __syncthreads();
     if (ltc == 5) col_phases<NB, INV, 0, 5>(tile, tws, base, P.ncols, ltc, p);  // the common 32-column tile
     else col_phases<NB, INV, 0, -1>(tile, tws, base, P.ncols, ltc, p);
+}
+
+// The rows' last-phase twiddles by thread (RowTw), from the plan's table: thread r of row hi takes
+// entries (r << t) .. (r << t) + 2^t - 1 of the row's part of stage logN - 4 + t.
+__global__ void k_build_row_tw(const uint2* __restrict__ tw, uint2* __restrict__ twl, uint32_t N, int lpr, uint32_t total) {
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;  // (prime, row, thread)
+    if (x >= total) return;
+    const uint32_t r = x % lpr, hi = x / lpr % 16, j = x / lpr / 16;
+    const uint2* src = tw + (size_t)j * N;
+    uint2* dst = twl + (size_t)(x / lpr) * (2 * row_tw_stride(lpr));
+    for (int t = 0; t < 4; ++t)
+        for (int m = 0; m < (1 << t); ++m) {
+            const uint2 w = src[(N >> (4 - t)) + ((hi * lpr) << t) + (r << t) + m];
+            if (t == 0) dst[14 * lpr + r] = w;
+            else dst[2 * (((1 << (t - 1)) - 1 + (m >> 1)) * lpr + r) + (m & 1)] = w;
+        }
+}
+
+size_t row_tw_words(const DevPlan& P) { return P.w2 >= 5 ? (size_t)P.K * 16 * row_tw_stride(1 << (P.w2 - 4)) : 0; }
+
+void build_row_twiddles(const DevPlan& P, uint4* twl, cudaStream_t s) {
+    const int lpr = 1 << (P.w2 - 4);
+    const uint32_t total = (uint32_t)P.K * 16 * lpr;
+    const cudaError_t e = launch_kernel(k_build_row_tw, dim3((total + 255) / 256), dim3(256), 0, s, false, P.tw,
+                                        reinterpret_cast<uint2*>(twl), P.N, lpr, total);
+    if (e != cudaSuccess) throw_cuda(e, "launch k_build_row_tw");
 }
 
 namespace {
@@ -875,6 +859,14 @@ template <int NB>
 void launch_cols_nb(bool inv, dim3 grid, size_t smem, cudaStream_t s, const DevPlan& P, uint32_t* R, uint32_t col0,
                     int ltc, bool pdl) {
     if (launch_cols_tma<NB>(inv, grid, s, P, R, col0, ltc, pdl)) return;
+    if (NB == 4 && ltc >= 1) {
+        const uint32_t pairs = (grid.x << ltc) / 2;
+        const cudaError_t e = launch_kernel(inv ? k_ntt_cols16<true> : k_ntt_cols16<false>,
+                                            dim3((pairs + 255) / 256, grid.y, grid.z), dim3(256), 0, s, pdl, P, R, col0,
+                                            pairs);
+        if (e != cudaSuccess) throw_cuda(e, inv ? "launch k_ntt_cols16<inverse>" : "launch k_ntt_cols16<forward>");
+        return;
+    }
     if (POLYMULT_COL2 && NB >= 7 && NB <= 8 && ltc >= 6) {
         // 2^ltc columns as 2^(ltc - 6) tiles of 64
         const dim3 g2(grid.x << (ltc - 6), grid.y, grid.z);
@@ -892,31 +884,45 @@ void launch_cols_nb(bool inv, dim3 grid, size_t smem, cudaStream_t s, const DevP
 // the row kernel of a mode for line length 2^NB and the plan's w1: a compile-time w1 for the
 // splits of N = 4096 .. 65536 that the batches and the engine use, else w1 from the plan
 template <int NB, int MODE>
-auto row_kernel(int w1) {
+auto row_kernel(int w1, bool quad) {
+    if constexpr (NB >= 5) {
+        if (quad) return k_ntt_rows<NB, MODE, 4, true>;  // the 16-row split
+    }
+    (void)quad;
     if constexpr (POLYMULT_ROW_STATIC && NB >= 6 && NB <= 8) {
-        if (w1 == NB) return k_ntt_rows<NB, MODE, NB>;
-        if (w1 == NB - 1) return k_ntt_rows<NB, MODE, NB - 1>;
+        if (w1 == NB) return k_ntt_rows<NB, MODE, NB, false>;
+        if (w1 == NB - 1) return k_ntt_rows<NB, MODE, NB - 1, false>;
     }
     (void)w1;
-    return k_ntt_rows<NB, MODE, -1>;
+    return k_ntt_rows<NB, MODE, -1, false>;
 }
 
 template <int NB>
 void launch_rows_nb(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                    const uint32_t* ra_sel, bool pdl) {
+                    const uint32_t* ra_sel, bool pdl, bool quad) {
     // grid comes as (row blocks, primes, batch); the static form takes it as (batch, row blocks, primes)
     const dim3 g = POLYMULT_ROW_STATIC ? dim3(grid.z, grid.x, grid.y) : grid;
-    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P.w1)
-                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P.w1)
-                                                             : row_kernel<NB, ROWS_FWD>(P.w1),
-                                        g, dim3(128), 0, s, pdl, P, R, RA, ra_sel);
+    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P.w1, quad)
+                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P.w1, quad)
+                                                             : row_kernel<NB, ROWS_FWD>(P.w1, quad),
+                                        g, dim3(RowCfg<NB>::THREADS), 0, s, pdl, P, R, RA, ra_sel);
     if (e != cudaSuccess)
         throw_cuda(e, mode == ROWS_BOTH    ? "launch k_ntt_rows<both operands>"
                       : mode == ROWS_FUSED ? "launch k_ntt_rows<fused>"
                                            : "launch k_ntt_rows<forward>");
 }
 
-// Applies F<NB>::run(...) for the line length 2^nb, nb in [0, 10].
+// Applies F<NB>::run(...) for the line length 2^nb: nb in [0, 10] for columns, [0, 12] for rows.
+template <template <int> class F, class... A>
+void dispatch_nb(int nb, A&&... a);
+template <template <int> class F, class... A>
+void dispatch_rows(int nb, A&&... a) {
+    switch (nb) {
+        case 11: F<11>::run(a...); break;
+        case 12: F<12>::run(a...); break;
+        default: dispatch_nb<F>(nb, a...);
+    }
+}
 template <template <int> class F, class... A>
 void dispatch_nb(int nb, A&&... a) {
     switch (nb) {
@@ -995,8 +1001,9 @@ struct ColProbeF {
 template <int NB>
 struct RowProbeF {
     static void run() {
-        const void* fns[3] = {(const void*)k_ntt_rows<NB, ROWS_FWD, -1>, (const void*)k_ntt_rows<NB, ROWS_FUSED, -1>,
-                              (const void*)k_ntt_rows<NB, ROWS_BOTH, -1>};
+        const void* fns[3] = {(const void*)k_ntt_rows<NB, ROWS_FWD, -1, false>,
+                              (const void*)k_ntt_rows<NB, ROWS_FUSED, -1, false>,
+                              (const void*)k_ntt_rows<NB, ROWS_BOTH, -1, false>};
         for (const void* f : fns) {
             cudaFuncAttributes fa{};
             const cudaError_t e = cudaFuncGetAttributes(&fa, f);
@@ -1017,13 +1024,13 @@ void launch_ntt_cols(bool inv, dim3 grid, size_t smem, cudaStream_t s, const Dev
 }
 
 void launch_ntt_rows(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                     const uint32_t* ra_sel, bool pdl) {
-    dispatch_nb<RowsF>(P.w2, mode, grid, s, P, R, RA, ra_sel, pdl);
+                     const uint32_t* ra_sel, bool pdl, bool quad) {
+    dispatch_rows<RowsF>(P.w2, mode, grid, s, P, R, RA, ra_sel, pdl, quad);
 }
 
 int ntt_rows_per_cta(int w2) {
     int r = 0;
-    dispatch_nb<RowsPerCtaF>(w2, &r);
+    dispatch_rows<RowsPerCtaF>(w2, &r);
     return r;
 }
 
@@ -1034,7 +1041,7 @@ void ntt_set_smem_limit(int bytes, int w1, int w2) {
 
 void ntt_probe_images(int w1, int w2) {
     if (w1 > 0) dispatch_nb<ColProbeF>(w1, w2);
-    dispatch_nb<RowProbeF>(w2);
+    dispatch_rows<RowProbeF>(w2);
 }
 
 size_t ntt_cols_smem(const DevPlan& P, int ltc) {

@@ -16,8 +16,8 @@
 //     captured once into a CUDA graph and replayed by pm_batch_run with one launch call;
 //   * residue scratch is allocated once at init: per stream, the largest class on it (the
 //     classes of one stream run one after the other and reuse it).
-// The autotuner (PM_BATCH_TUNE) times, per class, every split w1 in logN/2 - 1 .. logN/2 + 1
-// that the kernels support and both GEMM forms (where the tensor-core form fits) on the
+// The autotuner (PM_BATCH_TUNE) times, per class, the fused 16-row form (where it applies), every
+// split w1 in logN/2 - 1 .. logN/2 + 1 that the kernels support and both GEMM forms (where the tensor-core form fits) on the
 // class's own operands, CUDA events around 3 repetitions after a warm-up, and keeps the
 // fastest; then, on that engine, the column-pass kernel (TMA pipeline / one tile per CTA), the
 // CRT GEMM's A placement (tensor / shared memory) and 1, 2 or 4 launch groups per class.
@@ -53,7 +53,8 @@ std::string cache_path() {
     return std::string(home ? home : "/tmp") + "/.cache/polymult_b200/tune.txt";
 }
 
-// The tuner's choice for one class.  col_tma / crt_tm: -1 = the engine's default.
+// The tuner's choice for one class.  w1 -1: the fused 16-row split; col_tma / crt_tm -1: the
+// engine's default.
 struct Choice {
     int gemm = 0, w1 = 0;
     int col_tma = -1, crt_tm = -1;
@@ -201,6 +202,8 @@ void Batch::choose_configs(int gemm_request) {
             const int forms[2] = {GEMM_AUTO, GEMM_PLAIN};
             for (int f : forms) {
                 if (gemm_request != GEMM_AUTO && f != gemm_request) continue;
+                // (-1: the engine's own choice, the fused 16-row split where it applies)
+                if (f == GEMM_AUTO) cand.push_back({f, -1});
                 for (int w1 = logN / 2 - 1; w1 <= logN / 2 + 1; ++w1)
                     if (w1 >= 0 && w1 <= 10 && logN - w1 >= (logN > 0 ? 1 : 0) && logN - w1 <= 10)
                         cand.push_back({f, w1});
@@ -214,13 +217,14 @@ void Batch::choose_configs(int gemm_request) {
                     EngineOptions o = opt;
                     o.w1 = w1;
                     e.reset(new Engine(s.N, s.W, s.L, s.q, f, device_, o));
+                    if (w1 < 0 && !e->fused()) continue;  // then it is the square split, a candidate below
                 } catch (const Unsupported&) {
                     continue;  // this form / split does not fit the point
                 } catch (const InvalidPoint&) {
                     continue;
                 }
                 e->reserve((size_t)s.count * e->plan().N);
-                const size_t words = (size_t)s.count * e->plan().K * e->plan().N;
+                const size_t words = (size_t)s.count * e->residue_words();
                 if (probe) cudaFree(probe);
                 probe = nullptr;
                 cuda_check(cudaMalloc(&probe, 2 * words * 4), "cudaMalloc tuning scratch");
@@ -246,7 +250,7 @@ void Batch::choose_configs(int gemm_request) {
             std::vector<int> cols{ch.col_tma}, crts{ch.crt_tm};
             if (e.col_tma_applies()) cols.push_back(1 - ch.col_tma);
             if (e.crt_tm_applies()) crts.push_back(1 - ch.crt_tm);
-            const size_t words = (size_t)s.count * e.plan().K * e.plan().N;
+            const size_t words = (size_t)s.count * e.residue_words();
             for (uint32_t g : {1u, 2u, 4u}) {
                 if (g > s.count) break;
                 e.reserve((size_t)per_group(s.count, g) * e.plan().N);
@@ -338,8 +342,7 @@ void Batch::alloc_scratch() {
         const size_t s = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
         load[s] += work(i);
         sched_[s].push_back(i);
-        const Plan& P = cls_[i].eng->plan();
-        need[s] = std::max(need[s], (size_t)per_group(cls_[i].src.count, cls_[i].groups) * P.K * P.N);
+        need[s] = std::max(need[s], (size_t)per_group(cls_[i].src.count, cls_[i].groups) * cls_[i].eng->residue_words());
     }
     streams_.assign(ns, nullptr);
     scratch_.assign(ns, nullptr);

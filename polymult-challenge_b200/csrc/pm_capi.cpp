@@ -204,7 +204,9 @@ int pm_set_pipeline(pm_context* ctx, int flags, int32_t in_body, int32_t out_bod
     if (flags & ~PM_PIPELINE_PINNED) return fail(PM_ERR_INVALID, "unknown pipeline flags");
     if (in_body <= 0 || out_body <= 0) return fail(PM_ERR_INVALID, "chunk divisors must be positive");
     const int kind = (flags & PM_PIPELINE_PINNED) ? 1 : 0;
-    const uint32_t nc = ctx->engine->plan().ncols;
+    // (the columns of the square split, whatever split the engine runs)
+    const pm::Plan& P = ctx->engine->plan();
+    const uint32_t nc = P.N >> (P.logN / 2);
     if ((uint32_t)in_body > nc || (uint32_t)out_body > nc) return fail(PM_ERR_INVALID, "chunk divisor above ncols");
     return guarded([&] {
         ctx->engine->set_chunk_schedule((uint32_t)in_body, (uint32_t)out_body, kind);
@@ -259,8 +261,8 @@ int pm_batch_get_class(const pm_batch* batch, uint32_t index, pm_batch_class_inf
     const pm::Engine& e = b.engine(index);
     std::memset(out, 0, sizeof *out);
     out->K = e.plan().K;
-    out->w1 = e.plan().w1;
-    out->w2 = e.plan().w2;
+    out->w1 = e.split_w1();
+    out->w2 = e.plan().logN - e.split_w1();
     out->gemm_form = e.gemm_form();
     out->tuned_ms = b.tuned_ms(index);
     out->col_tma = e.col_tma() && e.col_tma_applies() ? 1 : 0;

@@ -9,7 +9,7 @@
 // z + delta reaches 2^W, and then z - q = (z + delta) mod 2^W: so the last step adds delta and
 // keeps the sum (minus 2^W) when bit W is set, else takes delta back off.  There is no
 // data-dependent loop count (only carry ripples past the fourth limb, which almost never run);
-// bits beyond the bound flag DEV_ERR_FOLD.
+// bits beyond the bound flag DEV_ERR_FOLD.  Params: W, delta, fold_count and status of the point.
 #pragma once
 
 #include "pm_device.cuh"
@@ -46,7 +46,8 @@ __device__ __forceinline__ uint32_t crt_sub64(uint32_t* z, uint64_t v) {
     return b & 1u;
 }
 
-__device__ __forceinline__ void crt_reduce_mod_q(uint32_t* z, int zl, const DevPlan& P) {
+template <class Params>
+__device__ __forceinline__ void crt_reduce_mod_q(uint32_t* z, int zl, const Params& P) {
     const int wl = P.W >> 5, wb = P.W & 31;
     const uint32_t keep = wb ? (1u << wb) - 1u : 0u;  // bits of limb wl below bit W
     // bits from W + 64 up lie outside every bound the host derived

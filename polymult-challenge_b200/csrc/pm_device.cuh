@@ -36,6 +36,7 @@ struct DevPlan {
     const uint32_t* crt_cc;   // [KP]
     const float* rcp;         // [KP]
     const uint2* tw;          // [K][N] {psi^bitrev(k), floor(psi^bitrev(k) 2^32 / p)} (Shoup form)
+    const uint4* twl;         // the 16-row split's last row stages in thread order (RowTw, k_ntt.cu)
     const uint32_t* dec24;    // [DP][KP] 2^(24 d) R mod p_j
     const uint32_t* crt24;    // [K+1][DP] 24-bit digits of Q_j = (M/p_j) mod q; row K: of T_1
     const uint32_t* t1;       // [L] T_1 = (-M) mod q
@@ -69,6 +70,18 @@ struct CrtPrimeBlocks {
     int j0[MAX], k[MAX], kp[MAX], kb[MAX];
     const unsigned char* b[MAX];
 };
+
+// Quad layout of the residue arrays, used by the 16-row split: four primes share 128-byte lines,
+//   word (j, n) of a batch entry = (j / 4) 4N + (n / 8) 32 + (j % 4) 8 + n % 8,
+// KP primes' room per entry.  A kernel that holds a prime per lane (8 columns of one row each)
+// moves whole lines, 8 a warp instead of 32; a row kernel, one prime a block, moves whole
+// sectors of lines that its three neighbour blocks share.
+// Word of (prime j, coefficient 0) of batch entry b:
+__device__ __forceinline__ size_t residue_base(uint32_t b, int KP, int j, size_t N) {
+    return ((size_t)b * KP + (j & ~3)) * N + (size_t)(j & 3) * 8;
+}
+// offset of coefficient n (a multiple of 8, or within its 8) from there; additive over disjoint bits
+__host__ __device__ constexpr uint32_t residue_off(uint32_t n) { return ((n >> 3) << 5) | (n & 7u); }
 
 __device__ __forceinline__ uint32_t chunk_pos_to_n(const DevPlan& P, const ChunkMap& C, uint32_t pos) {
     return ((pos >> C.lcw) << P.w2) + C.col0 + (pos & (C.cw - 1));

@@ -172,6 +172,13 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
                                             std::to_string(prop.major * 10 + prop.minor));
     num_sms_ = prop.multiProcessorCount;
     smem_optin_ = prop.sharedMemPerBlockOptin;
+    // The 16-row split where both of its GEMM kernels take the point; else the square one.  Points
+    // of more than 128 primes keep the square split: a 4096-point row pass costs them more (92
+    // against 55 us a multiply at N = 65536, W = 3000) than the decomposition in prime blocks saves
+    // by taking the column pass along (137 against 139 us).
+    const bool try16 = opt.w1 < 0 && (gemm_request == GEMM_AUTO || gemm_request == GEMM_TENSOR) && plan_.logN >= 9 &&
+                       plan_.logN <= 16 && dec16_shape(dec16_) && crt16_shape(crt16_);
+    if (try16) set_split16(plan_);
     try {
         upload_tables();
         setup_launch_shapes();
@@ -201,6 +208,7 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
         crt_tm_ok_ = crt_tc_ && plan_.KP <= 128 && dp_.crt_nrows <= 256 && dp_.crt_kbytes <= 512 &&
                      crt_tm_smem(dp_) <= smem_optin_;
         crt_tm_ = POLYMULT_CRT_TM && crt_tm_ok_;
+        if (try16) make_fused();
         // multiplies per launch group of run_device: up to POLYMULT_GROUP_WORDS residue words
         // per operand (default 256 Mi: 32 multiplies at N = 65536, W = 1747, 2 GB of residue
         // scratch), at most 256.  Measured there: 8 per group 9081 mults/s, 16 9435, 32 9646 --
@@ -344,6 +352,8 @@ void Engine::setup_launch_shapes() {
         cuda_check(cudaFuncGetAttributes(&fa, pr.fn), (std::string("kernel image ") + pr.name).c_str());
     }
     ntt_set_smem_limit(mx, plan_.w1, plan_.w2);
+    dec16_set_smem_limit(mx);
+    crt16_set_smem_limit(mx);
     cuda_check(cudaFuncSetAttribute(k_rns_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, mx), "smem attr");
     cuda_check(cudaFuncSetAttribute(k_crt_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, mx), "smem attr");
     cuda_check(cudaFuncSetAttribute(k_rns_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, mx), "smem attr");
@@ -384,7 +394,7 @@ void Engine::ensure_scratch(uint32_t group) {
     d_ra_ = d_rb_ = nullptr;
     group_ = 0;
     scratch_words_ = 0;
-    const size_t words = (size_t)group * plan_.K * plan_.N;
+    const size_t words = (size_t)group * residue_words();
     cuda_check(scratch_malloc(reinterpret_cast<void**>(&d_ra_), words * 4), "cudaMalloc residues");
     const cudaError_t e = scratch_malloc(reinterpret_cast<void**>(&d_rb_), words * 4);
     if (e != cudaSuccess) {
@@ -595,6 +605,85 @@ bool Engine::make_dec_blocks() {
     return true;
 }
 
+// Shape of the fused decomposition: at most 128 primes (TMEM lanes), their constant image beside
+// the operand tile and at least two raw pieces; two operand buffers and pieces of 8 rows where
+// they fit.  False where none fits.
+bool Engine::dec16_shape(Dec16Args& A) const {
+    const int K = plan_.K, L = (int)plan_.L;
+    if (K > 128 || L > 64) return false;  // L: t0 of dec_reduce stays below 2^32
+    A = Dec16Args{};
+    A.kb = plan_.dec_gemm.k_bytes;
+    A.L = L;
+    A.K = K;
+    A.KP = plan_.KP;
+    A.q = K <= 32 ? 4 : K <= 64 ? 2 : 1;
+    A.a_zero = 128 - 128 / A.q;
+    A.a_rows = A.q > 1 ? A.a_zero + 128 : (K + 7) / 8 * 8;
+    A.a_bytes = (uint32_t)(4 * A.a_rows * A.kb);
+    // pitch of a row segment: 4 words past a multiple of 32, so that the same limb of 8 rows falls
+    // on different banks
+    A.segw = 8 * L + ((4 - 8 * L) & 31);
+    for (A.nb_buf = 2; A.nb_buf >= 1; --A.nb_buf)
+        for (A.rp = 8; A.rp >= 2; A.rp /= 2)
+            for (A.ring = DEC16_MAX_RING; A.ring >= 2; --A.ring)
+                if (dec16_smem(A) <= smem_optin_) return true;
+    return false;
+}
+
+// Column chunks that the fused kernels take: whole 8-column tiles.
+bool Engine::quad_chunks(const std::vector<Chunk>& v) const {
+    for (const Chunk& c : v)
+        if (c.cw % 8 || c.col0 % 8) return false;
+    return true;
+}
+
+void Engine::make_fused() {
+    Dec16Args& D = dec16_;
+    for (int g = 0; g < 2; ++g)
+        D.img[g] = dev_upload(dev_allocs_, dec16_image(plan_, D.a_rows, D.a_zero, g == 1), &table_bytes_);
+    std::vector<uint32_t> wsh(plan_.KP);
+    for (int j = 0; j < plan_.KP; ++j) wsh[j] = (uint32_t)((1ull << 48) / plan_.p[j]);
+    D.wsh = dev_upload(dev_allocs_, wsh, &table_bytes_);
+    D.p = dp_.p;
+    D.tw16 = reinterpret_cast<const uint2*>(dev_upload(dev_allocs_, tw16_table(plan_), &table_bytes_));
+    D.N = plan_.N;
+    D.status = dp_.status;
+    D.wait_clocks = dp_.wait_clocks;
+    smem_dec16_ = dec16_smem(D);
+    Crt16Args& C = crt16_;
+    C.img = dev_upload(dev_allocs_, crt16_image(plan_, C.nz, C.nrows, C.kb), &table_bytes_);
+    C.N = plan_.N;
+    C.fold_count = plan_.fold_count;
+    C.delta = plan_.delta;
+    C.p = dp_.p;
+    C.t1 = dp_.t1;
+    C.tw16 = D.tw16;
+    C.status = dp_.status;
+    C.wait_clocks = dp_.wait_clocks;
+    uint4* twl = dev_alloc<uint4>(dev_allocs_, row_tw_words(dp_), &table_bytes_);
+    build_row_twiddles(dp_, twl, nullptr);
+    cuda_check(cudaStreamSynchronize(nullptr), "row twiddles");
+    dp_.twl = twl;
+    fused_ = true;
+}
+
+// Shape of the fused CRT: every prime in one tile, the result bytes and the quotient's 6 in at most
+// 256 MMA columns, primes above 2^29 (the quotient constants' 3 bytes), everything in shared memory.
+bool Engine::crt16_shape(Crt16Args& A) const {
+    A = Crt16Args{};
+    A.L = (int)plan_.L;
+    A.W = (int)plan_.W;
+    A.K = plan_.K;
+    A.KP = plan_.KP;
+    A.nz = 4 * A.L + 4;
+    A.nrows = (A.nz + 6 + 15) / 16 * 16;
+    A.kb = (4 * plan_.KP + 31) / 32 * 32;
+    if (plan_.KP > 128 || A.nrows > 256 || crt16_smem(A) > smem_optin_) return false;
+    for (int j = 0; j < plan_.K; ++j)
+        if (plan_.p[j] <= (1u << 29)) return false;
+    return true;
+}
+
 // Blocks of a CRT whose primes do not fit one tile: prime blocks of the largest multiple of 4
 // (at most 128) and result-byte blocks of at most 256 bytes (TMEM columns) such that the
 // partial-mode kernel fits shared memory.  Each block gets its own B image -- rows v0.. of the
@@ -767,6 +856,7 @@ int Engine::kernel_launches_per_group() const {
     const int crt = !crt_blocked_ || crt_wide_ok_
                         ? 1
                         : (int)(crt_byte_launches_.empty() ? crt_blocks_.size() : crt_byte_launches_.size()) + 1;
+    if (fused_) return 3;
     // column passes of a, b and the inverse, and one row pass for both operands
     return 2 * dec + crt + (plan_.w1 > 0 ? 4 : 1);
 }
@@ -819,15 +909,25 @@ void Engine::launch_cols(bool inv, uint32_t* R, Chunk ch, uint32_t nb, cudaStrea
     launch_ntt_cols(inv, grid, smem, s, dp_, R, ch.col0, ltc, pdl);
 }
 
-void Engine::launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s,
-                         const uint32_t* ra_sel, bool pdl) const {
-    dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl);
+// Whether a row pass behind k_dec16 takes the programmatic launch.  Its blocks then start on SMs
+// still set up for k_dec16's 200 KB of shared memory and keep running with the little L1 that
+// leaves (the twiddles live there); after an ordinary launch the SMs are set up for the row pass.
+// Overlap wins while the pass is about three rounds of blocks (N = 32768, W = 868: 45.3 against
+// 47.4 us a multiply), the larger L1 beyond (N = 65536, W = 1747: 124 against 132 us alone, 103
+// against 116 us in launches of 32).
+bool Engine::rows_overlap(uint32_t nb) const {
+    return (uint64_t)nb * plan_.K * plan_.N / 16 <= 3ull * 896 * (uint64_t)num_sms_;
 }
 
-void Engine::launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl) const {
+void Engine::launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s,
+                         const uint32_t* ra_sel, bool pdl, bool quad) const {
     dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl);
+    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl && (!quad || rows_overlap(nb)), quad);
+}
+
+void Engine::launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool quad) const {
+    dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
+    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl && (!quad || rows_overlap(nb)), quad);
 }
 
 void Engine::launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff,
@@ -890,6 +990,70 @@ void Engine::launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out,
     }
 }
 
+void Engine::launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl) const {
+    A.col0 = ch.col0;
+    A.cw = ch.cw;
+    A.nbatch = nb;
+    A.use_bulk = 1;
+    for (uint32_t o = 0; o < A.nops; ++o)
+        if ((uintptr_t)A.src[o] % 16 != 0) A.use_bulk = 0;
+    const uint32_t tiles = ch.cw / 8 * nb, sms = (uint32_t)num_sms_;
+    // as many tiles per accumulator as the image has lane groups, as long as every SM has work
+    A.qrun = A.q;
+    while (A.qrun > 1 && A.nops * ((tiles + A.qrun - 1) / A.qrun) < sms) A.qrun /= 2;
+    const uint32_t supers = (tiles + A.qrun - 1) / A.qrun;
+    launch_dec16(A, std::min(sms, A.nops * supers), smem_dec16_, s, pdl);
+}
+
+void Engine::launch_fwd(const uint32_t* src, Chunk ch, uint32_t nb, uint32_t* R, cudaStream_t s, bool ra, bool pdl,
+                        bool quad) const {
+    if (quad) {
+        Dec16Args A = dec16_;
+        A.nops = 1;
+        A.src[0] = src;
+        A.R[0] = R;
+        A.ra_op = ra ? 0 : 1;
+        launch_dec16_ops(A, ch, nb, s, pdl);
+        return;
+    }
+    launch_dec(src, ch, nb, R, s, ra, pdl);
+    launch_cols(false, R, ch, nb, s, true);
+}
+
+void Engine::launch_fwd2(const uint32_t* a, const uint32_t* b, uint32_t nb, uint32_t* RA, uint32_t* RB, cudaStream_t s,
+                         bool pdl) const {
+    const Chunk all{0, plan_.ncols};
+    if (fused()) {
+        Dec16Args A = dec16_;
+        A.nops = 2;
+        A.src[0] = a;
+        A.src[1] = b;
+        A.R[0] = RA;
+        A.R[1] = RB;
+        A.ra_op = 0;
+        launch_dec16_ops(A, all, nb, s, pdl);
+        return;
+    }
+    launch_fwd(a, all, nb, RA, s, true, pdl, false);
+    launch_fwd(b, all, nb, RB, s, false, true, false);
+}
+
+void Engine::launch_inv(uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff, bool pdl,
+                        bool quad) const {
+    if (quad) {
+        Crt16Args A = crt16_;
+        A.R = R;
+        A.out = out;
+        A.col0 = ch.col0;
+        A.cw = ch.cw;
+        A.nbatch = nb;
+        launch_crt16(A, std::min<uint32_t>(ch.cw / 8 * nb, (uint32_t)num_sms_), s, pdl);
+        return;
+    }
+    launch_cols(true, R, ch, nb, s, pdl);
+    launch_crt(R, ch, nb, out, s, poff, true);
+}
+
 // ---------------------------------------------------------------------------------------
 // device-resident multiply
 // ---------------------------------------------------------------------------------------
@@ -905,13 +1069,9 @@ void Engine::run_device(const uint32_t* a, const uint32_t* b, uint32_t* c, uint3
         const uint32_t* ai = a + (size_t)i * cw;
         const uint32_t* bi = b + (size_t)i * cw;
         // every launch but the call's first follows a kernel of this sequence
-        launch_dec(ai, all, nb, d_ra_, s, true, i > 0);
-        launch_cols(false, d_ra_, all, nb, s, true);
-        launch_dec(bi, all, nb, d_rb_, s, false, true);
-        launch_cols(false, d_rb_, all, nb, s, true);
-        launch_rows_both(d_rb_, d_ra_, nb, s, true);
-        launch_cols(true, d_rb_, all, nb, s, true);
-        launch_crt(d_rb_, all, nb, c + (size_t)i * cw, s, 0, true);
+        launch_fwd2(ai, bi, nb, d_ra_, d_rb_, s, i > 0);
+        launch_rows_both(d_rb_, d_ra_, nb, s, true, fused());
+        launch_inv(d_rb_, all, nb, c + (size_t)i * cw, s, 0, true, fused());
     }
     cuda_check(cudaGetLastError(), "kernel launch");
 }
@@ -932,20 +1092,26 @@ void Engine::time_stages(const uint32_t* a, const uint32_t* b, uint32_t* c, uint
             // the sequence of run_device; stage 2 (a's own row pass) is empty, as the row pass
             // of stage 5 transforms both operands' rows
             cuda_check(cudaEventRecord(ev[0], s), "record");
-            launch_dec(a, all, count, d_ra_, s, true);
+            // one kernel for both operands' decompositions and column passes: stages 1, 3 and 4 are
+            // then the bare time between two event records, as is the inverse column pass inside
+            // the fused CRT
+            const bool f = fused();
+            if (f) launch_fwd2(a, b, count, d_ra_, d_rb_, s, false);
+            else launch_dec(a, all, count, d_ra_, s, true);
             cuda_check(cudaEventRecord(ev[1], s), "record");
-            launch_cols(false, d_ra_, all, count, s);
+            if (!f) launch_cols(false, d_ra_, all, count, s);
             cuda_check(cudaEventRecord(ev[2], s), "record");
             cuda_check(cudaEventRecord(ev[3], s), "record");
-            launch_dec(b, all, count, d_rb_, s);
+            if (!f) launch_dec(b, all, count, d_rb_, s);
             cuda_check(cudaEventRecord(ev[4], s), "record");
-            launch_cols(false, d_rb_, all, count, s);
+            if (!f) launch_cols(false, d_rb_, all, count, s);
             cuda_check(cudaEventRecord(ev[5], s), "record");
-            launch_rows_both(d_rb_, d_ra_, count, s);
+            launch_rows_both(d_rb_, d_ra_, count, s, false, f);
             cuda_check(cudaEventRecord(ev[6], s), "record");
-            launch_cols(true, d_rb_, all, count, s);
+            if (!f) launch_cols(true, d_rb_, all, count, s);
             cuda_check(cudaEventRecord(ev[7], s), "record");
-            launch_crt(d_rb_, all, count, c, s);
+            if (f) launch_inv(d_rb_, all, count, c, s, 0, false, true);
+            else launch_crt(d_rb_, all, count, c, s);
             cuda_check(cudaEventRecord(ev[8], s), "record");
             cuda_check(cudaGetLastError(), "kernel launch");
             cuda_check(cudaEventSynchronize(ev[S]), "sync");
@@ -975,13 +1141,9 @@ void Engine::run_group(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32
                        cudaStream_t s) const {
     if (nb == 0) return;
     const Chunk all{0, plan_.ncols};
-    launch_dec(a, all, nb, ra, s, true);
-    launch_cols(false, ra, all, nb, s, true);
-    launch_dec(b, all, nb, rb, s, false, true);
-    launch_cols(false, rb, all, nb, s, true);
-    launch_rows_both(rb, ra, nb, s, true);
-    launch_cols(true, rb, all, nb, s, true);
-    launch_crt(rb, all, nb, c, s, 0, true);
+    launch_fwd2(a, b, nb, ra, rb, s, false);
+    launch_rows_both(rb, ra, nb, s, true, fused());
+    launch_inv(rb, all, nb, c, s, 0, true, fused());
     cuda_check(cudaGetLastError(), "kernel launch");
 }
 
@@ -1042,6 +1204,9 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     const int kind = direct_in[0] && direct_in[1] && direct_out ? 1 : 0;
     const std::vector<Chunk>& cout = cout_[kind];
     const size_t nout = cout.size();
+    // the fused kernels work on whole 8-column tiles: a schedule with narrower chunks runs the
+    // decomposition, the column passes and the CRT as kernels of their own
+    const bool quad = fused() && quad_chunks(cin_[kind]) && quad_chunks(cout);
     // input items (operand, column chunk): both operands in the schedule's input chunks; with
     // direct copies a moves in one piece (each copy costs a few microseconds of DMA set-up, and
     // a's transform is hidden under b's transfer anyway) and only b is chunked
@@ -1124,15 +1289,14 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         if (last)
             for (int q = na; q < k; ++q) cuda_check(cudaStreamWaitEvent(sc, ev_done_in_[q], 0), "wait");
         cuda_check(cudaStreamWaitEvent(sc, ev_in_[hi], 0), "wait");
-        launch_dec(d_in_[P] + off, ch, 1, dR[P], sc, P == 0);
-        launch_cols(false, dR[P], ch, 1, sc, true);
+        launch_fwd(d_in_[P] + off, ch, 1, dR[P], sc, P == 0, false, quad);
         if (!last) {
             cuda_check(cudaEventRecord(ev_done_in_[k], sc), "record");
             mark("in" + std::to_string(k), sc);
         }
         if (k == na - 1) {  // a complete: its row pass overlaps b's transfer
             for (int q = 0; q < na; ++q) cuda_check(cudaStreamWaitEvent(s_comp_[0], ev_done_in_[q], 0), "wait");
-            launch_rows(false, d_ra_, nullptr, 1, s_comp_[0]);
+            launch_rows(false, d_ra_, nullptr, 1, s_comp_[0], nullptr, false, quad);
             mark("rowA", s_comp_[0]);
         }
     };
@@ -1183,7 +1347,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     }
     // stream 0 has run a's row pass and b's last chunk after the others
     cudaStream_t s0 = s_comp_[0];
-    launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true);
+    launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true, quad);
     if (kind == 0) cuda_check(cudaEventRecord(ev_fused_, s0), "record");
     mark("fused", s0);
     auto issue_out = [&](size_t oc) {
@@ -1195,9 +1359,8 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         const int si = kind == 1 ? 0 : (int)(oc % 3);
         cudaStream_t sc = s_comp_[si];
         if (si != 0) cuda_check(cudaStreamWaitEvent(sc, ev_fused_, 0), "wait");
-        launch_cols(true, d_rb_, ch, 1, sc, si == 0);
         // output chunks run on three streams: each gets its own region of the partial buffers
-        launch_crt(d_rb_, ch, 1, d_out_ + off, sc, (size_t)ch.col0 * nrows, true);
+        launch_inv(d_rb_, ch, 1, d_out_ + off, sc, (size_t)ch.col0 * nrows, si == 0, quad);
         cuda_check(cudaEventRecord(ev_crt_[oc], sc), "record");
         mark("crt" + std::to_string(oc), sc);
         cuda_check(cudaStreamWaitEvent(s_d2h_, ev_crt_[oc], 0), "wait");

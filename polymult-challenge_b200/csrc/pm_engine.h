@@ -16,6 +16,7 @@
 
 #include "pm_device.cuh"
 #include "pm_hostpool.h"
+#include "pm_kernels.cuh"
 #include "pm_plan.h"
 
 namespace pm {
@@ -56,7 +57,9 @@ struct Chunk {
 // Construction options beyond the point itself.
 struct EngineOptions {
     bool host_pipeline = true;  // pinned staging + streams for run_host (not needed by batches)
-    int w1 = -1;                // 4-step split nrows = 2^w1 (-1: logN / 2)
+    // 4-step split nrows = 2^w1; -1: 16 rows with the column stages inside the GEMM kernels where
+    // those apply (tensor-core forms, at most 128 primes, 2^9 <= N <= 2^16), else logN / 2
+    int w1 = -1;
 };
 
 class Engine {
@@ -108,8 +111,15 @@ class Engine {
     void set_variant(bool col_tma, bool crt_tm);
     bool col_tma() const { return dp_.col_tma != 0; }
     bool crt_tm() const { return crt_tm_; }
+    // whether the column stages run inside the GEMM kernels (the 16-row split), and with it the
+    // residues of whole operands lie in the quad layout
+    bool fused() const { return fused_; }
+    // residue words of one operand's scratch (the quad layout rounds the primes up to fours)
+    size_t residue_words() const { return (size_t)(fused_ ? plan_.KP : plan_.K) * plan_.N; }
     bool col_tma_applies() const;
-    bool crt_tm_applies() const { return crt_tm_ok_; }
+    bool crt_tm_applies() const { return crt_tm_ok_ && !fused_; }
+    // the split of the separate column and row passes (a fused engine: the square split's)
+    int split_w1() const { return fused_ ? plan_.logN / 2 : plan_.w1; }
 
     const Plan& plan() const { return plan_; }
     const DevPlan& dev() const { return dp_; }
@@ -129,11 +139,22 @@ class Engine {
     void launch_dec(const uint32_t* src, Chunk ch, uint32_t nb, uint32_t* R, cudaStream_t s, bool ra = false,
                     bool pdl = false) const;
     void launch_cols(bool inv, uint32_t* R, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl = false) const;
-    void launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s,
-                     const uint32_t* ra_sel = nullptr, bool pdl = false) const;
+    void launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, const uint32_t* ra_sel,
+                     bool pdl, bool quad) const;
+    // Decomposition and forward column pass of one chunk, or of both operands of nb multiplies: one
+    // kernel where the 16-row form applies, else a decomposition and a column pass each.  `quad`
+    // (here, in the row passes and the inverse): the multiply runs the 16-row form, its residues
+    // in the quad layout; all of its launches must agree (fused() for whole operands).
+    void launch_fwd(const uint32_t* src, Chunk ch, uint32_t nb, uint32_t* R, cudaStream_t s, bool ra, bool pdl,
+                    bool quad) const;
+    void launch_fwd2(const uint32_t* a, const uint32_t* b, uint32_t nb, uint32_t* RA, uint32_t* RB, cudaStream_t s,
+                     bool pdl) const;
+    // Inverse column pass and CRT of one chunk (one kernel, or two or more).
+    void launch_inv(uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff, bool pdl,
+                    bool quad) const;
     // both operands' row passes in one kernel: forward rows of R (b) and RA (a, after its column
     // pass, read only), pointwise product, inverse rows into R
-    void launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl = false) const;
+    void launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool quad) const;
     // `poff`: first coefficient of this launch's region of the blocked CRT's partial buffers --
     // launches that may run concurrently (other streams) must use disjoint regions
     void launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff = 0,
@@ -147,6 +168,12 @@ class Engine {
         int ring = 2;      // raw input tiles in flight
     };
     bool make_dec_blocks();
+    bool dec16_shape(Dec16Args& A) const;
+    bool crt16_shape(Crt16Args& A) const;
+    void make_fused();
+    void launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl) const;
+    bool rows_overlap(uint32_t nb) const;
+    bool quad_chunks(const std::vector<Chunk>& v) const;
     // (prime block, result-byte block) launches of a CRT too large for one tile
     struct CrtBlock {
         DevPlan dp;
@@ -185,6 +212,11 @@ class Engine {
     bool crt_tm_ = false;                   // the single-tile CRT takes k_crt_tm (A in tensor memory)
     bool crt_tm_ok_ = false;                // k_crt_tm applies to this point
     bool crt_blocked_ = false;              // the tensor-core CRT runs in blocks (K > one tile)
+    // the 16-row split: GEMM kernels with the column stages inside (k_dec16.cu, k_crt16.cu)
+    bool fused_ = false;
+    Dec16Args dec16_{};
+    Crt16Args crt16_{};
+    size_t smem_dec16_ = 0;
     std::vector<DecBlock> dec_blocks_;
     std::vector<CrtBlock> crt_blocks_;
     uint32_t* d_zp_ = nullptr;              // blocked CRT: partial integers [coefficients][L + 3]

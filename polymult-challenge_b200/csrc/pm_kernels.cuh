@@ -43,7 +43,10 @@ void launch_ntt_cols(bool inv, dim3 grid, size_t smem, cudaStream_t s, const Dev
 // inverse; 2 (both): forward stages of R and of RA (after its column pass) side by side,
 // pointwise, inverse stages into R
 void launch_ntt_rows(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                     const uint32_t* ra_sel = nullptr, bool pdl = false);
+                     const uint32_t* ra_sel = nullptr, bool pdl = false, bool quad = false);
+// the row passes' last-phase twiddles in thread order (quad layout only): 16-byte words, and their build
+size_t row_tw_words(const DevPlan& P);
+void build_row_twiddles(const DevPlan& P, uint4* twl, cudaStream_t s);
 // rows of 2^w2 words per row-pass CTA (grid.x = ceil(nrows / this))
 int ntt_rows_per_cta(int w2);
 // line lengths 2^w1 (columns) and 2^w2 (rows) select the compile-time specialisations
@@ -86,6 +89,57 @@ __global__ void k_crt_finish(DevPlan P, const uint32_t* zp, const float* sp, uin
 // crt_nrows <= 256, column chunks of at least 4 columns starting on a multiple of 4.
 __global__ void k_crt_tm(DevPlan P, const uint32_t* R, ChunkMap C, uint32_t npos, uint32_t nbatch, uint32_t* out);
 size_t crt_tm_smem(const DevPlan& P);
+
+// ---- GEMM kernels fused with the 16-row column pass (nrows = 16, ncols = N / 16)
+// Decomposition + forward column pass (k_dec16.cu): points of at most 128 primes.  A launch covers
+// one or both operands of its multiplies.
+struct Dec16Args {
+    const uint32_t* src[2];
+    uint32_t* R[2];               // quad layout
+    uint32_t nops;
+    uint32_t ra_op;               // which operand takes the gamma image (>= nops: none)
+    const unsigned char* img[2];  // A image: plain constants, constants times gamma_j (operand RA)
+    int a_rows, a_zero;           // rows per constant-byte block, zero rows before its primes
+    uint32_t a_bytes;             // the image's size
+    int kb, L, q, qrun;           // K bytes; limbs; lane groups of the image; tiles per accumulator used
+    int nb_buf, ring, rp, segw;   // operand buffers; raw pieces in flight; rows and word pitch of a piece
+    uint32_t N, col0, cw, nbatch;
+    int K, KP;
+    const uint32_t* p;            // [KP]
+    const uint32_t* wsh;          // [KP] floor(2^48 / p)
+    const uint2* tw16;            // [15][KP] twiddles 1..15 of every prime
+    uint32_t* status;
+    long long wait_clocks;
+    int use_bulk;
+};
+constexpr int DEC16_THREADS = 384;
+constexpr int DEC16_MAX_RING = 8;
+size_t dec16_smem(const Dec16Args& A);
+void launch_dec16(const Dec16Args& A, uint32_t grid, size_t smem, cudaStream_t s, bool pdl);
+void dec16_set_smem_limit(int bytes);
+// Inverse column pass + CRT (k_crt16.cu): points of at most 128 primes.
+struct Crt16Args {
+    const uint32_t* R;
+    uint32_t* out;
+    const unsigned char* img;     // B image: rows = result bytes, then the bytes of sum y_j 2^53 / p_j
+    int nrows, nz, kb;            // B rows; rows of result bytes (multiple of 4); K bytes
+    int K, KP, L, W;
+    uint32_t N, col0, cw, nbatch;
+    int fold_count;
+    uint64_t delta;
+    const uint32_t* p;            // [KP]
+    const uint32_t* t1;           // [L]
+    const uint2* tw16;            // [15][KP]
+    uint32_t* status;
+    long long wait_clocks;
+};
+constexpr int CRT16_PROD_WARPS = 8;
+constexpr int CRT16_EPI_WARPS = 8;
+constexpr int CRT16_THREADS = 32 * (CRT16_PROD_WARPS + CRT16_EPI_WARPS + 1);
+size_t crt16_smem(const Crt16Args& A);
+void launch_crt16(const Crt16Args& A, uint32_t grid, cudaStream_t s, bool pdl);
+void crt16_set_smem_limit(int bytes);
+
 // 64-bit digests of `count` arrays of `words` words (k_digest.cu): out_dev[count] (device) is
 // cleared and filled on stream s; digest_host computes the same value on the host
 void launch_digest(const uint32_t* x, uint64_t words, uint32_t count, uint64_t* out_dev, cudaStream_t s);

@@ -536,4 +536,45 @@ void set_split(Plan& P, int w1) {
     P.ncols = 1u << w2;
 }
 
+void set_split16(Plan& P) {
+    if (P.logN < 9 || P.logN > 16) throw InvalidPoint("16-row split outside 2^9 <= N <= 2^16");
+    P.w1 = 4;
+    P.w2 = P.logN - 4;
+    P.nrows = 16;
+    P.ncols = 1u << P.w2;
+}
+
+std::vector<uint8_t> dec16_image(const Plan& P, int rows, int zero, bool gamma) {
+    const int kb = P.dec_gemm.k_bytes;
+    std::vector<uint8_t> img((size_t)4 * rows * kb, 0);
+    for (int j = 0; j < P.K; ++j) {
+        const u64 pj = P.p[j];
+        u64 c = gamma ? mulmod(P.crt_c[j], invmod((1ull << 32) % pj, pj), pj) : 1;
+        for (int s = 0; s < 4 * (int)P.L; ++s, c = mulmod(c, 256, pj))
+            for (int t = 0; t < 4; ++t)
+                img[(size_t)t * rows * kb + umma_kmajor_offset(zero + j, s, kb)] = (uint8_t)(c >> (8 * t));
+    }
+    return img;
+}
+
+std::vector<uint8_t> crt16_image(const Plan& P, int nz, int nrows, int kb) {
+    std::vector<uint8_t> img((size_t)nrows * kb, 0);
+    for (int j = 0; j < P.K; ++j)
+        for (int t = 0; t < 4; ++t) {
+            for (int v = 0; v < std::min(nz, P.crt_gemm.n_rows); ++v)
+                img[umma_kmajor_offset(v, 4 * j + t, kb)] = P.crt_b[umma_kmajor_offset(v, 4 * j + t, P.crt_gemm.k_bytes)];
+            const u64 c = (1ull << 53) / P.p[j];  // below 2^24 for p above 2^29
+            for (int b = 0; b < 3; ++b) img[umma_kmajor_offset(nz + t + b, 4 * j + t, kb)] = (uint8_t)(c >> (8 * b));
+        }
+    return img;
+}
+
+std::vector<uint32_t> tw16_table(const Plan& P) {
+    std::vector<u32> t((size_t)15 * P.KP * 2, 0);
+    for (int j = 0; j < P.K; ++j)
+        for (u32 k = 1; k < 16; ++k)
+            for (int h = 0; h < 2; ++h) t[((size_t)(k - 1) * P.KP + j) * 2 + h] = P.tw[((size_t)j * P.N + k) * 2 + h];
+    return t;
+}
+
 }  // namespace pm

@@ -97,6 +97,20 @@ Plan make_plan(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q);
 // w1 with both line lengths in [1, 2^10] gives the same transform.  Throws InvalidPoint.
 void set_split(Plan& P, int w1);
 
+// Changes the split to 16 rows (w1 = 4, ncols = N / 16 up to 2^12), the split of the GEMM kernels
+// that run the column stages themselves (k_dec16.cu, k_crt16.cu).  2^9 <= N <= 2^16.
+void set_split16(Plan& P);
+
+// Tables of those kernels.  dec16_image: the decomposition's A operand -- per constant byte t a
+// block of `rows` rows (zero rows [0, zero), then a prime per row) x dec K
+// bytes: byte t of 2^(8s) mod p_j, times gamma_j (see dec_b_ra) if `gamma`.
+std::vector<uint8_t> dec16_image(const Plan& P, int rows, int zero, bool gamma);
+// crt16_image: the CRT's B operand without the v column: rows [0, nz) the result bytes against
+// byte 4j+t of y_j, rows nz .. nz+5 the bytes of floor(2^53 / p_j) placed the same way; nrows x kb.
+std::vector<uint8_t> crt16_image(const Plan& P, int nz, int nrows, int kb);
+// [15][KP] Shoup pairs: twiddles 1..15 of every prime, the column stages of 16 rows.
+std::vector<uint32_t> tw16_table(const Plan& P);
+
 // Offset in bytes of element (row, kbyte) inside a K-major no-swizzle canonical tile
 // whose rows hold k_bytes bytes.
 inline size_t umma_kmajor_offset(int row, int kbyte, int k_bytes) {

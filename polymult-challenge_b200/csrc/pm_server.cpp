@@ -44,7 +44,7 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
     eng_.reset(new Engine(N, W, L, q, gemm_request, device, opt));
     try {
         const Plan& P = eng_->plan();
-        const size_t cw = P.coeff_words(), rw = P.residue_words();
+        const size_t cw = P.coeff_words(), rw = eng_->residue_words();
         const uint64_t fixed = (uint64_t)nres_ * rw * 4 + eng_->table_bytes();
         const uint64_t per_req = (uint64_t)(2 * cw + rw) * 4;
         if (hbm_budget <= fixed + per_req)
@@ -80,9 +80,8 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
             cuda_check(cudaMemcpyAsync(s0.in, resident + (size_t)k * cw, cw * 4, cudaMemcpyHostToDevice, s0.stream),
                        "resident upload");
             uint32_t* rk = resident_ + (size_t)k * rw;
-            eng_->launch_dec(s0.in, all, 1, rk, s0.stream, /*ra=*/true);  // the fused pass's RA operand
-            eng_->launch_cols(false, rk, all, 1, s0.stream);
-            eng_->launch_rows(false, rk, nullptr, 1, s0.stream);
+            eng_->launch_fwd(s0.in, all, 1, rk, s0.stream, /*ra=*/true, false, eng_->fused());  // the fused pass's RA operand
+            eng_->launch_rows(false, rk, nullptr, 1, s0.stream, nullptr, false, eng_->fused());
             cuda_check(cudaStreamSynchronize(s0.stream), "resident transform");
         }
         eng_->throw_if_status();
@@ -139,11 +138,10 @@ void Server::launch(Slot& s, const uint32_t* sel, const uint32_t* const* a, uint
     cuda_check(cudaMemcpyAsync(s.sel_d, s.sel_h, nb * 4, cudaMemcpyHostToDevice, s.stream), "selector H2D");
     const Chunk all{0, P.ncols};
     // after the copies the launches follow one another (each may overlap the previous one's tail)
-    eng_->launch_dec(s.in, all, nb, s.res, s.stream);
-    eng_->launch_cols(false, s.res, all, nb, s.stream, true);
-    eng_->launch_rows(true, s.res, resident_, nb, s.stream, s.sel_d, true);
-    eng_->launch_cols(true, s.res, all, nb, s.stream, true);
-    eng_->launch_crt(s.res, all, nb, s.out, s.stream, (size_t)(&s - slots_.data()) * cap_ * P.N, true);
+    const bool f = eng_->fused();
+    eng_->launch_fwd(s.in, all, nb, s.res, s.stream, false, false, f);
+    eng_->launch_rows(true, s.res, resident_, nb, s.stream, s.sel_d, true, f);
+    eng_->launch_inv(s.res, all, nb, s.out, s.stream, (size_t)(&s - slots_.data()) * cap_ * P.N, true, f);
     if (digest) {
         launch_digest(s.out, cw, nb, s.dig_d, s.stream);
         cuda_check(cudaMemcpyAsync(s.dig_h, s.dig_d, nb * 8, cudaMemcpyDeviceToHost, s.stream), "digest D2H");

@@ -58,6 +58,8 @@ uint32_t* scratch_address(int device) {
 // The body of pm_run_device_static (pm_capi.cpp maps its exceptions to status codes and
 // restores the caller's current device).
 void run_device_static(Engine& e, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c, cudaStream_t stream) {
+    // (K N and not the quad layout's KP N: both are within the limit or neither, as N divides it by
+    // multiples of four primes)
     const size_t words = (size_t)e.plan().K * e.plan().N;
     if (2 * words > kStaticScratchWords)
         throw InvalidPoint("pm_run_device_static: K*N = " + std::to_string(words) +
@@ -67,7 +69,7 @@ void run_device_static(Engine& e, const uint32_t* d_a, const uint32_t* d_b, uint
     if (dev < 0 || dev >= kMaxDevices) throw InvalidPoint("device index out of range");
     cuda_check(cudaSetDevice(dev), "cudaSetDevice");
     uint32_t* ra = scratch_address(dev);
-    e.run_device_with_scratch(d_a, d_b, d_c, ra, ra + words, stream);
+    e.run_device_with_scratch(d_a, d_b, d_c, ra, ra + e.residue_words(), stream);
 }
 
 void forget_static_scratch_address(int device) {

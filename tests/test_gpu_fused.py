@@ -1,0 +1,89 @@
+"""The fused form (decomposition + forward column pass, row pass on the quad layout, inverse column
+pass + CRT; the 16-row split) against the plain form of the same point, whose kernels share none of
+its code, at the edges of its ranges.  Results are integers: every byte must be equal."""
+import numpy as np
+import pytest
+
+from conftest import ensure_library, orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _torch():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+def _q(N, W):
+    """Largest number below 2^W that is 1 mod 2N (the library needs no primality)."""
+    return (1 << W) - 2 * N + 1
+
+
+def _operands(torch, N, W, count, seed, off):
+    """[count, N, L] operands below q, `off` words past a 256-byte boundary; the largest value in
+    a few coefficients."""
+    L = (W + 31) // 32
+    rng = np.random.default_rng(seed)
+    x = rng.integers(0, 1 << 32, size=(count, N, L), dtype=np.uint64).astype(np.uint32)
+    if W % 32:
+        x[..., -1] &= np.uint32((1 << (W % 32)) - 1)
+    x[..., -1] &= np.uint32(~(1 << ((W - 1) % 32)) & 0xFFFFFFFF)  # below 2^(W-1) < q
+    x[:, [0, 1, N // 2, N - 1]] = orc.limbs_of(_q(N, W) - 1, L)
+    buf = torch.zeros(x.size + 64, dtype=torch.int32, device="cuda")
+    v = buf[off:off + x.size].view(count, N, L)
+    v.copy_(torch.from_numpy(x.view(np.int32)))
+    return x, v
+
+
+# primes K around the lane groups (32 / 33, 64 / 65 and the largest), limb counts of every residue
+# mod 4, the shortest and longest rows, tile counts that leave lane groups of a super-tile empty,
+# and more tiles than one round of CTAs; (512, 1820) is the first point past the fused CRT's shared
+# memory (more than 120 primes) and runs the separate passes
+POINTS = [(512, 64, 1), (512, 470, 3), (512, 476, 5), (1024, 948, 2), (1024, 956, 1), (512, 1786, 3), (512, 1820, 3), (2048, 97, 40),
+          (2048, 130, 7), (4096, 256, 33), (8192, 1001, 3), (16384, 300, 9), (32768, 868, 2), (65536, 64, 3),
+          (65536, 1747, 2)]
+
+
+@pytest.mark.parametrize("N,W,count", POINTS)
+@pytest.mark.parametrize("off", [0, 1])
+def test_fused_form_equals_plain_form(N, W, count, off):
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    q = orc.limbs_of(_q(N, W), L)
+    _, a = _operands(torch, N, W, count, N + W, off)
+    _, b = _operands(torch, N, W, count, N + W + 1, 0)
+    s = torch.cuda.current_stream().cuda_stream
+    out = {}
+    for gemm in ("tensor", "plain"):
+        c = torch.full((count, N, L), -1, dtype=torch.int32, device="cuda")
+        with polymult.Multiplier(N, W, q, gemm=gemm) as m:
+            if gemm == "tensor":
+                assert m.info()["launches_per_multiply"] == (3 if W < 1800 else 7)
+            m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), count, s)
+            m.sync()
+        out[gemm] = c
+    assert torch.equal(out["tensor"], out["plain"])
+
+
+@pytest.mark.parametrize("body", [1, 4, 16])
+@pytest.mark.parametrize("N,W", [(512, 200), (4096, 300)])
+def test_host_chunks_of_any_width(N, W, body):
+    """Column chunks of whole 8-column tiles run the fused kernels, narrower ones the separate
+    passes; the products are the same."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    xa, a = _operands(torch, N, W, 1, 5, 0)
+    xb, b = _operands(torch, N, W, 1, 6, 0)
+    c = torch.zeros((1, N, L), dtype=torch.int32, device="cuda")
+    with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L), gemm="tensor") as m:
+        m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, torch.cuda.current_stream().cuda_stream)
+        m.sync()
+        m.set_pipeline(body, body)
+        got = m.multiply(xa[0], xb[0])
+    assert np.array_equal(got, c.cpu().numpy().view(np.uint32)[0])
