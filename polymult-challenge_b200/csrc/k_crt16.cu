@@ -25,21 +25,26 @@
 namespace pm {
 
 // ----------------------------------------------------------------------------------------
-// Persistent, 544 threads, one CTA per SM.
-//   producers (warps 0-7): warp w takes prime groups g = w, w + 8, ... (4 primes x 8 columns a
+// Persistent, 896 threads, one CTA per SM.
+//   producers (warps 0-15): warp w takes prime groups g = w, w + 16, ... (4 primes x 8 columns a
 //     round); the next round's 16 residues are loaded while this round's network runs.  The K bytes
 //     form two blocks (the rounds' first and second half): a block is written once the previous
 //     tile's MMAs over it are complete, and its MMAs run while the next block is computed.
-//   epilogue (warps 8-15): two threads per coefficient (low and high limbs), one of two TMEM
+//   epilogue (warps 16-23): two threads per coefficient (low and high limbs), one of two TMEM
 //     accumulators per tile.  The two warps of a TMEM lane quarter hold whole rows of the tile and
 //     synchronise only with one another;
-//   warp 16 issues the MMAs.
+//   warp 24 issues the MMAs.
 // smem: [B image nrows x kb][A 128 x kb][z 128 x zs][T_1 L][twiddles 15 x KP][bars][slot][abort]
 // ----------------------------------------------------------------------------------------
 namespace {
 __host__ __device__ inline int crt16_t1_words(int L) { return (L + 4 + 3) & ~3; }
 constexpr int C16_PROD = 32 * CRT16_PROD_WARPS;
 constexpr int C16_EPI = 32 * CRT16_EPI_WARPS;
+// registers per thread: 896 threads start with 72; the producers (four warpgroups) and the MMA
+// warpgroup give theirs to the epilogue (two): 4 x 64 + 2 x 104 + 40 = 7 x 72
+constexpr int C16_PROD_REGS = 64, C16_EPI_REGS = 104, C16_MMA_REGS = 40;
+static_assert(CRT16_PROD_WARPS / 4 * C16_PROD_REGS + CRT16_EPI_WARPS / 4 * C16_EPI_REGS + C16_MMA_REGS <=
+              (CRT16_PROD_WARPS + CRT16_EPI_WARPS + 4) / 4 * 72, "a warp's share of its SM sub-partition");
 }
 
 // LN >= 0: log2 of the row length N / 16 at compile time (row addresses become immediates).
@@ -90,6 +95,7 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
 
     if (warp < CRT16_PROD_WARPS) {
         // ---------------- producers ----------------
+        regs_dec<C16_PROD_REGS>();
         const int c = lane & 7, jj = lane >> 3;
         const size_t N = LN >= 0 ? (size_t)16 << (LN >= 0 ? LN : 0) : A.N;
         const size_t step = N / 16 * 4;  // words between rows of a quad
@@ -141,8 +147,10 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
             while (round(u, w) && round(w, u)) {
             }
         }
-    } else if (warp == CRT16_PROD_WARPS + CRT16_EPI_WARPS) {
+    } else if (warp >= CRT16_PROD_WARPS + CRT16_EPI_WARPS) {
         // ---------------- MMA issue ----------------
+        regs_dec<C16_MMA_REGS>();
+        if (warp == CRT16_PROD_WARPS + CRT16_EPI_WARPS) {
         const uint32_t mine = elect_one();
         const uint32_t idesc = idesc_u8(A.nrows);
         const uint64_t ad0 = sdesc(smem_addr(a_s), 128u, sbo), bd0 = sdesc(smem_addr(b_s), 128u, sbo);
@@ -178,8 +186,10 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
                 if (blocks[blk]) mbar_wait_bounded(a_free + blk, (blocks[blk] - 1) & 1, A.wait_clocks);
         }
         __syncwarp();
+        }
     } else {
         // ---------------- epilogue ----------------
+        regs_inc<C16_EPI_REGS>();
         const int hf = (warp - CRT16_PROD_WARPS) >> 2, quarter = warp & 3;
         const int m = quarter * 32 + lane;
         const int nl = A.nz / 4;                    // limbs under the result-byte columns (L + 1)
@@ -221,23 +231,32 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
                     t[k] = (uint64_t)v * t1[k] + r[4 * k] + (uint64_t)r[4 * k + 1] * 256u +
                            (uint64_t)r[4 * k + 2] * 65536u + (uint64_t)r[4 * k + 3] * 16777216u;
             };
-            uint32_t r[16], rn[16];
+            uint32_t ra[16], rn[16];
             if (got && l < l1) tmem_ld16_async(tacc + (uint32_t)(4 * l), rn);
-            for (; l + 4 <= l1; l += 4) {  // the next step's load runs under this step
-                if (got) tmem_wait_ld_16(rn);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) r[k] = rn[k];
-                if (got && l + 4 < l1) tmem_ld16_async(tacc + (uint32_t)(4 * l + 16), rn);
+            // four limbs from x, loaded before; the next step's load (y) runs under them
+            auto step = [&](uint32_t (&x)[16], uint32_t (&y)[16]) {
+                if (got) tmem_wait_ld_16(x);
+                if (got && l + 4 < l1) tmem_ld16_async(tacc + (uint32_t)(4 * l + 16), y);
                 const uint4 q1 = *reinterpret_cast<const uint4*>(t1_s + l);
                 const uint32_t t1[4] = {q1.x, q1.y, q1.z, q1.w};
                 uint64_t t[4];
-                limbs4(r, t1, t);
+                limbs4(x, t1, t);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     t[k] += carry;
                     z[l + k] = (uint32_t)t[k];
                     carry = t[k] >> 32;
                 }
+                l += 4;
+            };
+            while (l + 8 <= l1) {
+                step(rn, ra);
+                step(ra, rn);
+            }
+            if (l + 4 <= l1) {
+                step(rn, ra);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) rn[k] = ra[k];
             }
             if (l < l1) {  // the last limbs: the loaded columns past them belong to the quotient
                 if (got) tmem_wait_ld_16(rn);
@@ -266,7 +285,7 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
                     z[x] = (uint32_t)t;
                     carry = t >> 32;
                 }
-                crt_reduce_mod_q(z, zl, A);
+                crt_reduce_fast(z, zl, A);
             }
             named_sync(2 + quarter, 64);
             // the quarter's rows of the tile: 4 runs of 8 coefficients, contiguous in the result; warp

@@ -67,9 +67,18 @@ struct RowCfg : LineCfg<NB> {
     }
 };
 
-template <int NB>
+// Before the reads of an exchange between phases K and K + 1 of a row (either direction).  Only the
+// exchange next to phase 0 crosses warps: phase 0 spreads a thread's elements over the whole row,
+// while from phase 1 on the threads of one block of 2^(b0(0)) elements -- a warp or less -- hold
+// nothing else, and also wrote and read nothing else before: between exchanges, and after the
+// last, a warp is enough.  (With a block barrier on both sides of every exchange the 4096-point
+// rows lost 7% of their issue slots to them.)
+template <int NB, int K>
 __device__ __forceinline__ void region_sync() {
-    if constexpr (RowCfg<NB>::LPR > 32) __syncthreads();
+    using C = RowCfg<NB>;
+    static_assert(C::LPR <= 32 || (1 << (C::b0(0) > 4 ? C::b0(0) - 4 : 0)) <= 32, "phase 1's threads of a block are in one warp");
+    if constexpr (K == 0 && C::LPR == C::THREADS) __syncthreads();
+    else if constexpr (K == 0 && C::LPR > 32) named_sync(1 + (int)threadIdx.x / C::LPR, C::LPR);
     else __syncwarp();
 }
 
@@ -194,9 +203,9 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
         }
         if constexpr (K + 1 < C::NPH) {
             row_xchg<NB, K, true>(v, region, rho, r);
-            region_sync<NB>();
+            region_sync<NB, K>();
             row_xchg<NB, K + 1, false>(v, region, rho, r);
-            region_sync<NB>();
+            __syncwarp();
             row_forward<NB, K + 1, QUAD>(v, region, rho, r, twj, twl, w1, hi, p);
         }
     }
@@ -225,10 +234,10 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
         if constexpr (K + 1 < C::NPH) {
             row_xchg<NB, K, true>(v, region, rho, r);
             row_xchg<NB, K, true>(u, region_u, rho, r);
-            region_sync<NB>();
+            region_sync<NB, K>();
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             row_xchg<NB, K + 1, false>(u, region_u, rho, r);
-            region_sync<NB>();
+            __syncwarp();
             row_forward2<NB, K + 1, QUAD>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
         }
     }
@@ -260,9 +269,9 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
         }
         if constexpr (K > 0) {
             row_xchg<NB, K, true>(v, region, rho, r);
-            region_sync<NB>();
+            region_sync<NB, K - 1>();
             row_xchg<NB, K - 1, false>(v, region, rho, r);
-            region_sync<NB>();
+            if constexpr (K > 1) __syncwarp();
             row_inverse<NB, K - 1, QUAD>(v, region, rho, r, twj, twl, w1, hi_m, p);
         }
     }
@@ -287,8 +296,9 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
 // fused form (host pipeline, server) keeps a 4-byte stack slot at 7 (8 bytes at 6).
 enum : int { ROWS_FWD = 0, ROWS_FUSED = 1, ROWS_BOTH = 2 };
 __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
-    if (nb == 12) return 3;                      // 256 threads, 80 registers
-    if (nb >= 10) return 6;                      // 80 registers
+    if (nb == 12) return 3;                      // 256 threads, 80 registers (4 at 64: 52.7 -> 54.5 us at N = 65536, W = 1747)
+    if (nb == 11) return 7;                      // 72 registers (12.1 -> 11.6 us at N = 32768, W = 868)
+    if (nb == 10) return 6;                      // 80 registers (7 spill: 13.3 -> 14.2 us at N = 16384, W = 1747)
     return nb >= 9 ? (mode == ROWS_FWD ? 5 : 4) : (mode == ROWS_FWD ? 8 : 7);
 }
 // POLYMULT_ROW_STATIC: the row kernels take the column-stage count w1 (and with it nrows and N)

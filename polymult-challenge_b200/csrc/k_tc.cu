@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const u
                     carry = t >> 32;
                 }
                 if (part.mode == CRT_FULL) {
-                    crt_reduce_mod_q(z, zl, P);
+                    crt_reduce_fast(z, zl, P);
                 } else {
                     uint32_t* zr = zp_s + (size_t)m * zs;
                     uint64_t c2 = 0;
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tm(DevPlan P, const u
                     z[k] = (uint32_t)t;
                     carry = t >> 32;
                 }
-                crt_reduce_mod_q(z, zl, P);
+                crt_reduce_fast(z, zl, P);
             }
             named_sync(2, CRT_EPI_THREADS);
             uint32_t* o = out + ((size_t)bt * npos + pos0) * L;
@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(TC_M) k_crt_finish(DevPlan P, const uint32_t* 
             z[l] = (uint32_t)t;
             carry = t >> 32;
         }
-        crt_reduce_mod_q(z, zl, P);
+        crt_reduce_fast(z, zl, P);
     }
     __syncthreads();
     for (int w = threadIdx.x; w < cnt * L; w += TC_M) {

@@ -75,4 +75,31 @@ __device__ __forceinline__ void crt_reduce_mod_q(uint32_t* z, int zl, const Para
     }
 }
 
+// crt_reduce_mod_q for the usual point and value: one fold, W well above the folded limbs, and no
+// carry out of the four low limbs in the fold or in the final + delta, which then leaves z + delta
+// below 2^W: the folded value is the result.  Everything else (a carry comes with probability
+// 2^-64 or so) takes the general form.  One round of loads instead of the general form's chain of
+// dependent ones.
+template <class Params>
+__device__ __forceinline__ void crt_reduce_fast(uint32_t* z, int zl, const Params& P) {
+    const int wl = P.W >> 5, wb = P.W & 31;
+    if (P.fold_count == 1 && wl >= 4) {
+        const uint32_t t0 = z[wl], t1 = z[wl + 1], t2 = z[wl + 2];
+        uint32_t s[4] = {z[0], z[1], z[2], z[3]};
+        uint32_t outside = wb ? t2 >> wb : t2;  // bits from W + 64 up
+        for (int l = wl + 3; l < zl; ++l) outside |= z[l];
+        const uint64_t h = ((uint64_t)__funnelshift_r(t1, t2, wb) << 32) | __funnelshift_r(t0, t1, wb);
+        uint32_t c = crt_add128(s, h * P.delta, __umul64hi(h, P.delta));
+        uint32_t d[4] = {s[0], s[1], s[2], s[3]};
+        c |= crt_add128(d, P.delta, 0);
+        if (c == 0 && outside == 0) {
+#pragma unroll
+            for (int l = 0; l < 4; ++l) z[l] = s[l];
+            z[wl] = wb ? t0 & ((1u << wb) - 1u) : 0u;
+            return;
+        }
+    }
+    crt_reduce_mod_q(z, zl, P);
+}
+
 }  // namespace pm

@@ -133,9 +133,9 @@ struct Crt16Args {
     uint32_t* status;
     long long wait_clocks;
 };
-constexpr int CRT16_PROD_WARPS = 8;
+constexpr int CRT16_PROD_WARPS = 16;
 constexpr int CRT16_EPI_WARPS = 8;
-constexpr int CRT16_THREADS = 32 * (CRT16_PROD_WARPS + CRT16_EPI_WARPS + 1);
+constexpr int CRT16_THREADS = 32 * (CRT16_PROD_WARPS + CRT16_EPI_WARPS + 4);  // the last warpgroup: one MMA warp
 size_t crt16_smem(const Crt16Args& A);
 void launch_crt16(const Crt16Args& A, uint32_t grid, cudaStream_t s, bool pdl);
 void crt16_set_smem_limit(int bytes);

@@ -87,3 +87,33 @@ def test_host_chunks_of_any_width(N, W, body):
         m.set_pipeline(body, body)
         got = m.multiply(xa[0], xb[0])
     assert np.array_equal(got, c.cpu().numpy().view(np.uint32)[0])
+
+
+@pytest.mark.parametrize("N,W,gemm", [(512, 300, "tensor"), (512, 128, "tensor"), (256, 300, "tensor"), (512, 3000, "tensor"),
+                                      (512, 300, "plain")])
+def test_reduction_at_its_carries(N, W, gemm):
+    """a = 1: the products are b's coefficients, chosen so that the reduction's sums carry out of the
+    low limbs (runs of ones of every length, values next to q and to multiples of 2^32)."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    q = _q(N, W)
+    vals = [(1 << k) - 1 for k in range(1, W)] + [(1 << W) - 1 - (1 << k) for k in range(2 * N.bit_length(), W)]
+    vals += [q - 1 - k for k in range(40)] + [1 << k for k in range(W - 1)]
+    vals = [v for v in vals if v < q]
+    a = np.zeros((N, L), dtype=np.uint32)
+    a[0, 0] = 1
+    s = torch.cuda.current_stream().cuda_stream
+    da = torch.from_numpy(a.view(np.int32)).cuda()
+    with polymult.Multiplier(N, W, orc.limbs_of(q, L), gemm=gemm) as m:
+        for i in range(0, len(vals), N):
+            part = vals[i:i + N]
+            b = np.zeros((N, L), dtype=np.uint32)
+            for k, v in enumerate(part):
+                b[k] = orc.limbs_of(v, L)
+            db = torch.from_numpy(b.view(np.int32)).cuda()
+            c = torch.zeros_like(db)
+            m.multiply_device(da.data_ptr(), db.data_ptr(), c.data_ptr(), 1, s)
+            m.sync()
+            assert torch.equal(c, db)
