@@ -52,9 +52,12 @@ __device__ __forceinline__ uint32_t dec_reduce(uint32_t r0, uint32_t r1, uint32_
 //   warp 9 keeps a ring of raw pieces filled: the row segments of `rp` rows of a tile (8 columns x
 //     L limbs each, contiguous in the operand), one bulk copy per lane;
 //   warps 10-11 re-lay each piece out as the K-major operand, in one of `nb_buf` buffers.
-// The four hand work to one another through mbarriers only.  One thread doing all of it (and
-// forming every descriptor and address anew) took 19,000 clocks a tile at L = 55, K = 118, against
-// the epilogue's 5,000.
+// The four hand work to one another through mbarriers only.  One thread doing all of it (and forming
+// every descriptor and address anew) took 19,000 clocks a tile at L = 55, K = 118, against the
+// epilogue's 5,500; the re-layout by branches 6,400 (its warps get the issue slots and the
+// instruction cache that the epilogue leaves); 4-byte cp.async straight into the operand 15,000.
+// Measured 5,800 clocks a tile: 23.6 us for both operands of a multiply at N = 65536, W = 1747
+// (separate decompositions and column passes: 48), the epilogue waiting for 7% of it.
 // A CTA works for one operand (blockIdx.x mod nops), so that its constant image is loaded once and
 // both operands of a multiply share a launch.
 // Few primes (K <= 32 or 64): q = 4 or 2 tiles share an accumulator.  Lanes are split into q groups
@@ -69,6 +72,11 @@ constexpr int D16_RELAY_THREADS = 64;
 constexpr int D16_LOAD_REGS = 56, D16_EPI_REGS = 224;
 static_assert(D16_LOAD_REGS + 2 * D16_EPI_REGS <= 3 * 168, "a warp's share of its SM sub-partition");
 
+// LV: words per aligned load of a coefficient's limbs (4, 2 or 1 as L mod 4 is 0, 2 or odd); 0: an
+// operand off the 16-byte alignment of bulk copies, read limb by limb.  The re-layout has to be
+// short and branch-free: its warps get the instruction cache and the issue slots that the epilogue
+// leaves, and with these cases chosen at run time it took 6,400 clocks a tile (L = 55).
+template <int LV>
 __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constant__ Dec16Args A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int kb = A.kb, q = A.q, qrun = A.qrun, L = A.L;
@@ -174,7 +182,7 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
             __syncwarp();
         } else if (warp == 9) {
             // ---------------- raw copies ----------------
-            if (A.use_bulk) {
+            if constexpr (LV > 0) {
                 uint32_t k = 0;
                 bool ok = true;
                 for (uint32_t i = 0; i < my_super && ok; ++i)
@@ -204,7 +212,7 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
         } else {
             // ---------------- re-layout ----------------
             const int tid = threadIdx.x - D16_EPI_THREADS - 64;
-            const int groups = kb / 16, gfull = L / 4;
+            const int groups = (L + 3) / 4;  // (K bytes past a row's L limbs meet zero constants: whatever is there)
             // a coefficient of the piece (rp rows x 8 columns) and a share of its 16-byte groups;
             // consecutive threads take consecutive rows of one column, so that their 16-byte stores
             // (rows of a core matrix) and, by the segment pitch, their loads fall on different banks
@@ -231,51 +239,40 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
                         const uint32_t sl = k % A.ring;
                         const int n = 128 * s + 16 * c + pc * A.rp + r;
                         unsigned char* dst = bt + (size_t)(n >> 3) * sbo + (n & 7) * 16;
-                        if (!A.use_bulk) {  // an operand off the 16-byte alignment of bulk copies
-                            const uint32_t* row = gsrc + (size_t)pc * A.rp * A.cw * L;
-                            for (int g = g0; g < groups; g += gstep) {
-                                uint4 v;
-                                v.x = 4 * g < L ? __ldg(row + 4 * g) : 0u;
-                                v.y = 4 * g + 1 < L ? __ldg(row + 4 * g + 1) : 0u;
-                                v.z = 4 * g + 2 < L ? __ldg(row + 4 * g + 2) : 0u;
-                                v.w = 4 * g + 3 < L ? __ldg(row + 4 * g + 3) : 0u;
-                                *reinterpret_cast<uint4*>(dst + (size_t)g * 128) = v;
+                        if constexpr (LV > 0) {
+                            ok = wait_or_abort(raw_full + sl, (k / A.ring) & 1, abort_f, A.wait_clocks);
+                            if (!ok) break;
+                        }
+                        const uint32_t* row = LV > 0 ? raw_s + sl * piece_words + row_off : gsrc + (size_t)pc * A.rp * A.cw * L;
+                        // a batch's loads before its stores: the compiler must assume that they alias
+#pragma unroll 1
+                        for (int g = g0; g < groups; g += 4 * gstep) {
+                            uint4 v[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                // (past the row's end: its first group, not stored)
+                                const int l = g + u * gstep < groups ? 4 * (g + u * gstep) : 0;
+                                if constexpr (LV == 4) {
+                                    v[u] = *reinterpret_cast<const uint4*>(row + l);
+                                } else if constexpr (LV == 2) {
+                                    const uint2 u0 = *reinterpret_cast<const uint2*>(row + l);
+                                    const uint2 u1 = *reinterpret_cast<const uint2*>(row + l + 2);
+                                    v[u] = make_uint4(u0.x, u0.y, u1.x, u1.y);
+                                } else if constexpr (LV == 1) {
+                                    v[u] = make_uint4(row[l], row[l + 1], row[l + 2], row[l + 3]);
+                                } else {
+                                    v[u] = make_uint4(__ldg(row + l), __ldg(row + min(l + 1, L - 1)),
+                                                      __ldg(row + min(l + 2, L - 1)), __ldg(row + min(l + 3, L - 1)));
+                                }
                             }
-                            continue;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                                if (g + u * gstep < groups) *reinterpret_cast<uint4*>(dst + (g + u * gstep) * 128) = v[u];
                         }
-                        ok = wait_or_abort(raw_full + sl, (k / A.ring) & 1, abort_f, A.wait_clocks);
-                        if (!ok) break;
-                        const uint32_t* row = raw_s + sl * piece_words + row_off;
-                        int g = g0;
-                        if ((L & 3) == 0) {
-#pragma unroll 4
-                            for (; g < gfull; g += gstep)
-                                *reinterpret_cast<uint4*>(dst + g * 128) = *reinterpret_cast<const uint4*>(row + 4 * g);
-                        } else if ((L & 1) == 0) {
-#pragma unroll 4
-                            for (; g < gfull; g += gstep) {
-                                const uint2 u0 = *reinterpret_cast<const uint2*>(row + 4 * g);
-                                const uint2 u1 = *reinterpret_cast<const uint2*>(row + 4 * g + 2);
-                                *reinterpret_cast<uint4*>(dst + g * 128) = make_uint4(u0.x, u0.y, u1.x, u1.y);
-                            }
-                        } else {
-#pragma unroll 4
-                            for (; g < gfull; g += gstep)
-                                *reinterpret_cast<uint4*>(dst + g * 128) =
-                                    make_uint4(row[4 * g], row[4 * g + 1], row[4 * g + 2], row[4 * g + 3]);
+                        if constexpr (LV > 0) {
+                            fence_smem_to_async();  // the reads above, before the slot's next copy
+                            mbar_arrive(raw_empty + sl);
                         }
-                        // the last, partial group and the zero padding up to kb
-                        for (; g < groups; g += gstep) {
-                            const int l0 = 4 * g;
-                            uint4 v;
-                            v.x = l0 < L ? row[l0] : 0u;
-                            v.y = l0 + 1 < L ? row[l0 + 1] : 0u;
-                            v.z = l0 + 2 < L ? row[l0 + 2] : 0u;
-                            v.w = 0u;
-                            *reinterpret_cast<uint4*>(dst + g * 128) = v;
-                        }
-                        fence_smem_to_async();  // the reads above, before the slot's next copy
-                        mbar_arrive(raw_empty + sl);
                     }
                 }
                 fence_smem_to_async();
@@ -366,13 +363,17 @@ size_t dec16_smem(const Dec16Args& A) {
 }
 
 void launch_dec16(const Dec16Args& A, uint32_t grid, size_t smem, cudaStream_t s, bool pdl) {
-    const cudaError_t e = launch_kernel(k_dec16, dim3(grid), dim3(DEC16_THREADS), smem, s, pdl, A);
+    const bool bulk = (uintptr_t)A.src[0] % 16 == 0 && (A.nops == 1 || (uintptr_t)A.src[1] % 16 == 0);
+    const cudaError_t e = launch_kernel(!bulk ? k_dec16<0> : A.L % 4 == 0 ? k_dec16<4> : A.L % 2 == 0 ? k_dec16<2> : k_dec16<1>,
+                                        dim3(grid), dim3(DEC16_THREADS), smem, s, pdl, A);
     if (e != cudaSuccess) throw_cuda(e, "launch k_dec16");
 }
 
 void dec16_set_smem_limit(int bytes) {
-    const cudaError_t e = cudaFuncSetAttribute(k_dec16, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) throw_cuda(e, "k_dec16 attribute");
+    for (auto f : {k_dec16<0>, k_dec16<1>, k_dec16<2>, k_dec16<4>}) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) throw_cuda(e, "k_dec16 attribute");
+    }
 }
 
 }  // namespace pm

@@ -994,9 +994,6 @@ void Engine::launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s
     A.col0 = ch.col0;
     A.cw = ch.cw;
     A.nbatch = nb;
-    A.use_bulk = 1;
-    for (uint32_t o = 0; o < A.nops; ++o)
-        if ((uintptr_t)A.src[o] % 16 != 0) A.use_bulk = 0;
     const uint32_t tiles = ch.cw / 8 * nb, sms = (uint32_t)num_sms_;
     // as many tiles per accumulator as the image has lane groups, as long as every SM has work
     A.qrun = A.q;

@@ -110,7 +110,6 @@ struct Dec16Args {
     const uint2* tw16;            // [15][KP] twiddles 1..15 of every prime
     uint32_t* status;
     long long wait_clocks;
-    int use_bulk;
 };
 constexpr int DEC16_THREADS = 384;
 constexpr int DEC16_MAX_RING = 8;
