@@ -150,7 +150,18 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
                 unsigned char* dst = a_s + (size_t)(mm >> 3) * sbo + (mm & 7) * 16;
                 const int gfull = mm < cnt ? L / 4 : 0;
                 int g = 0;
-#pragma unroll 4
+                // four groups' loads before their stores, which the compiler must assume to alias: at
+                // 65536 x 3000 bits 47.5 -> 45.9 us an operand, at 4000 bits 107 -> 97
+                for (; g + 4 <= gfull; g += 4) {
+                    uint4 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint32_t* w = row + 4 * (g + u);
+                        v[u] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(dst + (size_t)(g + u) * 128) = v[u];
+                }
                 for (; g < gfull; ++g)
                     *reinterpret_cast<uint4*>(dst + (size_t)g * 128) =
                         make_uint4(row[4 * g], row[4 * g + 1], row[4 * g + 2], row[4 * g + 3]);

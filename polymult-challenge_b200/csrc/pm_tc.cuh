@@ -156,11 +156,10 @@ __device__ __forceinline__ void issue_gemm_rows(uint32_t tmem_col, uint32_t a_ba
                                                 int kbytes, bool acc = false) {
     const uint32_t sbo = 8u * (uint32_t)kbytes;
     const uint32_t idesc = idesc_u8(nn);
-    for (int kk = 0; kk < kbytes / 32; ++kk) {
-        const uint64_t ad = sdesc(a_base + 256u * kk, 128u, sbo);
-        const uint64_t bd = sdesc(b_base + (uint32_t)(row0 >> 3) * sbo + 256u * kk, 128u, sbo);
+    uint64_t ad = sdesc(a_base, 128u, sbo), bd = sdesc(b_base + (uint32_t)(row0 >> 3) * sbo, 128u, sbo);
+#pragma unroll 4
+    for (int kk = 0; kk < kbytes / 32; ++kk, ad += 16, bd += 16)  // 256 bytes in 16-byte units
         umma_u8(tmem_col, ad, bd, idesc, (kk > 0 || acc) ? 1u : 0u);
-    }
 }
 
 // 4-byte asynchronous global -> shared copy (no register staging); cp_async_wait_all waits for
