@@ -3,8 +3,8 @@
 // the inverse column pass does not go through memory.
 //
 // A tile is 128 coefficients, 16 rows x 8 columns of the 4-step matrix.  Producers hold a column
-// of one prime in registers (16 rows; a warp's 4 primes x 8 columns of a row are one 128-byte line
-// of the quad layout), run the four
+// of one prime in registers (16 rows; a warp's 4 primes x 8 columns of a row are halves of two
+// lines of the pair layout), run the four
 // inverse stages as a radix-16 network, and write the 16 results -- y_j, in [0, 2p), since one
 // operand was decomposed times the CRT's per-prime factor -- straight into the tcgen05 A operand
 // (K-major bytes: a residue is the 4 K bytes 4j .. 4j + 3 of its coefficient's row).  The GEMM is
@@ -98,13 +98,12 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
         regs_dec<C16_PROD_REGS>();
         const int c = lane & 7, jj = lane >> 3;
         const size_t N = LN >= 0 ? (size_t)16 << (LN >= 0 ? LN : 0) : A.N;
-        const size_t step = N / 16 * 4;  // words between rows of a quad
+        const size_t step = N / 16 * 2;  // words between rows
         auto load = [&](uint32_t tile, int rd, uint32_t (&x)[16]) {
             const int g = rd * CRT16_PROD_WARPS + warp;
             if (tile >= ntiles || g >= G) return;
             const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-            // lane = 8 (prime in the quad) + column
-            const uint32_t* s = A.R + residue_base(b, A.KP, 4 * g, N) + (A.col0 + 8 * cx) * 4 + lane;
+            const uint32_t* s = A.R + residue_base(b, A.KP, 4 * g + jj, N) + residue_off(A.col0 + 8 * cx) + c;
 #pragma unroll
             for (int e = 0; e < 16; ++e) x[e] = s[e * step];
         };

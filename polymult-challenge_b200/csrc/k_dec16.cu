@@ -11,7 +11,7 @@
 // With a prime per thread the epilogue holds all 16 rows of a column in registers: p, its
 // reduction constant and the pass's 15 twiddles depend on the thread alone, the 4 column stages
 // are a radix-16 network between registers, and a row's 8 columns leave as one 32-byte store,
-// next to the same 8 columns of the three neighbouring primes (the quad layout, pm_device.cuh).
+// next to the same 8 columns of the neighbouring prime (the pair layout, pm_device.cuh).
 //
 // What bounds it: per 128-coefficient tile and SM sub-partition, the integer multiply-add pipe
 // (128 reductions of 1 high + 1 low product, 256 butterflies of 1 high + 2 low: ~3200 clocks) is
@@ -343,11 +343,11 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
             }
             if (mine && tile < ntiles && *abort_f == 0) {
                 const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-                uint32_t* o = A.R[op] + residue_base(b, A.KP, j, N) + (A.col0 + 8 * cx) * 4;
+                uint32_t* o = A.R[op] + residue_base(b, A.KP, j, N) + residue_off(A.col0 + 8 * cx);
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const uint32_t w[8] = {lo[0][e], lo[1][e], lo[2][e], lo[3][e], hi[0][e], hi[1][e], hi[2][e], hi[3][e]};
-                    st_global_v8(o + e * (4 * ncols), w);
+                    st_global_v8(o + e * (2 * ncols), w);
                 }
             }
         }

@@ -120,9 +120,9 @@ __device__ __forceinline__ void row_xchg(uint32_t (&v)[RowCfg<NB>::E], uint32_t*
     }
 }
 
-// global <-> registers in the layout of phase K: rows of consecutive words, or (QUAD) a row of the
-// quad layout, whose element x lies at residue_off(x)
-template <int NB, int K, bool LOAD, bool QUAD>
+// global <-> registers in the layout of phase K: rows of consecutive words, or (PAIR) a row of the
+// pair layout, whose element x lies at residue_off(x)
+template <int NB, int K, bool LOAD, bool PAIR>
 __device__ __forceinline__ void row_global(uint32_t (&v)[RowCfg<NB>::E], uint32_t* row, int r, bool active) {
     using C = RowCfg<NB>;
     if (!active) {
@@ -131,30 +131,50 @@ __device__ __forceinline__ void row_global(uint32_t (&v)[RowCfg<NB>::E], uint32_
             for (int e = 0; e < C::E; ++e) v[e] = 0;
         return;
     }
-    // the register bits of x are zero in the base, and residue_off is additive over disjoint bits
-    const uint32_t x0 = (uint32_t)row_x<NB, K>(r, 0);
-    uint32_t* g0 = row + (QUAD ? residue_off(x0) : x0);
-    if constexpr (C::b0(K) == 0 && C::E >= 4) {  // runs of 4 words (at least), 16-byte aligned
+    if constexpr (PAIR) {
+        // the register bits of x are zero in the base, and residue_off is additive over disjoint bits
+        uint32_t* g0 = row + residue_off((uint32_t)row_x<NB, K>(r, 0));
+        if constexpr (C::b0(K) == 0) {
+#pragma unroll
+            for (int q = 0; q < C::E / 4; ++q) {
+                uint4* g = reinterpret_cast<uint4*>(g0 + residue_off(4 * q));
+                if (LOAD) {
+                    const uint4 u = *g;
+                    v[4 * q] = u.x;
+                    v[4 * q + 1] = u.y;
+                    v[4 * q + 2] = u.z;
+                    v[4 * q + 3] = u.w;
+                } else {
+                    *g = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < C::E; ++e) {
+                uint32_t* g = g0 + residue_off((uint32_t)e << C::b0(K));
+                if (LOAD) v[e] = *g;
+                else *g = v[e];
+            }
+        }
+    } else if constexpr (C::b0(K) == 0 && C::E >= 4) {  // E consecutive words, 16-byte aligned
+        uint4* g = reinterpret_cast<uint4*>(row + row_x<NB, K>(r, 0));
 #pragma unroll
         for (int q = 0; q < C::E / 4; ++q) {
-            uint4* g = reinterpret_cast<uint4*>(g0 + (QUAD ? residue_off(4 * q) : 4 * q));
             if (LOAD) {
-                const uint4 u = *g;
+                const uint4 u = g[q];
                 v[4 * q] = u.x;
                 v[4 * q + 1] = u.y;
                 v[4 * q + 2] = u.z;
                 v[4 * q + 3] = u.w;
             } else {
-                *g = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                g[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
         }
     } else {
 #pragma unroll
         for (int e = 0; e < C::E; ++e) {
-            constexpr int b0 = C::b0(K);
-            uint32_t* g = g0 + (QUAD ? residue_off((uint32_t)e << b0) : (uint32_t)e << b0);
-            if (LOAD) v[e] = *g;
-            else *g = v[e];
+            if (LOAD) v[e] = row[row_x<NB, K>(r, e)];
+            else row[row_x<NB, K>(r, e)] = v[e];
         }
     }
 }
@@ -182,7 +202,7 @@ __host__ __device__ constexpr int row_tw_stride(int lpr) { return 7 * lpr + lpr 
 
 // Forward phases K..NPH-1 of a row (registers in the layout of phase K on entry, of phase
 // NPH-1 on exit).  Stage ls of row hi, group gi uses tw[2^(w1+ls) + hi 2^ls + gi].
-template <int NB, int K, bool QUAD>
+template <int NB, int K, bool PAIR>
 __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
                                             const uint2* twj, const uint4* twl, int w1, uint32_t hi, uint32_t p) {
     using C = RowCfg<NB>;
@@ -195,7 +215,7 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        if constexpr (QUAD && K == C::NPH - 1) {
+        if constexpr (PAIR && K == C::NPH - 1) {
             auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
             radix_fwd<C::RB, C::t0(K)>(v, ltw, p);
         } else {
@@ -206,14 +226,14 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
             region_sync<NB, K>();
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             __syncwarp();
-            row_forward<NB, K + 1, QUAD>(v, region, rho, r, twj, twl, w1, hi, p);
+            row_forward<NB, K + 1, PAIR>(v, region, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
 
 // row_forward on two operands' rows of the same prime and row index (b in v, a in u), each in
 // its own shared-memory region for the exchanges.
-template <int NB, int K, bool QUAD>
+template <int NB, int K, bool PAIR>
 __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint32_t (&u)[RowCfg<NB>::E],
                                              uint32_t* region, uint32_t* region_u, int rho, int r, const uint2* twj,
                                              const uint4* twl, int w1, uint32_t hi, uint32_t p) {
@@ -225,7 +245,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        if constexpr (QUAD && K == C::NPH - 1) {
+        if constexpr (PAIR && K == C::NPH - 1) {
             auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
             radix_fwd2<C::RB, C::t0(K)>(v, u, ltw, p);
         } else {
@@ -238,7 +258,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             row_xchg<NB, K + 1, false>(u, region_u, rho, r);
             __syncwarp();
-            row_forward2<NB, K + 1, QUAD>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
+            row_forward2<NB, K + 1, PAIR>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
@@ -246,7 +266,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
 // Inverse phases K down to 0 (registers in the layout of phase K on entry, phase 0 on exit).
 // The inverse twiddle of (ls, hi, gi) is the forward entry of the mirrored row nrows-1-hi at
 // 2^ls - 1 - gi.
-template <int NB, int K, bool QUAD>
+template <int NB, int K, bool PAIR>
 __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
                                             const uint2* twj, const uint4* twl, int w1, uint32_t hi_m, uint32_t p) {
     using C = RowCfg<NB>;
@@ -259,7 +279,7 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<true>{twj + (1u << (w1 + ls)) + (hi_m << ls) + (1u << ls) - ((hip + 1u) << t), 1 << t};
         };
-        if constexpr (QUAD && K == C::NPH - 1) {  // thread LPR - 1 - r's entries of the mirrored row, reversed
+        if constexpr (PAIR && K == C::NPH - 1) {  // thread LPR - 1 - r's entries of the mirrored row, reversed
             auto ltw = [&](int t) {
                 return RowTw<C::LPR, true>{twl + (size_t)hi_m * row_tw_stride(C::LPR), C::LPR - 1 - r, 1 << t};
             };
@@ -271,8 +291,8 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
             row_xchg<NB, K, true>(v, region, rho, r);
             region_sync<NB, K - 1>();
             row_xchg<NB, K - 1, false>(v, region, rho, r);
-            if constexpr (K > 1) __syncwarp();
-            row_inverse<NB, K - 1, QUAD>(v, region, rho, r, twj, twl, w1, hi_m, p);
+            __syncwarp();
+            row_inverse<NB, K - 1, PAIR>(v, region, rho, r, twj, twl, w1, hi_m, p);
         }
     }
 }
@@ -309,8 +329,8 @@ __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
 #ifndef POLYMULT_ROW_STATIC
 #define POLYMULT_ROW_STATIC 1
 #endif
-// QUAD: the residues lie in the quad layout (the 16-row split).
-template <int NB, int MODE, int W1, bool QUAD>
+// PAIR: the residues lie in the pair layout (the 16-row split).
+template <int NB, int MODE, int W1, bool PAIR>
 __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)) k_ntt_rows(DevPlan P, uint32_t* __restrict__ R,
                                                                            const uint32_t* __restrict__ RA,
                                                                            const uint32_t* __restrict__ ra_sel) {
@@ -343,40 +363,44 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
     const bool active = hi < nrows;
     const uint32_t hic = active ? hi : nrows - 1;  // keeps twiddle reads in range
     const uint32_t p = P.p[j], pinv = P.pinv[j];
-    auto row_off = [&](uint32_t z) {
-        return QUAD ? residue_base(z, P.KP, j, Nn) + (size_t)hic * (4u << NB)
-                    : ((size_t)z * P.K + j) * Nn + (size_t)hic * (1u << NB);
-    };
-    const size_t off = row_off(zb);
+    size_t off;
+    if constexpr (PAIR) {
+        auto qo = [&](size_t z) { return residue_base((uint32_t)z, P.KP, j, Nn) + (size_t)hic * (2u << NB); };
+        off = qo(zb);
+    }
+    else off = ((size_t)zb * P.K + j) * Nn + (size_t)hic * (1u << NB);
     uint32_t* row = R + off;
     const uint2* twj = P.tw + (size_t)j * Nn;
-    const uint4* twl = QUAD ? P.twl + (size_t)j * nrows * row_tw_stride(C::LPR) : nullptr;
+    const uint4* twl = nullptr;
+    if constexpr (PAIR) twl = P.twl + (size_t)j * nrows * row_tw_stride(C::LPR);
 
     uint32_t v[C::E];
     pdl_trigger();
     pdl_wait();
-    row_global<NB, 0, true, QUAD>(v, row, r, active);
+    row_global<NB, 0, true, PAIR>(v, row, r, active);
     if constexpr (MODE == ROWS_BOTH) {
         uint32_t a[C::E];
-        row_global<NB, 0, true, QUAD>(a, const_cast<uint32_t*>(RA + off), r, active);
-        row_forward2<NB, 0, QUAD>(v, a, region, region + REGION_WORDS, rho, r, twj, twl, w1, hic, p);
+        row_global<NB, 0, true, PAIR>(a, const_cast<uint32_t*>(RA + off), r, active);
+        row_forward2<NB, 0, PAIR>(v, a, region, region + REGION_WORDS, rho, r, twj, twl, w1, hic, p);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1, QUAD>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
-        row_global<NB, 0, false, QUAD>(v, row, r, active);
+        row_inverse<NB, C::NPH - 1, PAIR>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_global<NB, 0, false, PAIR>(v, row, r, active);
     } else if constexpr (MODE == ROWS_FUSED) {
-        row_forward<NB, 0, QUAD>(v, region, rho, r, twj, twl, w1, hic, p);
+        row_forward<NB, 0, PAIR>(v, region, rho, r, twj, twl, w1, hic, p);
         uint32_t a[C::E];
         const size_t za = ra_sel ? (size_t)__ldg(ra_sel + zb) : (size_t)zb;
-        const size_t offa = row_off((uint32_t)za);
-        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true, QUAD>(a, const_cast<uint32_t*>(RA + offa), r, active);
+        size_t offa;
+        if constexpr (PAIR) offa = residue_base((uint32_t)za, P.KP, j, Nn) + (size_t)hic * (2u << NB);
+        else offa = (za * P.K + j) * Nn + (size_t)hic * (1u << NB);
+        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true, PAIR>(a, const_cast<uint32_t*>(RA + offa), r, active);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1, QUAD>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
-        row_global<NB, 0, false, QUAD>(v, row, r, active);
+        row_inverse<NB, C::NPH - 1, PAIR>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_global<NB, 0, false, PAIR>(v, row, r, active);
     } else {
-        row_forward<NB, 0, QUAD>(v, region, rho, r, twj, twl, w1, hic, p);
-        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), false, QUAD>(v, row, r, active);
+        row_forward<NB, 0, PAIR>(v, region, rho, r, twj, twl, w1, hic, p);
+        row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), false, PAIR>(v, row, r, active);
     }
 }
 
@@ -894,11 +918,11 @@ void launch_cols_nb(bool inv, dim3 grid, size_t smem, cudaStream_t s, const DevP
 // the row kernel of a mode for line length 2^NB and the plan's w1: a compile-time w1 for the
 // splits of N = 4096 .. 65536 that the batches and the engine use, else w1 from the plan
 template <int NB, int MODE>
-auto row_kernel(int w1, bool quad) {
+auto row_kernel(int w1, bool pair) {
     if constexpr (NB >= 5) {
-        if (quad) return k_ntt_rows<NB, MODE, 4, true>;  // the 16-row split
+        if (pair) return k_ntt_rows<NB, MODE, 4, true>;  // the 16-row split
     }
-    (void)quad;
+    (void)pair;
     if constexpr (POLYMULT_ROW_STATIC && NB >= 6 && NB <= 8) {
         if (w1 == NB) return k_ntt_rows<NB, MODE, NB, false>;
         if (w1 == NB - 1) return k_ntt_rows<NB, MODE, NB - 1, false>;
@@ -909,12 +933,12 @@ auto row_kernel(int w1, bool quad) {
 
 template <int NB>
 void launch_rows_nb(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                    const uint32_t* ra_sel, bool pdl, bool quad) {
+                    const uint32_t* ra_sel, bool pdl, bool pair) {
     // grid comes as (row blocks, primes, batch); the static form takes it as (batch, row blocks, primes)
     const dim3 g = POLYMULT_ROW_STATIC ? dim3(grid.z, grid.x, grid.y) : grid;
-    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P.w1, quad)
-                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P.w1, quad)
-                                                             : row_kernel<NB, ROWS_FWD>(P.w1, quad),
+    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P.w1, pair)
+                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P.w1, pair)
+                                                             : row_kernel<NB, ROWS_FWD>(P.w1, pair),
                                         g, dim3(RowCfg<NB>::THREADS), 0, s, pdl, P, R, RA, ra_sel);
     if (e != cudaSuccess)
         throw_cuda(e, mode == ROWS_BOTH    ? "launch k_ntt_rows<both operands>"
@@ -1034,8 +1058,8 @@ void launch_ntt_cols(bool inv, dim3 grid, size_t smem, cudaStream_t s, const Dev
 }
 
 void launch_ntt_rows(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                     const uint32_t* ra_sel, bool pdl, bool quad) {
-    dispatch_rows<RowsF>(P.w2, mode, grid, s, P, R, RA, ra_sel, pdl, quad);
+                     const uint32_t* ra_sel, bool pdl, bool pair) {
+    dispatch_rows<RowsF>(P.w2, mode, grid, s, P, R, RA, ra_sel, pdl, pair);
 }
 
 int ntt_rows_per_cta(int w2) {

@@ -71,17 +71,21 @@ struct CrtPrimeBlocks {
     const unsigned char* b[MAX];
 };
 
-// Quad layout of the residue arrays, used by the 16-row split: four primes share 128-byte lines,
-//   word (j, n) of a batch entry = (j / 4) 4N + (n / 8) 32 + (j % 4) 8 + n % 8,
+// Pair layout of the residue arrays, used by the 16-row split: two primes share 128-byte lines,
+//   word (j, n) of a batch entry = (j / 2) 2N + (n / 16) 32 + (j % 2) 16 + n % 16,
 // KP primes' room per entry.  A kernel that holds a prime per lane (8 columns of one row each)
-// moves whole lines, 8 a warp instead of 32; a row kernel, one prime a block, moves whole
-// sectors of lines that its three neighbour blocks share.
+// touches 16 lines a warp store instead of 32; a row kernel, one prime a block, reads 32
+// elements from 2 lines instead of 1.  With four primes a line the two prime-per-lane kernels were
+// faster (65536 x 1747 bits x 32: decomposition 23.6 against 25.5 us a multiply, CRT 17.4 against
+// 19.8) and the row pass slower (52.1 against 48.8); in sum the pairs gain 1 to 2 % (95.0 -> 93.9;
+// 32768 x 868 bits x 16: 23.4 -> 22.8) except at few large multiplies (x 4: 391 against 398 us).
 // Word of (prime j, coefficient 0) of batch entry b:
 __device__ __forceinline__ size_t residue_base(uint32_t b, int KP, int j, size_t N) {
-    return ((size_t)b * KP + (j & ~3)) * N + (size_t)(j & 3) * 8;
+    return ((size_t)b * KP + (j & ~1)) * N + (size_t)(j & 1) * 16;
 }
-// offset of coefficient n (a multiple of 8, or within its 8) from there; additive over disjoint bits
-__host__ __device__ constexpr uint32_t residue_off(uint32_t n) { return ((n >> 3) << 5) | (n & 7u); }
+// offset of coefficient n from there; additive over disjoint bits, and a row of ncols >= 16 elements
+// takes 2 ncols words
+__host__ __device__ constexpr uint32_t residue_off(uint32_t n) { return ((n >> 4) << 5) | (n & 15u); }
 
 __device__ __forceinline__ uint32_t chunk_pos_to_n(const DevPlan& P, const ChunkMap& C, uint32_t pos) {
     return ((pos >> C.lcw) << P.w2) + C.col0 + (pos & (C.cw - 1));

@@ -631,7 +631,7 @@ bool Engine::dec16_shape(Dec16Args& A) const {
 }
 
 // Column chunks that the fused kernels take: whole 8-column tiles.
-bool Engine::quad_chunks(const std::vector<Chunk>& v) const {
+bool Engine::pair_chunks(const std::vector<Chunk>& v) const {
     for (const Chunk& c : v)
         if (c.cw % 8 || c.col0 % 8) return false;
     return true;
@@ -920,14 +920,14 @@ bool Engine::rows_overlap(uint32_t nb) const {
 }
 
 void Engine::launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s,
-                         const uint32_t* ra_sel, bool pdl, bool quad) const {
+                         const uint32_t* ra_sel, bool pdl, bool pair) const {
     dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl && (!quad || rows_overlap(nb)), quad);
+    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl && (!pair || rows_overlap(nb)), pair);
 }
 
-void Engine::launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool quad) const {
+void Engine::launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool pair) const {
     dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl && (!quad || rows_overlap(nb)), quad);
+    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl && (!pair || rows_overlap(nb)), pair);
 }
 
 void Engine::launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff,
@@ -1003,8 +1003,8 @@ void Engine::launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s
 }
 
 void Engine::launch_fwd(const uint32_t* src, Chunk ch, uint32_t nb, uint32_t* R, cudaStream_t s, bool ra, bool pdl,
-                        bool quad) const {
-    if (quad) {
+                        bool pair) const {
+    if (pair) {
         Dec16Args A = dec16_;
         A.nops = 1;
         A.src[0] = src;
@@ -1036,8 +1036,8 @@ void Engine::launch_fwd2(const uint32_t* a, const uint32_t* b, uint32_t nb, uint
 }
 
 void Engine::launch_inv(uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff, bool pdl,
-                        bool quad) const {
-    if (quad) {
+                        bool pair) const {
+    if (pair) {
         Crt16Args A = crt16_;
         A.R = R;
         A.out = out;
@@ -1203,7 +1203,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     const size_t nout = cout.size();
     // the fused kernels work on whole 8-column tiles: a schedule with narrower chunks runs the
     // decomposition, the column passes and the CRT as kernels of their own
-    const bool quad = fused() && quad_chunks(cin_[kind]) && quad_chunks(cout);
+    const bool pair = fused() && pair_chunks(cin_[kind]) && pair_chunks(cout);
     // input items (operand, column chunk): both operands in the schedule's input chunks; with
     // direct copies a moves in one piece (each copy costs a few microseconds of DMA set-up, and
     // a's transform is hidden under b's transfer anyway) and only b is chunked
@@ -1286,14 +1286,14 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         if (last)
             for (int q = na; q < k; ++q) cuda_check(cudaStreamWaitEvent(sc, ev_done_in_[q], 0), "wait");
         cuda_check(cudaStreamWaitEvent(sc, ev_in_[hi], 0), "wait");
-        launch_fwd(d_in_[P] + off, ch, 1, dR[P], sc, P == 0, false, quad);
+        launch_fwd(d_in_[P] + off, ch, 1, dR[P], sc, P == 0, false, pair);
         if (!last) {
             cuda_check(cudaEventRecord(ev_done_in_[k], sc), "record");
             mark("in" + std::to_string(k), sc);
         }
         if (k == na - 1) {  // a complete: its row pass overlaps b's transfer
             for (int q = 0; q < na; ++q) cuda_check(cudaStreamWaitEvent(s_comp_[0], ev_done_in_[q], 0), "wait");
-            launch_rows(false, d_ra_, nullptr, 1, s_comp_[0], nullptr, false, quad);
+            launch_rows(false, d_ra_, nullptr, 1, s_comp_[0], nullptr, false, pair);
             mark("rowA", s_comp_[0]);
         }
     };
@@ -1344,7 +1344,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     }
     // stream 0 has run a's row pass and b's last chunk after the others
     cudaStream_t s0 = s_comp_[0];
-    launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true, quad);
+    launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true, pair);
     if (kind == 0) cuda_check(cudaEventRecord(ev_fused_, s0), "record");
     mark("fused", s0);
     auto issue_out = [&](size_t oc) {
@@ -1357,7 +1357,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         cudaStream_t sc = s_comp_[si];
         if (si != 0) cuda_check(cudaStreamWaitEvent(sc, ev_fused_, 0), "wait");
         // output chunks run on three streams: each gets its own region of the partial buffers
-        launch_inv(d_rb_, ch, 1, d_out_ + off, sc, (size_t)ch.col0 * nrows, si == 0, quad);
+        launch_inv(d_rb_, ch, 1, d_out_ + off, sc, (size_t)ch.col0 * nrows, si == 0, pair);
         cuda_check(cudaEventRecord(ev_crt_[oc], sc), "record");
         mark("crt" + std::to_string(oc), sc);
         cuda_check(cudaStreamWaitEvent(s_d2h_, ev_crt_[oc], 0), "wait");

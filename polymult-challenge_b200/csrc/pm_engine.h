@@ -112,9 +112,9 @@ class Engine {
     bool col_tma() const { return dp_.col_tma != 0; }
     bool crt_tm() const { return crt_tm_; }
     // whether the column stages run inside the GEMM kernels (the 16-row split), and with it the
-    // residues of whole operands lie in the quad layout
+    // residues of whole operands lie in the pair layout
     bool fused() const { return fused_; }
-    // residue words of one operand's scratch (the quad layout rounds the primes up to fours)
+    // residue words of one operand's scratch (the pair layout rounds the primes up to fours)
     size_t residue_words() const { return (size_t)(fused_ ? plan_.KP : plan_.K) * plan_.N; }
     bool col_tma_applies() const;
     bool crt_tm_applies() const { return crt_tm_ok_ && !fused_; }
@@ -140,21 +140,21 @@ class Engine {
                     bool pdl = false) const;
     void launch_cols(bool inv, uint32_t* R, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl = false) const;
     void launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, const uint32_t* ra_sel,
-                     bool pdl, bool quad) const;
+                     bool pdl, bool pair) const;
     // Decomposition and forward column pass of one chunk, or of both operands of nb multiplies: one
-    // kernel where the 16-row form applies, else a decomposition and a column pass each.  `quad`
+    // kernel where the 16-row form applies, else a decomposition and a column pass each.  `pair`
     // (here, in the row passes and the inverse): the multiply runs the 16-row form, its residues
-    // in the quad layout; all of its launches must agree (fused() for whole operands).
+    // in the pair layout; all of its launches must agree (fused() for whole operands).
     void launch_fwd(const uint32_t* src, Chunk ch, uint32_t nb, uint32_t* R, cudaStream_t s, bool ra, bool pdl,
-                    bool quad) const;
+                    bool pair) const;
     void launch_fwd2(const uint32_t* a, const uint32_t* b, uint32_t nb, uint32_t* RA, uint32_t* RB, cudaStream_t s,
                      bool pdl) const;
     // Inverse column pass and CRT of one chunk (one kernel, or two or more).
     void launch_inv(uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff, bool pdl,
-                    bool quad) const;
+                    bool pair) const;
     // both operands' row passes in one kernel: forward rows of R (b) and RA (a, after its column
     // pass, read only), pointwise product, inverse rows into R
-    void launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool quad) const;
+    void launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool pair) const;
     // `poff`: first coefficient of this launch's region of the blocked CRT's partial buffers --
     // launches that may run concurrently (other streams) must use disjoint regions
     void launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff = 0,
@@ -173,7 +173,7 @@ class Engine {
     void make_fused();
     void launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl) const;
     bool rows_overlap(uint32_t nb) const;
-    bool quad_chunks(const std::vector<Chunk>& v) const;
+    bool pair_chunks(const std::vector<Chunk>& v) const;
     // (prime block, result-byte block) launches of a CRT too large for one tile
     struct CrtBlock {
         DevPlan dp;

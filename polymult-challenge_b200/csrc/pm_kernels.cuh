@@ -43,8 +43,8 @@ void launch_ntt_cols(bool inv, dim3 grid, size_t smem, cudaStream_t s, const Dev
 // inverse; 2 (both): forward stages of R and of RA (after its column pass) side by side,
 // pointwise, inverse stages into R
 void launch_ntt_rows(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
-                     const uint32_t* ra_sel = nullptr, bool pdl = false, bool quad = false);
-// the row passes' last-phase twiddles in thread order (quad layout only): 16-byte words, and their build
+                     const uint32_t* ra_sel = nullptr, bool pdl = false, bool pair = false);
+// the row passes' last-phase twiddles in thread order (pair layout only): 16-byte words, and their build
 size_t row_tw_words(const DevPlan& P);
 void build_row_twiddles(const DevPlan& P, uint4* twl, cudaStream_t s);
 // rows of 2^w2 words per row-pass CTA (grid.x = ceil(nrows / this))
@@ -95,7 +95,7 @@ size_t crt_tm_smem(const DevPlan& P);
 // one or both operands of its multiplies.
 struct Dec16Args {
     const uint32_t* src[2];
-    uint32_t* R[2];               // quad layout
+    uint32_t* R[2];               // pair layout
     uint32_t nops;
     uint32_t ra_op;               // which operand takes the gamma image (>= nops: none)
     const unsigned char* img[2];  // A image: plain constants, constants times gamma_j (operand RA)

@@ -1,4 +1,4 @@
-"""The fused form (decomposition + forward column pass, row pass on the quad layout, inverse column
+"""The fused form (decomposition + forward column pass, row pass on the pair layout, inverse column
 pass + CRT; the 16-row split) against the plain form of the same point, whose kernels share none of
 its code, at the edges of its ranges.  Results are integers: every byte must be equal."""
 import numpy as np
