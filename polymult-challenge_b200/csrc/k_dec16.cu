@@ -49,8 +49,8 @@ __device__ __forceinline__ uint32_t dec_reduce(uint32_t r0, uint32_t r1, uint32_
 //     (64 coefficients, 256 TMEM columns each), releasing a half as soon as its last TMEM load is
 //     done, so that the next tile's MMAs of that half run under this tile's butterflies;
 //   warp 8 issues the MMAs of the two halves, each once the epilogue has released it;
-//   warp 9 keeps a ring of raw pieces filled: the row segments of `rp` rows of a tile (8 columns x
-//     L limbs each, contiguous in the operand), one bulk copy per lane;
+//   warp 9 keeps a ring of raw pieces filled: the row segments of `npo` row octets of the super-tile
+//     (8 columns x L limbs each, contiguous in the operand), one bulk copy per row;
 //   warps 10-11 re-lay each piece out as the K-major operand, in one of `nb_buf` buffers.
 // The four hand work to one another through mbarriers only.  One thread doing all of it (and forming
 // every descriptor and address anew) took 19,000 clocks a tile at L = 55, K = 118, against the
@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
     const size_t b_bytes = (size_t)q * TC_M * kb;
     uint32_t* raw_s = reinterpret_cast<uint32_t*>(b_s + A.nb_buf * b_bytes);
     const int segw = A.segw;                     // words between a piece's row segments
-    const size_t piece_words = (size_t)A.rp * segw;
+    const int npo = A.npo;                       // row octets of a piece
+    const size_t piece_words = (size_t)A.piece_octets * 8 * segw;
     const int tws = A.KP;                         // entries per row of the twiddle table
     uint2* tw_s = reinterpret_cast<uint2*>(raw_s + A.ring * piece_words);
     uint64_t* bars = reinterpret_cast<uint64_t*>(tw_s + 15 * tws);
@@ -102,8 +103,8 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
     volatile int* abort_f = reinterpret_cast<volatile int*>(slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // super-tiles me, me + mates, ... of the operand; a tile's pieces in row order
-    const int ppt = 16 / A.rp;  // pieces per tile
+    // super-tiles me, me + mates, ... of the operand; their row octets (two a tile) in pieces of npo
+    const int npieces = 2 * qrun / npo;  // of a super-tile
     const uint32_t my_super = me < nsuper ? (nsuper - me + mates - 1) / mates : 0;
 
     if (threadIdx.x == D16_EPI_THREADS) {
@@ -185,23 +186,27 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
             if constexpr (LV > 0) {
                 uint32_t k = 0;
                 bool ok = true;
-                for (uint32_t i = 0; i < my_super && ok; ++i)
-                    for (int s = 0; s < qrun && ok; ++s) {
-                        const uint32_t tile = (me + i * mates) * (uint32_t)qrun + s;
-                        if (tile >= ntiles) break;
-                        const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-                        const uint32_t* g = src + (((size_t)b * 16 + lane) * A.cw + 8 * cx) * L;
-                        const size_t gstep = (size_t)A.rp * A.cw * L;
-                        for (int pc = 0; pc < ppt && ok; ++pc, ++k, g += gstep) {
-                            const uint32_t sl = k % A.ring, use = k / A.ring;
-                            if (use > 0) ok = wait_or_abort(raw_empty + sl, (use - 1) & 1, abort_f, A.wait_clocks);
-                            ok = __all_sync(0xffffffffu, ok);
-                            if (!ok) break;
-                            if (lane == 0) mbar_arrive_expect_tx(raw_full + sl, 32u * L * A.rp);
-                            __syncwarp();
-                            if (lane < A.rp) bulk_g2s(raw_s + sl * piece_words + lane * segw, g, 32u * L, raw_full + sl);
+                for (uint32_t i = 0; i < my_super && ok; ++i) {
+                    const uint32_t t0 = (me + i * mates) * (uint32_t)qrun;
+                    for (int pc = 0; pc < npieces && ok; ++pc) {
+                        const int o0 = pc * npo;  // the piece's first octet
+                        const int no = min(npo, 2 * (int)min((uint32_t)qrun, ntiles - t0) - o0);  // with tiles
+                        if (no <= 0) break;
+                        const uint32_t sl = k % A.ring, use = k / A.ring;
+                        if (use > 0) ok = wait_or_abort(raw_empty + sl, (use - 1) & 1, abort_f, A.wait_clocks);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        if (lane == 0) mbar_arrive_expect_tx(raw_full + sl, 32u * L * 8u * no);
+                        __syncwarp();
+                        for (int x = lane; x < 8 * no; x += 32) {
+                            const int row = 8 * o0 + x;  // row of the super-tile
+                            const uint32_t tile = t0 + (row >> 4), b = tile / tiles_x, cx = tile - b * tiles_x;
+                            bulk_g2s(raw_s + sl * piece_words + x * segw,
+                                     src + (((size_t)b * 16 + (row & 15)) * A.cw + 8 * cx) * L, 32u * L, raw_full + sl);
                         }
+                        ++k;
                     }
+                }
                 // every copy issued lands before the CTA exits (the latest per slot)
                 __syncwarp();
                 if (lane == 0)
@@ -213,45 +218,50 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
             // ---------------- re-layout ----------------
             const int tid = threadIdx.x - D16_EPI_THREADS - 64;
             const int groups = (L + 3) / 4;  // (K bytes past a row's L limbs meet zero constants: whatever is there)
-            // a coefficient of the piece (rp rows x 8 columns) and a share of its 16-byte groups;
-            // consecutive threads take consecutive rows of one column, so that their 16-byte stores
-            // (rows of a core matrix) and, by the segment pitch, their loads fall on different banks
-            const int lrp = A.rp == 8 ? 3 : A.rp == 4 ? 2 : 1;
-            const int ci = tid & (8 * A.rp - 1), g0 = tid >> (3 + lrp), gstep = D16_RELAY_THREADS >> (3 + lrp);
-            const int r = ci & (A.rp - 1), c = ci >> lrp;
+            // a coefficient of an octet (8 rows x 8 columns) each; consecutive threads take consecutive
+            // rows of one column, so that their 16-byte stores (rows of a core matrix) and, by the raw
+            // rows' pitch, their loads fall on different banks
+            const int r = tid & 7, c = tid >> 3;
             const int row_off = r * segw + c * L;
             uint32_t k = 0;
             bool ok = true;
             for (uint32_t i = 0; i < my_super && ok; ++i) {
                 const int buf = A.nb_buf == 2 ? (int)(i & 1) : 0;
-                unsigned char* bt = b_s + buf * b_bytes;
+                const uint32_t t0 = (me + i * mates) * (uint32_t)qrun;
                 // the MMAs that last read this buffer (super-tile i - nb_buf) are complete
                 if (i >= (uint32_t)A.nb_buf) {
                     const uint32_t o = i - A.nb_buf;
                     ok = wait_or_abort(mma_done + 2 * (o & 1) + 1, (o >> 1) & 1, abort_f, A.wait_clocks);
                 }
-                for (int s = 0; s < qrun && ok; ++s) {
-                    const uint32_t tile = (me + i * mates) * (uint32_t)qrun + s;
-                    if (tile >= ntiles) break;
-                    const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-                    const uint32_t* gsrc = src + (((size_t)b * 16 + r) * A.cw + 8 * cx + c) * L;
-                    for (int pc = 0; pc < ppt && ok; ++pc, ++k) {
-                        const uint32_t sl = k % A.ring;
-                        const int n = 128 * s + 16 * c + pc * A.rp + r;
-                        unsigned char* dst = bt + (size_t)(n >> 3) * sbo + (n & 7) * 16;
-                        if constexpr (LV > 0) {
-                            ok = wait_or_abort(raw_full + sl, (k / A.ring) & 1, abort_f, A.wait_clocks);
-                            if (!ok) break;
+                // octet o's rows of column c: operand rows 16 c + 8 (o & 1) + r of tile o / 2
+                unsigned char* bt = b_s + buf * b_bytes + (size_t)(2 * c) * sbo + r * 16;
+                for (int pc = 0; pc < npieces && ok; ++pc) {
+                    const int o0 = pc * npo;
+                    const int no = min(npo, 2 * (int)min((uint32_t)qrun, ntiles - t0) - o0);
+                    if (no <= 0) break;
+                    const uint32_t sl = k % A.ring;
+                    if constexpr (LV > 0) {
+                        ok = wait_or_abort(raw_full + sl, (k / A.ring) & 1, abort_f, A.wait_clocks);
+                        if (!ok) break;
+                    }
+                    ++k;
+#pragma unroll 1
+                    for (int oc = 0; oc < no; ++oc) {
+                        const int o = o0 + oc;
+                        unsigned char* dst = bt + (size_t)(16 * (o >> 1) + (o & 1)) * sbo;
+                        const uint32_t* row = raw_s + sl * piece_words + (8 * oc) * segw + row_off;
+                        if constexpr (LV == 0) {
+                            const uint32_t tile = t0 + (o >> 1), b = tile / tiles_x, cx = tile - b * tiles_x;
+                            row = src + (((size_t)b * 16 + 8 * (o & 1) + r) * A.cw + 8 * cx + c) * L;
                         }
-                        const uint32_t* row = LV > 0 ? raw_s + sl * piece_words + row_off : gsrc + (size_t)pc * A.rp * A.cw * L;
                         // a batch's loads before its stores: the compiler must assume that they alias
 #pragma unroll 1
-                        for (int g = g0; g < groups; g += 4 * gstep) {
+                        for (int g = 0; g < groups; g += 4) {
                             uint4 v[4];
 #pragma unroll
                             for (int u = 0; u < 4; ++u) {
                                 // (past the row's end: its first group, not stored)
-                                const int l = g + u * gstep < groups ? 4 * (g + u * gstep) : 0;
+                                const int l = g + u < groups ? 4 * (g + u) : 0;
                                 if constexpr (LV == 4) {
                                     v[u] = *reinterpret_cast<const uint4*>(row + l);
                                 } else if constexpr (LV == 2) {
@@ -267,12 +277,12 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
                             }
 #pragma unroll
                             for (int u = 0; u < 4; ++u)
-                                if (g + u * gstep < groups) *reinterpret_cast<uint4*>(dst + (g + u * gstep) * 128) = v[u];
+                                if (g + u < groups) *reinterpret_cast<uint4*>(dst + (g + u) * 128) = v[u];
                         }
-                        if constexpr (LV > 0) {
-                            fence_smem_to_async();  // the reads above, before the slot's next copy
-                            mbar_arrive(raw_empty + sl);
-                        }
+                    }
+                    if constexpr (LV > 0) {
+                        fence_smem_to_async();  // the reads above, before the slot's next copy
+                        mbar_arrive(raw_empty + sl);
                     }
                 }
                 fence_smem_to_async();
@@ -358,7 +368,7 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
 }
 
 size_t dec16_smem(const Dec16Args& A) {
-    return (size_t)A.a_bytes + (size_t)A.nb_buf * A.q * TC_M * A.kb + (size_t)A.ring * A.rp * A.segw * 4 +
+    return (size_t)A.a_bytes + (size_t)A.nb_buf * A.q * TC_M * A.kb + (size_t)A.ring * A.piece_octets * 8 * A.segw * 4 +
            (size_t)15 * A.KP * 8 + (9 + 2 * DEC16_MAX_RING) * 8 + 16;
 }
 

@@ -606,8 +606,8 @@ bool Engine::make_dec_blocks() {
 }
 
 // Shape of the fused decomposition: at most 128 primes (TMEM lanes), their constant image beside
-// the operand tile and at least two raw pieces; two operand buffers and pieces of 8 rows where
-// they fit.  False where none fits.
+// the operand tile and at least two raw pieces; two operand buffers where they fit.  False where
+// none fits.
 bool Engine::dec16_shape(Dec16Args& A) const {
     const int K = plan_.K, L = (int)plan_.L;
     if (K > 128 || L > 64) return false;  // L: t0 of dec_reduce stays below 2^32
@@ -623,9 +623,11 @@ bool Engine::dec16_shape(Dec16Args& A) const {
     // pitch of a row segment: 4 words past a multiple of 32, so that the same limb of 8 rows falls
     // on different banks
     A.segw = 8 * L + ((4 - 8 * L) & 31);
+    // the largest pieces (up to a super-tile's 2q octets: each costs the copy and re-layout warps a
+    // round of barriers) of which three are in flight, else two
     for (A.nb_buf = 2; A.nb_buf >= 1; --A.nb_buf)
-        for (A.rp = 8; A.rp >= 2; A.rp /= 2)
-            for (A.ring = DEC16_MAX_RING; A.ring >= 2; --A.ring)
+        for (A.ring = 3; A.ring >= 2; --A.ring)
+            for (A.piece_octets = 2 * A.q; A.piece_octets >= 1; A.piece_octets /= 2)
                 if (dec16_smem(A) <= smem_optin_) return true;
     return false;
 }
@@ -998,6 +1000,7 @@ void Engine::launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s
     // as many tiles per accumulator as the image has lane groups, as long as every SM has work
     A.qrun = A.q;
     while (A.qrun > 1 && A.nops * ((tiles + A.qrun - 1) / A.qrun) < sms) A.qrun /= 2;
+    A.npo = std::min(A.piece_octets, 2 * A.qrun);
     const uint32_t supers = (tiles + A.qrun - 1) / A.qrun;
     launch_dec16(A, std::min(sms, A.nops * supers), smem_dec16_, s, pdl);
 }

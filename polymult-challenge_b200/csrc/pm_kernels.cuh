@@ -102,7 +102,8 @@ struct Dec16Args {
     int a_rows, a_zero;           // rows per constant-byte block, zero rows before its primes
     uint32_t a_bytes;             // the image's size
     int kb, L, q, qrun;           // K bytes; limbs; lane groups of the image; tiles per accumulator used
-    int nb_buf, ring, rp, segw;   // operand buffers; raw pieces in flight; rows and word pitch of a piece
+    int nb_buf, ring;             // operand buffers; raw pieces in flight
+    int piece_octets, npo, segw;  // row octets a piece has room for and takes; word pitch of its rows
     uint32_t N, col0, cw, nbatch;
     int K, KP;
     const uint32_t* p;            // [KP]
