@@ -893,7 +893,7 @@ template <int NB>
 void launch_cols_nb(bool inv, dim3 grid, size_t smem, cudaStream_t s, const DevPlan& P, uint32_t* R, uint32_t col0,
                     int ltc, bool pdl) {
     if (launch_cols_tma<NB>(inv, grid, s, P, R, col0, ltc, pdl)) return;
-    if (NB == 4 && ltc >= 1) {
+    if (NB == 4 && ltc >= 1 && col0 % 2 == 0) {  // its pairs of columns are 8-byte aligned
         const uint32_t pairs = (grid.x << ltc) / 2;
         const cudaError_t e = launch_kernel(inv ? k_ntt_cols16<true> : k_ntt_cols16<false>,
                                             dim3((pairs + 255) / 256, grid.y, grid.z), dim3(256), 0, s, pdl, P, R, col0,

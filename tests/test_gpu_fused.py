@@ -70,10 +70,10 @@ def test_fused_form_equals_plain_form(N, W, count, off):
 
 
 @pytest.mark.parametrize("body", [1, 4, 16])
-@pytest.mark.parametrize("N,W", [(512, 200), (4096, 300)])
+@pytest.mark.parametrize("N,W", [(512, 200), (1024, 64), (4096, 300)])
 def test_host_chunks_of_any_width(N, W, body):
     """Column chunks of whole 8-column tiles run the fused kernels, narrower ones the separate
-    passes; the products are the same."""
+    passes (N = 1024 in sixteenths: two columns from an odd one on); the products are the same."""
     torch = _torch()
     import polymult
     ensure_library()
