@@ -539,13 +539,22 @@ void Engine::setup_host_pipeline() {
     for (auto& s : s_comp_) cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     cuda_check(cudaStreamCreateWithFlags(&s_h2d_, cudaStreamNonBlocking), "stream");
     cuda_check(cudaStreamCreateWithFlags(&s_d2h_, cudaStreamNonBlocking), "stream");
-    // default schedules by operand size (the tuner refines them): a point of a few hundred KB
-    // moves in one chunk each way (its copies take microseconds, each chunk costs a few of set-up
-    // and four launches), a few MB in quarters, larger points in eighths with narrow heads
-    const size_t opb = plan_.coeff_words() * 4;
-    const uint32_t body = opb < (1u << 20) ? 1 : opb < (8u << 20) ? 4 : 8;
-    set_chunk_schedule(std::min<uint32_t>(body, plan_.ncols), std::min<uint32_t>(body, plan_.ncols), 0);
-    set_chunk_schedule(std::min<uint32_t>(body, plan_.ncols), std::min<uint32_t>(body, plan_.ncols), 1);
+    // Default schedules by operand size (the tuner refines them).  Each chunk costs its copies'
+    // set-up and a few launches on the critical path and buys overlap with the transfers: one
+    // chunk each way while the operand is small, and the longer the transfers the finer.  Staged
+    // calls also overlap the host's own copying, so they split earlier.  Measured medians, us:
+    //   staged, one chunk against quarters: 1.0 MB 153 / 188, 2.1 MB 232 / 256, 3.7 MB 376 / 364;
+    //     quarters against eighths: 10.8 MB 796 / 846, 24.6 MB 1829 / 1860, 28.8 MB 1965 / 1941;
+    //   direct, one chunk against (2, 3): 3.7 MB 274 / 288, 5.4 MB 370 / 377, 7.3 MB 488 / 490,
+    //     14.4 MB 912 / 904; (2, 3) against (4, 3): 14.4 MB 904 / 904, 24.6 MB 1535 / 1529,
+    //     28.8 MB 1819 / 1778; eighths: 14.4 MB 945, 28.8 MB 1838.
+    const size_t opb = plan_.coeff_words() * 4, MB = 1u << 20;
+    auto schedule = [&](uint32_t in_body, uint32_t out_body, int kind) {
+        set_chunk_schedule(std::min(in_body, plan_.ncols), std::min(out_body, plan_.ncols), kind);
+    };
+    const uint32_t staged = opb < 3 * MB ? 1 : opb < 26 * MB ? 4 : 8;
+    schedule(staged, staged, 0);
+    schedule(opb < 6 * MB ? 1 : opb < 16 * MB ? 2 : 4, opb < 6 * MB ? 1 : 3, 1);
     cuda_check(cudaEventCreateWithFlags(&ev_fused_, cudaEventDisableTiming), "event");
     // 7 workers by default: they copy while the caller issues a chunk's CUDA calls, and the caller
     // joins them once it is done (8 copying threads at most).  On the 16-CPU B200 hosts measured,
