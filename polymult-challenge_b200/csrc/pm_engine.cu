@@ -1066,6 +1066,20 @@ void Engine::launch_inv(uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaS
 // ---------------------------------------------------------------------------------------
 // device-resident multiply
 // ---------------------------------------------------------------------------------------
+namespace {
+// Whether a call's first launch may be a programmatic one, so that its prologue (tables, TMEM,
+// barriers) runs under whatever kernel the stream holds before it: the kernel reads only the plan's
+// tables before it waits for that kernel's completion, also one that never triggers.  Back to back
+// calls of 4096 x 256 bits: 18.9 -> 16.7 us, of 65536 x 1747 bits: 115.7 -> 111.9.  Not into a
+// capture, where the edge would come from a node that this library does not know.
+bool follows(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st == cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+}  // namespace
+
 void Engine::run_device(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32_t count, cudaStream_t s) {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     if (count == 0) return;
@@ -1077,8 +1091,7 @@ void Engine::run_device(const uint32_t* a, const uint32_t* b, uint32_t* c, uint3
         const uint32_t nb = std::min(g, count - i);
         const uint32_t* ai = a + (size_t)i * cw;
         const uint32_t* bi = b + (size_t)i * cw;
-        // every launch but the call's first follows a kernel of this sequence
-        launch_fwd2(ai, bi, nb, d_ra_, d_rb_, s, i > 0);
+        launch_fwd2(ai, bi, nb, d_ra_, d_rb_, s, i > 0 || follows(s));
         launch_rows_both(d_rb_, d_ra_, nb, s, true, fused());
         launch_inv(d_rb_, all, nb, c + (size_t)i * cw, s, 0, true, fused());
     }
@@ -1150,7 +1163,7 @@ void Engine::run_group(const uint32_t* a, const uint32_t* b, uint32_t* c, uint32
                        cudaStream_t s) const {
     if (nb == 0) return;
     const Chunk all{0, plan_.ncols};
-    launch_fwd2(a, b, nb, ra, rb, s, false);
+    launch_fwd2(a, b, nb, ra, rb, s, follows(s));
     launch_rows_both(rb, ra, nb, s, true, fused());
     launch_inv(rb, all, nb, c, s, 0, true, fused());
     cuda_check(cudaGetLastError(), "kernel launch");

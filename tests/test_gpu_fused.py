@@ -117,3 +117,36 @@ def test_reduction_at_its_carries(N, W, gemm):
             m.multiply_device(da.data_ptr(), db.data_ptr(), c.data_ptr(), 1, s)
             m.sync()
             assert torch.equal(c, db)
+
+
+@pytest.mark.parametrize("N,W", [(512, 300), (512, 3000), (4096, 256)])
+def test_call_between_other_kernels_of_its_stream(N, W):
+    """The first launch of a call may start under the kernel before it: operands written by that
+    kernel, and overwritten by the one after the call, give the products of calls run one by one."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    _, xs = _operands(torch, N, W, 6, 8, 0)
+    _, b = _operands(torch, N, W, 1, 9, 0)
+    s = torch.cuda.current_stream().cuda_stream
+    with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L), gemm="tensor") as m:
+        def run(a, c):
+            m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, s)
+        want = []
+        for i in range(6):
+            c = torch.zeros((N, L), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            run(xs[i], c)
+            m.sync()
+            want.append(c)
+        a, c = torch.zeros_like(xs[0]), torch.zeros_like(xs[0])
+        got = [torch.zeros_like(a) for _ in range(6)]
+        for i in range(6):
+            torch.bitwise_or(xs[i], 0, out=a)
+            run(a, c)
+            torch.bitwise_or(c, 0, out=got[i])
+            a.fill_(-1)
+        m.sync()
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
