@@ -1032,17 +1032,31 @@ struct ColProbeF {
         }
     }
 };
+// Checks the row kernels of the split and has them run with the least shared memory that holds
+// their resident blocks.  A block that starts on an SM just left by a GEMM kernel otherwise runs with
+// that kernel's 200 KB set aside and with the 28 KB of L1 that leaves: the twiddles live in L1
+// (a pass started under the decomposition, N = 65536, W = 1747, us a multiply: 98.4 in launches of 32
+// and 117.2 alone without this, 93.9 and 110.6 with it, 93.9 and 112.0 after a drained launch;
+// 65536 x 3000 bits x 4: 1015 -> 997 us).
 template <int NB>
 struct RowProbeF {
-    static void run() {
-        const void* fns[3] = {(const void*)k_ntt_rows<NB, ROWS_FWD, -1, false>,
-                              (const void*)k_ntt_rows<NB, ROWS_FUSED, -1, false>,
-                              (const void*)k_ntt_rows<NB, ROWS_BOTH, -1, false>};
-        for (const void* f : fns) {
+    template <int MODE>
+    static void probe(int w1) {
+        for (const bool pair : {false, true}) {
+            const void* f = (const void*)row_kernel<NB, MODE>(w1, pair);
             cudaFuncAttributes fa{};
-            const cudaError_t e = cudaFuncGetAttributes(&fa, f);
+            cudaError_t e = cudaFuncGetAttributes(&fa, f);
+            if (e == cudaSuccess) {
+                const int kb = (int)((rows_min_blocks(NB, MODE) * (fa.sharedSizeBytes + 1024) + 1023) / 1024);
+                e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, std::min(100, (kb * 100 + 227) / 228));
+            }
             if (e != cudaSuccess) throw_cuda(e, "NTT kernel image");
         }
+    }
+    static void run(int w1) {
+        probe<ROWS_FWD>(w1);
+        probe<ROWS_FUSED>(w1);
+        probe<ROWS_BOTH>(w1);
     }
 };
 template <int NB>
@@ -1075,7 +1089,7 @@ void ntt_set_smem_limit(int bytes, int w1, int w2) {
 
 void ntt_probe_images(int w1, int w2) {
     if (w1 > 0) dispatch_nb<ColProbeF>(w1, w2);
-    dispatch_rows<RowProbeF>(w2);
+    dispatch_rows<RowProbeF>(w2, w1);
 }
 
 size_t ntt_cols_smem(const DevPlan& P, int ltc) {

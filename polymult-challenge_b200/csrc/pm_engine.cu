@@ -920,25 +920,15 @@ void Engine::launch_cols(bool inv, uint32_t* R, Chunk ch, uint32_t nb, cudaStrea
     launch_ntt_cols(inv, grid, smem, s, dp_, R, ch.col0, ltc, pdl);
 }
 
-// Whether a row pass behind k_dec16 takes the programmatic launch.  Its blocks then start on SMs
-// still set up for k_dec16's 200 KB of shared memory and keep running with the little L1 that
-// leaves (the twiddles live there); after an ordinary launch the SMs are set up for the row pass.
-// Overlap wins while the pass is about three rounds of blocks (N = 32768, W = 868: 45.3 against
-// 47.4 us a multiply), the larger L1 beyond (N = 65536, W = 1747: 124 against 132 us alone, 103
-// against 116 us in launches of 32).
-bool Engine::rows_overlap(uint32_t nb) const {
-    return (uint64_t)nb * plan_.K * plan_.N / 16 <= 3ull * 896 * (uint64_t)num_sms_;
-}
-
 void Engine::launch_rows(bool fused, uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s,
                          const uint32_t* ra_sel, bool pdl, bool pair) const {
     dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl && (!pair || rows_overlap(nb)), pair);
+    launch_ntt_rows(fused, grid, s, dp_, R, RA, ra_sel, pdl, pair);
 }
 
 void Engine::launch_rows_both(uint32_t* R, const uint32_t* RA, uint32_t nb, cudaStream_t s, bool pdl, bool pair) const {
     dim3 grid((plan_.nrows + rpb_ - 1) / rpb_, plan_.K, nb);
-    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl && (!pair || rows_overlap(nb)), pair);
+    launch_ntt_rows(2, grid, s, dp_, R, RA, nullptr, pdl, pair);
 }
 
 void Engine::launch_crt(const uint32_t* R, Chunk ch, uint32_t nb, uint32_t* out, cudaStream_t s, size_t poff,

@@ -172,7 +172,6 @@ class Engine {
     bool crt16_shape(Crt16Args& A) const;
     void make_fused();
     void launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl) const;
-    bool rows_overlap(uint32_t nb) const;
     bool pair_chunks(const std::vector<Chunk>& v) const;
     // (prime block, result-byte block) launches of a CRT too large for one tile
     struct CrtBlock {
