@@ -18,8 +18,8 @@
 // Continuous batching: the caller's thread runs the loop.  Requests join a FIFO queue at
 // their arrival time; whenever a slot is free and the in-flight count allows, the slot takes
 // every queued request up to its capacity -- whatever their resident operand (the fused row
-// kernel reads resident transform sel[z] for batch entry z) -- and launches the batch on its
-// own stream: H2D copies, the five kernels, D2H copies, an event.  Batches of different slots
+// kernel reads resident transform sel[z] for batch entry z) -- and launches the batch: H2D copies,
+// the kernels (three, or five in the separate form), D2H copies, an event.  Batches of different slots
 // overlap on the device and on the copy engines; a slot's requests complete when its event
 // has fired, and the slot takes the next batch at once.  Latency = completion seen by the
 // loop - arrival time.
@@ -33,6 +33,13 @@
 #include <thread>
 
 namespace pm {
+
+// A piece's input at least: its copies must outlast what starting them behind an event costs.  Wall
+// time of a run, us, with pieces of one request / of 4 MB / of 8 MB / of whole batches:
+//   24 requests of 16384 x 1747 bits (3.6 MB each) 2842 / 2739 / 2455 / 2803; 17 of 32768 x 868 bits
+//   (3.7 MB) 1960 / 1793 / 1850 / 2145; 10 of 8192 x 3000 bits (3.1 MB) 993 / 965 / 1026 / 1414;
+//   4 of 65536 x 1747 bits (14.4 MB) 1673 / 1693 / 1705 / 2452.
+constexpr size_t PIECE_BYTES = 8u << 20;
 
 Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint32_t* resident, uint32_t nresident,
                uint64_t hbm_budget, uint32_t max_batch, uint32_t streams, int gemm_request, int device)
@@ -61,6 +68,11 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
         };
         resident_ = dalloc((size_t)nres_ * rw);
         eng_->reserve((size_t)ns * cap_ * P.N);  // a blocked CRT's partials: one region per slot
+        piece_ = (uint32_t)std::max<size_t>(1, (PIECE_BYTES + cw * 4 - 1) / (cw * 4));
+        if (cap_ > piece_) {
+            cuda_check(cudaStreamCreateWithFlags(&s_in_, cudaStreamNonBlocking), "stream");
+            cuda_check(cudaStreamCreateWithFlags(&s_out_, cudaStreamNonBlocking), "stream");
+        }
         slots_.resize(ns);
         for (Slot& s : slots_) {
             cuda_check(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "stream");
@@ -70,6 +82,10 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
             s.out = dalloc((size_t)cap_ * cw);
             s.sel_d = dalloc(cap_);
             s.dig_d = reinterpret_cast<uint64_t*>(dalloc(2 * (size_t)cap_));
+            s.ev_in.resize((cap_ + piece_ - 1) / piece_);
+            s.ev_c.resize(s.ev_in.size());
+            for (cudaEvent_t& e : s.ev_in) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+            for (cudaEvent_t& e : s.ev_c) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
             cuda_check(cudaHostAlloc(&s.sel_h, cap_ * 4, cudaHostAllocDefault), "cudaHostAlloc");
             cuda_check(cudaHostAlloc(&s.dig_h, cap_ * 8, cudaHostAllocDefault), "cudaHostAlloc");
         }
@@ -99,10 +115,18 @@ void Server::release() {
     for (Slot& s : slots_) {
         if (s.stream) cudaStreamDestroy(s.stream);
         if (s.done) cudaEventDestroy(s.done);
+        for (cudaEvent_t e : s.ev_in)
+            if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : s.ev_c)
+            if (e) cudaEventDestroy(e);
         if (s.sel_h) cudaFreeHost(s.sel_h);
         if (s.dig_h) cudaFreeHost(s.dig_h);
     }
     slots_.clear();
+    for (cudaStream_t* st : {&s_in_, &s_out_}) {
+        if (*st) cudaStreamDestroy(*st);
+        *st = nullptr;
+    }
     for (void* p : dev_) cudaFree(p);
     dev_.clear();
     for (void* p : host_) cudaFreeHost(p);
@@ -125,31 +149,59 @@ void Server::host_free(void* p) {
     host_.erase(it);
 }
 
-void Server::launch(Slot& s, const uint32_t* sel, const uint32_t* const* a, uint32_t* const* c, bool digest) {
+// the products of batch entries i0 .. i0 + n - 1, on the slot's stream
+void Server::compute(Slot& s, uint32_t i0, uint32_t n, bool digest) {
     const Plan& P = eng_->plan();
     const size_t cw = P.coeff_words();
+    const Chunk all{0, P.ncols};
+    // after the copies the launches follow one another (each may overlap the previous one's tail)
+    const bool f = eng_->fused();
+    uint32_t* res = s.res + i0 * eng_->residue_words();
+    eng_->launch_fwd(s.in + i0 * cw, all, n, res, s.stream, false, false, f);
+    eng_->launch_rows(true, res, resident_, n, s.stream, s.sel_d + i0, true, f);
+    eng_->launch_inv(res, all, n, s.out + i0 * cw, s.stream, ((size_t)(&s - slots_.data()) * cap_ + i0) * P.N, true, f);
+    if (digest) launch_digest(s.out + i0 * cw, cw, n, s.dig_d + i0, s.stream);
+}
+
+void Server::copy_out(Slot& s, uint32_t i0, uint32_t n, uint32_t* const* c, bool digest, cudaStream_t st) {
+    const size_t cw = eng_->plan().coeff_words();
+    if (digest)
+        cuda_check(cudaMemcpyAsync(s.dig_h + i0, s.dig_d + i0, n * 8, cudaMemcpyDeviceToHost, st), "digest D2H");
+    for (uint32_t i = i0; i < i0 + n; ++i)
+        cuda_check(cudaMemcpyAsync(c[s.reqs[i]], s.out + i * cw, cw * 4, cudaMemcpyDeviceToHost, st), "result D2H");
+}
+
+void Server::launch(Slot& s, const uint32_t* sel, const uint32_t* const* a, uint32_t* const* c, bool digest) {
+    const size_t cw = eng_->plan().coeff_words();
     const uint32_t nb = (uint32_t)s.reqs.size();
     for (uint32_t i = 0; i < nb; ++i) {
         const uint32_t r = s.reqs[i];
         if (sel[r] >= nres_) throw InvalidPoint("request " + std::to_string(r) + ": resident index out of range");
         s.sel_h[i] = sel[r];
-        cuda_check(cudaMemcpyAsync(s.in + i * cw, a[r], cw * 4, cudaMemcpyHostToDevice, s.stream), "request H2D");
     }
-    cuda_check(cudaMemcpyAsync(s.sel_d, s.sel_h, nb * 4, cudaMemcpyHostToDevice, s.stream), "selector H2D");
-    const Chunk all{0, P.ncols};
-    // after the copies the launches follow one another (each may overlap the previous one's tail)
-    const bool f = eng_->fused();
-    eng_->launch_fwd(s.in, all, nb, s.res, s.stream, false, false, f);
-    eng_->launch_rows(true, s.res, resident_, nb, s.stream, s.sel_d, true, f);
-    eng_->launch_inv(s.res, all, nb, s.out, s.stream, (size_t)(&s - slots_.data()) * cap_ * P.N, true, f);
-    if (digest) {
-        launch_digest(s.out, cw, nb, s.dig_d, s.stream);
-        cuda_check(cudaMemcpyAsync(s.dig_h, s.dig_d, nb * 8, cudaMemcpyDeviceToHost, s.stream), "digest D2H");
+    // A batch of several pieces runs as a pipeline: piece k + 1 is copied in while piece k is computed
+    // and piece k - 1 copied out (in one stream, its results waited for all of its inputs).  The pieces
+    // of all slots share one stream per direction: a copy engine takes them in turn anyway.
+    const uint32_t np = (nb + piece_ - 1) / piece_, n = (nb + np - 1) / np;
+    cudaStream_t in = np > 1 ? s_in_ : s.stream, out = np > 1 ? s_out_ : s.stream;
+    for (uint32_t k = 0, i0 = 0; i0 < nb; ++k, i0 += n) {
+        const uint32_t m = std::min(n, nb - i0);
+        for (uint32_t i = i0; i < i0 + m; ++i)
+            cuda_check(cudaMemcpyAsync(s.in + i * cw, a[s.reqs[i]], cw * 4, cudaMemcpyHostToDevice, in), "request H2D");
+        if (k == 0) cuda_check(cudaMemcpyAsync(s.sel_d, s.sel_h, nb * 4, cudaMemcpyHostToDevice, in), "selector H2D");
+        if (np > 1) {
+            cuda_check(cudaEventRecord(s.ev_in[k], in), "record");
+            cuda_check(cudaStreamWaitEvent(s.stream, s.ev_in[k], 0), "wait");
+        }
+        compute(s, i0, m, digest);
+        if (np > 1) cuda_check(cudaEventRecord(s.ev_c[k], s.stream), "record");
     }
-    for (uint32_t i = 0; i < nb; ++i)
-        cuda_check(cudaMemcpyAsync(c[s.reqs[i]], s.out + i * cw, cw * 4, cudaMemcpyDeviceToHost, s.stream),
-                   "result D2H");
-    cuda_check(cudaEventRecord(s.done, s.stream), "record");
+    // (after every launch: a copy into pageable memory holds the host until it is done)
+    for (uint32_t k = 0, i0 = 0; i0 < nb; ++k, i0 += n) {
+        if (np > 1) cuda_check(cudaStreamWaitEvent(out, s.ev_c[k], 0), "wait");
+        copy_out(s, i0, std::min(n, nb - i0), c, digest, out);
+    }
+    cuda_check(cudaEventRecord(s.done, out), "record");
     s.busy = true;
 }
 

@@ -32,6 +32,7 @@ class Server {
     struct Slot {
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;
+        std::vector<cudaEvent_t> ev_in, ev_c;  // a piece's inputs copied; its products computed
         uint32_t* in = nullptr;    // [cap][N][L]
         uint32_t* res = nullptr;   // [cap][K][N]
         uint32_t* out = nullptr;   // [cap][N][L]
@@ -43,6 +44,8 @@ class Server {
         bool busy = false;
     };
     void launch(Slot& s, const uint32_t* sel, const uint32_t* const* a, uint32_t* const* c, bool digest);
+    void compute(Slot& s, uint32_t i0, uint32_t n, bool digest);
+    void copy_out(Slot& s, uint32_t i0, uint32_t n, uint32_t* const* c, bool digest, cudaStream_t st);
     void release();
 
     std::unique_ptr<Engine> eng_;
@@ -50,6 +53,8 @@ class Server {
     uint32_t nres_ = 0;
     uint32_t* resident_ = nullptr;  // [nres][K][N] forward transforms (row-pass output)
     uint32_t max_batch_ = 1, max_inflight_ = 1, cap_ = 1;
+    uint32_t piece_ = 1;                             // requests that are copied and computed together
+    cudaStream_t s_in_ = nullptr, s_out_ = nullptr;  // copies of batches of several pieces
     std::vector<Slot> slots_;
     std::vector<void*> dev_, host_;
 };

@@ -131,3 +131,27 @@ def test_result_digests_match_the_results():
     w2 = want[0].copy()
     w2[N // 2, 3] ^= 1
     assert polymult.digest_host(w2) != polymult.digest_host(want[0])
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+@pytest.mark.parametrize("N,W,nreq", [(16384, 1747, 11), (8192, 3000, 10)])
+def test_batches_in_pieces_equal_alone(N, W, nreq, pinned):
+    """Batches of more than 8 MB are copied and computed in pieces (here of 3 requests, the last ones
+    smaller): the results and their digests are those of requests served alone, from page-locked and
+    from pageable buffers, and again on buffers that the first run has used."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    q, L, res, reqs, sel = _setup(N, W, 2, nreq, 5)
+    want = _alone(torch, N, W, q, L, res, reqs, sel)
+    with polymult.Server(N, W, orc.limbs_of(q, L), res) as srv:
+        a = srv.pinned(nreq) if pinned else np.zeros_like(reqs)
+        c = srv.pinned(nreq) if pinned else np.zeros_like(reqs)
+        for order in (np.arange(nreq), np.arange(nreq)[::-1]):
+            a[:] = reqs[order]
+            c[:] = 0
+            _, st, dig = srv.run(np.zeros(nreq), sel[order], list(a), list(c), digests=True)
+            assert st["requests"] == nreq
+            assert np.array_equal(np.array(c), want[order])
+            for i in range(nreq):
+                assert int(dig[i]) == polymult.digest_host(np.array(c[i]))
