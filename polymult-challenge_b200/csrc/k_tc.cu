@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
             }
             fence_smem_to_async();
             named_sync(1, DEC_LOAD_THREADS);
-            if (threadIdx.x == 0) {
+            if (warp == 0) {  // all of it: the MMAs are issued from a warp-uniform loop
                 const uint32_t nxt = tile + (uint32_t)ring * gridDim.x;
-                if (use_bulk && nxt < ntiles) {  // the ring slot was just consumed
+                if (lane == 0 && use_bulk && nxt < ntiles) {  // the ring slot was just consumed
                     int c2;
                     const uint32_t* s2 = tile_src(nxt, &c2);
                     bulk_g2s_all(raw, s2, (uint32_t)c2 * L * 4, bar_raw + buf);
@@ -189,18 +189,21 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
                     const uint32_t use = (i + (uint32_t)ring) / (uint32_t)ring;  // the slot's next use
                     raw_par = (raw_par & ~(1u << buf)) | ((use & 1u) << buf);
                 }
+                __syncwarp();
+                const uint32_t mine = elect_one();
                 bool ok = *abort_f == 0;
                 if (ok && !b_seen) ok = b_seen = wait_or_abort(bar_b, 0, abort_f, P.wait_clocks);
-                for (int h = 0; h < nhalves && ok; ++h) {
-                    if (i > 0) ok = wait_or_abort(acc_empty + h, (i - 1) & 1, abort_f, P.wait_clocks);
-                    if (!ok) break;
+                for (int h = 0; h < nhalves; ++h) {
+                    if (i > 0) ok = ok && wait_or_abort(acc_empty + h, (i - 1) & 1, abort_f, P.wait_clocks);
+                    if (!__all_sync(0xffffffffu, ok)) break;
                     tc_fence_after();
-                    if (h == 0) issue_gemm_rows(tmem, smem_addr(a_s), smem_addr(b_s), 0, n0, kb);
-                    else issue_gemm_rows(tmem + col1, smem_addr(a_s), smem_addr(b_s), n0, n1, kb);
-                    umma_commit(mma_done + h);
+                    if (h == 0) issue_gemm_rows(mine, tmem, smem_addr(a_s), smem_addr(b_s), 0, n0, kb);
+                    else issue_gemm_rows(mine, tmem + col1, smem_addr(a_s), smem_addr(b_s), n0, n1, kb);
+                    if (mine) umma_commit(mma_done + h);
                     last_commit = h;
                     last_commit_par = i & 1;
                 }
+                __syncwarp();
             }
         }
     } else {
@@ -483,7 +486,8 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const u
                 }
                 fence_smem_to_async();
                 named_sync(1, CRT_PROD_THREADS);
-                if (threadIdx.x == 0) {
+                if (warp == 0) {  // all of it: the MMAs are issued from a warp-uniform loop
+                    const uint32_t mine = elect_one();
                     bool ok = *S.abort == 0;
                     if (ok && !b_seen) ok = b_seen = wait_or_abort(bar_b, 0, S.abort, P.wait_clocks);
                     if (ok && pbs.n) {
@@ -494,24 +498,25 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const u
                         if (ok && pb == 0 && use_of(i) > 0)
                             ok = wait_or_abort(acc_empty + b, (use_of(i) - 1) & 1, S.abort, P.wait_clocks);
                     }
-                    if (ok) {
+                    if (__all_sync(0xffffffffu, ok)) {
                         tc_fence_after();
                         const uint32_t acc = tmem + (uint32_t)b * AS;
                         // MMA N is at most 256: a wider accumulator takes two row ranges of B
                         const int n_lo = min(nrows_b, 256);
-                        issue_gemm_rows(acc, smem_addr(S.a), smem_addr(S.b), 0, n_lo, kbb, pb > 0);
+                        issue_gemm_rows(mine, acc, smem_addr(S.a), smem_addr(S.b), 0, n_lo, kbb, pb > 0);
                         if (nrows_b > 256)
-                            issue_gemm_rows(acc + 256, smem_addr(S.a), smem_addr(S.b), 256, nrows_b - 256, kbb, pb > 0);
+                            issue_gemm_rows(mine, acc + 256, smem_addr(S.a), smem_addr(S.b), 256, nrows_b - 256, kbb, pb > 0);
                         if (pbs.n) {
-                            umma_commit(ab_free);
+                            if (mine) umma_commit(ab_free);
                             ++ab_commits;
                         }
                         if (last) {
-                            umma_commit(mma_done + b);
+                            if (mine) umma_commit(mma_done + b);
                             ++issued;
                         }
                     }
-                    if (last) mbar_arrive(v_ready + b);  // releases this tile's partial sums
+                    __syncwarp();
+                    if (last && lane == 0) mbar_arrive(v_ready + b);  // releases this tile's partial sums
                 }
             }
         }

@@ -22,17 +22,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, unsigned bytes, s32 accumulate; one thread.
-__device__ __forceinline__ void umma_u8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
 // One lane of a converged warp.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t e;
@@ -44,7 +33,8 @@ __device__ __forceinline__ uint32_t elect_one() {
     return e;
 }
 
-// umma_u8 by the lane with `mine` set, called by a whole converged warp: the loop around it then is
+// D[tmem] (+)= A[smem] * B[smem]^T, unsigned bytes, s32 accumulate, issued by the lane with `mine`
+// set and called by a whole converged warp: the loop around it then is
 // warp-uniform and its descriptors stay in uniform registers.  Issued from a branch of one lane an
 // MMA took ~80 clocks of descriptor moves (k_crt16, k_dec16), more than it runs at N <= 128.
 __device__ __forceinline__ void umma_u8_if(uint32_t mine, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -151,15 +141,16 @@ __device__ __forceinline__ uint32_t idesc_u8(int n) {
 }
 
 // Issues D[:, col0 : col0 + nn) = A * B[row0 : row0 + nn, :]^T into TMEM column col0.
-// acc: the first MMA adds to the accumulator too (a further block of the K dimension)
-__device__ __forceinline__ void issue_gemm_rows(uint32_t tmem_col, uint32_t a_base, uint32_t b_base, int row0, int nn,
+// acc: the first MMA adds to the accumulator too (a further block of the K dimension).  Called by a
+// whole converged warp, whose lane with `mine` set issues (umma_u8_if).
+__device__ __forceinline__ void issue_gemm_rows(uint32_t mine, uint32_t tmem_col, uint32_t a_base, uint32_t b_base, int row0, int nn,
                                                 int kbytes, bool acc = false) {
     const uint32_t sbo = 8u * (uint32_t)kbytes;
     const uint32_t idesc = idesc_u8(nn);
     uint64_t ad = sdesc(a_base, 128u, sbo), bd = sdesc(b_base + (uint32_t)(row0 >> 3) * sbo, 128u, sbo);
 #pragma unroll 4
     for (int kk = 0; kk < kbytes / 32; ++kk, ad += 16, bd += 16)  // 256 bytes in 16-byte units
-        umma_u8(tmem_col, ad, bd, idesc, (kk > 0 || acc) ? 1u : 0u);
+        umma_u8_if(mine, tmem_col, ad, bd, idesc, (kk > 0 || acc) ? 1u : 0u);
 }
 
 // 4-byte asynchronous global -> shared copy (no register staging); cp_async_wait_all waits for
