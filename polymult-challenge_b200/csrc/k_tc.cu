@@ -28,14 +28,15 @@ namespace pm {
 // ----------------------------------------------------------------------------------------
 // Decomposition.  Persistent, warp-specialised, 640 threads; tiles of 128 positions over
 // (batch, npos).
-//   loader group (warps 0-3): thread 0 keeps a ring of raw coefficient tiles filled by
+//   loader group (warps 0-7, two threads a tile row: with four warps and sixteen epilogue warps
+//     65536 x 4000 bits took 84.5 us an operand, now 81.6; with eight and sixteen 83.3): thread 0 keeps a ring of raw coefficient tiles filled by
 //     bulk copies (contiguous cnt*L words each, prefetched two tiles ahead); the group
 //     re-lays the tile out as the K-major A operand once the previous tile's MMAs have read
-//     A; thread 0 then issues the MMAs of the two prime halves -- half h once the epilogue
+//     A; warp 0 then issues the MMAs of the two prime halves -- half h once the epilogue
 //     has released TMEM half h -- with one commit per half (mma_done[h]);
-//   epilogue group (warps 4-19): warp w reads TMEM lane quarter w % 4, the 16-column chunks
-//     congruent to (w - 4) / 4 mod 4, of prime half 0 and then of half 1, and turns four byte
-//     columns into one sum, one REDC and a residue store; all 512 threads arrive on
+//   epilogue group (warps 8-19): warp w reads TMEM lane quarter w % 4, the 16-column chunks
+//     congruent to (w - 8) / 4 mod 3, of prime half 0 and then of half 1, and turns four byte
+//     columns into one sum, one REDC and a residue store; all 384 threads arrive on
 //     acc_empty[h] once they have read half h, so the next tile's half-0 MMA runs while they
 //     read half 1.
 // So tile i's epilogue (the long phase) overlaps tile i+1's copy, relayout and MMAs.  Bounded
@@ -43,7 +44,7 @@ namespace pm {
 // smem: [B image][A tile][raw ring 2 x 128*L words][bars: B, raw 2, mma_done 2, acc_empty 2]
 //       [slot][abort][{p, p^-1 mod 2^32} x KP]
 // ----------------------------------------------------------------------------------------
-constexpr int DEC_LOAD_THREADS = 128;
+constexpr int DEC_LOAD_THREADS = 256;
 constexpr int DEC_EPI_THREADS = RNS_TC_THREADS - DEC_LOAD_THREADS;
 constexpr int DEC_SUBS = DEC_EPI_THREADS / TC_M;  // epilogue warps per TMEM lane quarter
 static_assert(DEC_EPI_THREADS % TC_M == 0, "whole warps per lane quarter");
@@ -139,17 +140,18 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
             // the previous tile's MMAs must have read A (mma_done of its last half)
             if (i > 0) wait_or_abort(mma_done + (nhalves - 1), (i - 1) & 1, abort_f, P.wait_clocks);
             named_sync(1, DEC_LOAD_THREADS);  // raw tile visible to the whole group
-            // re-layout: thread = row mm; 16-byte group g = limbs 4g..4g+3 (zero past L or past
+            // re-layout: thread = half of row mm; 16-byte group g = limbs 4g..4g+3 (zero past L or past
             // cnt).  The full groups unpredicated and unrolled, so that several groups' loads are
-            // in flight at once (a latency chain per group otherwise: this group of 4 warps
-            // shares the SM with the 16 epilogue warps)
+            // in flight at once (a latency chain per group otherwise: these 8 warps
+            // share the SM with the 12 epilogue warps)
             {
-                static_assert(DEC_LOAD_THREADS == TC_M, "one loader thread per tile row");
-                const int mm = threadIdx.x;
+                static_assert(DEC_LOAD_THREADS == 2 * TC_M, "two loader threads per tile row");
+                const int mm = threadIdx.x & (TC_M - 1), g_half = (groups + 7) / 8 * 4;
+                const int g_end = threadIdx.x < TC_M ? min(g_half, groups) : groups;
                 const uint32_t* row = raw + mm * L;
                 unsigned char* dst = a_s + (size_t)(mm >> 3) * sbo + (mm & 7) * 16;
-                const int gfull = mm < cnt ? L / 4 : 0;
-                int g = 0;
+                const int gfull = mm < cnt ? min(L / 4, g_end) : 0;
+                int g = threadIdx.x < TC_M ? 0 : g_half;
                 // four groups' loads before their stores, which the compiler must assume to alias: at
                 // 65536 x 3000 bits 47.5 -> 45.9 us an operand, at 4000 bits 107 -> 97
                 for (; g + 4 <= gfull; g += 4) {
@@ -165,7 +167,7 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
                 for (; g < gfull; ++g)
                     *reinterpret_cast<uint4*>(dst + (size_t)g * 128) =
                         make_uint4(row[4 * g], row[4 * g + 1], row[4 * g + 2], row[4 * g + 3]);
-                for (; g < groups; ++g) {
+                for (; g < g_end; ++g) {
                     const int l0 = 4 * g;
                     uint4 v = make_uint4(0, 0, 0, 0);
                     if (mm < cnt) {

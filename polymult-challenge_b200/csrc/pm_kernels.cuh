@@ -148,7 +148,7 @@ uint64_t digest_host(const uint32_t* x, uint64_t words);
 // the bounded waits made to run out (pm_selftest_wait): 64 threads, one block
 __global__ void k_wait_selftest(uint32_t* status, long long limit);
 constexpr long long kWaitClocks = 2000000000ll;  // DevPlan::wait_clocks
-constexpr int RNS_TC_THREADS = 640;  // 4 loader warps + 16 epilogue warps (4 lane quarters x 2 prime halves x 2 column sets)
+constexpr int RNS_TC_THREADS = 640;  // 8 loader warps + 12 epilogue warps (4 lane quarters x 3 column sets)
 constexpr int CRT_TC_THREADS = 512;  // 256 producers + 256 epilogue threads, two per coefficient each
 size_t rns_tc_smem(const DevPlan& P, int ring = 2);
 size_t crt_tc_smem(const DevPlan& P, bool partial = false);
