@@ -69,10 +69,6 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
         resident_ = dalloc((size_t)nres_ * rw);
         eng_->reserve((size_t)ns * cap_ * P.N);  // a blocked CRT's partials: one region per slot
         piece_ = (uint32_t)std::max<size_t>(1, (PIECE_BYTES + cw * 4 - 1) / (cw * 4));
-        if (cap_ > piece_) {
-            cuda_check(cudaStreamCreateWithFlags(&s_in_, cudaStreamNonBlocking), "stream");
-            cuda_check(cudaStreamCreateWithFlags(&s_out_, cudaStreamNonBlocking), "stream");
-        }
         slots_.resize(ns);
         for (Slot& s : slots_) {
             cuda_check(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "stream");
@@ -82,6 +78,10 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
             s.out = dalloc((size_t)cap_ * cw);
             s.sel_d = dalloc(cap_);
             s.dig_d = reinterpret_cast<uint64_t*>(dalloc(2 * (size_t)cap_));
+            if (cap_ > piece_) {
+                cuda_check(cudaStreamCreateWithFlags(&s.in_stream, cudaStreamNonBlocking), "stream");
+                cuda_check(cudaStreamCreateWithFlags(&s.out_stream, cudaStreamNonBlocking), "stream");
+            }
             s.ev_in.resize((cap_ + piece_ - 1) / piece_);
             s.ev_c.resize(s.ev_in.size());
             for (cudaEvent_t& e : s.ev_in) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
@@ -113,7 +113,8 @@ void Server::release() {
     cudaSetDevice(device_);
     cudaDeviceSynchronize();
     for (Slot& s : slots_) {
-        if (s.stream) cudaStreamDestroy(s.stream);
+        for (cudaStream_t st : {s.stream, s.in_stream, s.out_stream})
+            if (st) cudaStreamDestroy(st);
         if (s.done) cudaEventDestroy(s.done);
         for (cudaEvent_t e : s.ev_in)
             if (e) cudaEventDestroy(e);
@@ -123,10 +124,6 @@ void Server::release() {
         if (s.dig_h) cudaFreeHost(s.dig_h);
     }
     slots_.clear();
-    for (cudaStream_t* st : {&s_in_, &s_out_}) {
-        if (*st) cudaStreamDestroy(*st);
-        *st = nullptr;
-    }
     for (void* p : dev_) cudaFree(p);
     dev_.clear();
     for (void* p : host_) cudaFreeHost(p);
@@ -179,11 +176,15 @@ void Server::launch(Slot& s, const uint32_t* sel, const uint32_t* const* a, uint
         if (sel[r] >= nres_) throw InvalidPoint("request " + std::to_string(r) + ": resident index out of range");
         s.sel_h[i] = sel[r];
     }
-    // A batch of several pieces runs as a pipeline: piece k + 1 is copied in while piece k is computed
-    // and piece k - 1 copied out (in one stream, its results waited for all of its inputs).  The pieces
-    // of all slots share one stream per direction: a copy engine takes them in turn anyway.
-    const uint32_t np = (nb + piece_ - 1) / piece_, n = (nb + np - 1) / np;
-    cudaStream_t in = np > 1 ? s_in_ : s.stream, out = np > 1 ? s_out_ : s.stream;
+    // A large batch with at most half of the slots in flight runs as a pipeline of pieces: piece
+    // k + 1 is copied in while piece k is computed and piece k - 1 copied out (in one stream, its results
+    // waited for all of its inputs).  Behind more batches it runs whole: their copies overlap its own,
+    // and copies behind events are slower to start (65536 x 1747 bits, a queue that never empties: 2970
+    // requests a second always in pieces, 3300 whole).
+    size_t busy = 0;
+    for (const Slot& o : slots_) busy += o.busy;
+    const uint32_t np = 2 * busy <= slots_.size() ? (nb + piece_ - 1) / piece_ : 1, n = (nb + np - 1) / np;
+    cudaStream_t in = np > 1 ? s.in_stream : s.stream, out = np > 1 ? s.out_stream : s.stream;
     for (uint32_t k = 0, i0 = 0; i0 < nb; ++k, i0 += n) {
         const uint32_t m = std::min(n, nb - i0);
         for (uint32_t i = i0; i < i0 + m; ++i)

@@ -31,6 +31,7 @@ class Server {
   private:
     struct Slot {
         cudaStream_t stream = nullptr;
+        cudaStream_t in_stream = nullptr, out_stream = nullptr;  // copies of a batch of several pieces
         cudaEvent_t done = nullptr;
         std::vector<cudaEvent_t> ev_in, ev_c;  // a piece's inputs copied; its products computed
         uint32_t* in = nullptr;    // [cap][N][L]
@@ -54,7 +55,6 @@ class Server {
     uint32_t* resident_ = nullptr;  // [nres][K][N] forward transforms (row-pass output)
     uint32_t max_batch_ = 1, max_inflight_ = 1, cap_ = 1;
     uint32_t piece_ = 1;                             // requests that are copied and computed together
-    cudaStream_t s_in_ = nullptr, s_out_ = nullptr;  // copies of batches of several pieces
     std::vector<Slot> slots_;
     std::vector<void*> dev_, host_;
 };
