@@ -72,9 +72,13 @@ def headline_config():
 #   decomposition: N*L*4 in + K*N*4 out; column/row passes: K*N*4 in + out;
 #   row pass of both operands (forward rows of a and b, pointwise, inverse rows of b; the
 #   device-resident group's "rows_fused" stage, its "rows_a" stage then empty): 2*K*N*4 in +
-#   K*N*4 out; CRT: K*N*4 in + N*L*4 out
-def stage_bytes(stage, N, L, K):
+#   K*N*4 out; CRT: K*N*4 in + N*L*4 out.  The fused form (three launches) decomposes both operands
+#   and runs their column stages in the stage "dec_a" and the inverse ones in "crt"; its other column
+#   and decomposition stages are empty.
+def stage_bytes(stage, N, L, K, fused=False):
     rn, cw = K * N * 4, N * L * 4
+    if fused and stage == "dec_a":
+        return 2 * (cw + rn)
     return {"dec_a": cw + rn, "dec_b": cw + rn, "cols_a": 2 * rn, "cols_b": 2 * rn, "rows_a": 2 * rn,
             "rows_fused": 3 * rn, "cols_inv": 2 * rn, "crt": rn + cw}[stage]
 
@@ -800,7 +804,8 @@ def run_ours(args):
     stages_plain = mp.time_stages(da.data_ptr(), db.data_ptr(), dc2.data_ptr(), B, 3, stream)
     dom = max(stages, key=stages.get)
     K = info["K"]
-    alg = stage_bytes(dom, N, L, K) * B
+    fused = info["launches_per_multiply"] == 3
+    alg = stage_bytes(dom, N, L, K, fused) * B
     peak, peak_kind = measured_peaks()
     achieved = alg / (stages[dom] / 1000.0) / 1e9
     traffic = None

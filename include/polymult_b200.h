@@ -234,8 +234,9 @@ typedef struct pm_pipeline_info {
  * PM_PIPELINE_PINNED: {1, 2, 3, 4, 5, 8, 16} squared on page-locked ones, 3 standing for the
  * chunks 1/2, 1/4, 1/4 of b and 1/4, 1/4, 1/2 of c, and 5 for 1/2, 1/4, 1/8, 1/8 of b and
  * 1/8, 1/8, 1/4, 1/2 of c), keeps the one with the lowest median wall time for that kind of
- * call, and describes it in *out.  Before any tuning the schedules follow the operand size (one
- * chunk below 1 MB, quarters below 8 MB, eighths above).  Synchronous; up to 25
+ * call, and describes it in *out.  Before any tuning the schedules follow the operand size
+ * (staged: one chunk below 3 MB, quarters below 26 MB, eighths above; page-locked: one chunk below
+ * 6 MB, b in 2 and c in the three of "3" below 16 MB, b in 4 above).  Synchronous; up to 25
  * (PM_PIPELINE_PINNED: 49) x (reps + 1) calls. */
 int pm_tune_pipeline(pm_context* ctx, int reps, int flags, pm_pipeline_info* out);
 int pm_get_pipeline(const pm_context* ctx, int flags, pm_pipeline_info* out);

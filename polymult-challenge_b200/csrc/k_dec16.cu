@@ -56,8 +56,10 @@ __device__ __forceinline__ uint32_t dec_reduce(uint32_t r0, uint32_t r1, uint32_
 // every descriptor and address anew) took 19,000 clocks a tile at L = 55, K = 118, against the
 // epilogue's 5,500; the re-layout by branches 6,400 (its warps get the issue slots and the
 // instruction cache that the epilogue leaves); 4-byte cp.async straight into the operand 15,000.
-// Measured 5,800 clocks a tile: 23.6 us for both operands of a multiply at N = 65536, W = 1747
-// (separate decompositions and column passes: 48), the epilogue waiting for 7% of it.
+// Measured 25.5 us for both operands of a multiply at N = 65536, W = 1747 in launches of 32 (separate
+// decompositions and column passes: 48): the epilogue is the limit, two warps an SM sub-partition with
+// 224 registers, which cannot cover one another's waits (issue 51%, multiply-add pipe 57%).  Three
+// groups of 152 registers would store 16 bytes at a time: 44.5 us, half sectors do not merge in L2.
 // A CTA works for one operand (blockIdx.x mod nops), so that its constant image is loaded once and
 // both operands of a multiply share a launch.
 // Few primes (K <= 32 or 64): q = 4 or 2 tiles share an accumulator.  Lanes are split into q groups

@@ -1,7 +1,11 @@
 // pm_engine.cu -- the multiply's runtime: device tables, scratch, launches, and the host
 // pipeline behind the reference-facing call.
 //
-// Device-resident multiply (run_device), per group of G multiplies sharing one launch each:
+// Device-resident multiply (run_device), per group of G multiplies sharing one launch each; the fused
+// form (the 16-row split, where its kernels hold the point):
+//   decompose(a, b) + the first four stages of both -> row pass of both, pointwise, inverse rows
+//   -> the last four inverse stages + CRT -> c
+// the separate form:
 //   decompose(a) -> column pass fwd(a) -> row pass fwd(a)
 //   decompose(b) -> column pass fwd(b) -> fused row pass (fwd b, * a, inv)
 //   column pass inv(b) -> CRT -> c
