@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
             uint32_t sv[8];
             if (got) {
                 tmem_ld8_async(tacc + (uint32_t)A.nz, sv);
-                tmem_wait_ld();
+                tmem_wait_ld_8(sv);
             } else {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) sv[k] = 0u;
@@ -256,6 +256,7 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
             }
             if (l + 4 <= l1) {
                 step(rn, ra);
+                if (got && l < l1) tmem_wait_ld_16(ra);  // a load in flight may not be copied
 #pragma unroll
                 for (int k = 0; k < 16; ++k) rn[k] = ra[k];
             }

@@ -110,6 +110,14 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// tmem_wait_ld tying one 8-column load's registers to the wait
+__device__ __forceinline__ void tmem_wait_ld_8(uint32_t (&a)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
+                 :
+                 : "memory");
+}
+
 // tmem_wait_ld tying one 16-column load's registers to the wait
 __device__ __forceinline__ void tmem_wait_ld_16(uint32_t (&a)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"

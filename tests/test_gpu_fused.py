@@ -150,3 +150,28 @@ def test_call_between_other_kernels_of_its_stream(N, W):
         m.sync()
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("L0", [2, 10, 18, 26, 34, 42, 50])
+def test_every_limb_count(L0):
+    """The CRT's epilogue takes a coefficient's limbs in halves, pairs of four-limb steps, a step left
+    over and up to three limbs behind it: every limb count of the fused form, so that each of these
+    endings is met by both halves."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    N, s = 512, torch.cuda.current_stream().cuda_stream
+    for L in range(L0, min(L0 + 8, 57)):
+        W = 32 * L - 13
+        _, a = _operands(torch, N, W, 2, 3 * L, 0)
+        _, b = _operands(torch, N, W, 2, 3 * L + 1, 0)
+        out = []
+        for gemm in ("tensor", "plain"):
+            c = torch.full((2, N, L), -1, dtype=torch.int32, device="cuda")
+            with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L), gemm=gemm) as m:
+                if gemm == "tensor":
+                    assert m.info()["launches_per_multiply"] == 3
+                m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 2, s)
+                m.sync()
+            out.append(c)
+        assert torch.equal(out[0], out[1]), L
