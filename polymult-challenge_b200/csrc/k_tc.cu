@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
                     }
                     tmem_ld16_async(tcol + (uint32_t)(16 * c16), r[0]);
                     if (two) tmem_ld16_async(tcol + (uint32_t)(16 * (c16 + DEC_SUBS)), r[1]);
-                    tmem_wait_ld();
+                    tmem_wait_ld_2x16(r[0], r[1]);
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         if (u == 1 && !two) break;
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const u
                 if (got) {
                     tmem_ld16_async(tacc + (uint32_t)(16 * c16), r[0]);
                     if (two) tmem_ld16_async(tacc + (uint32_t)(16 * (c16 + 1)), r[1]);
-                    tmem_wait_ld();
+                    tmem_wait_ld_2x16(r[0], r[1]);
                 } else {
 #pragma unroll
                     for (int k = 0; k < 16; ++k) r[0][k] = r[1][k] = 0u;
@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tm(DevPlan P, const u
                 if (got) {
                     tmem_ld16_async(tacc + (uint32_t)(16 * c16), r[0]);
                     if (two) tmem_ld16_async(tacc + (uint32_t)(16 * (c16 + 1)), r[1]);
-                    tmem_wait_ld();
+                    tmem_wait_ld_2x16(r[0], r[1]);
                 } else {
 #pragma unroll
                     for (int k = 0; k < 16; ++k) r[0][k] = r[1][k] = 0u;

@@ -87,7 +87,7 @@ __device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t (&r)[8])
                  : "memory");
 }
 
-// tmem_wait_ld for four 8-column loads, tying their registers to the wait
+// Waits for the warp's TMEM loads: four 8-column loads' registers
 __device__ __forceinline__ void tmem_wait_ld_4x8(uint32_t (&a)[8], uint32_t (&b)[8], uint32_t (&c)[8], uint32_t (&d)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
@@ -99,7 +99,9 @@ __device__ __forceinline__ void tmem_wait_ld_4x8(uint32_t (&a)[8], uint32_t (&b)
 }
 
 // 32 TMEM lanes (this warp's) x 16 consecutive 32-bit columns, without waiting: the registers
-// are valid after tmem_wait_ld().  Issuing several before one wait overlaps their latency.
+// are valid after a wait that names them (tmem_wait_ld_*): until then they may be neither read nor
+// copied, and only the wait's operands keep the compiler from doing so.  Issuing several before one
+// wait overlaps their latency.
 __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -108,9 +110,8 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// tmem_wait_ld tying one 8-column load's registers to the wait
+// one 8-column load's registers
 __device__ __forceinline__ void tmem_wait_ld_8(uint32_t (&a)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
@@ -118,11 +119,22 @@ __device__ __forceinline__ void tmem_wait_ld_8(uint32_t (&a)[8]) {
                  : "memory");
 }
 
-// tmem_wait_ld tying one 16-column load's registers to the wait
+// one 16-column load's registers
 __device__ __forceinline__ void tmem_wait_ld_16(uint32_t (&a)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
                    "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15])
+                 :
+                 : "memory");
+}
+
+// two 16-column loads' registers (where the second was not issued, its values pass through)
+__device__ __forceinline__ void tmem_wait_ld_2x16(uint32_t (&a)[16], uint32_t (&b)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
+                   "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
                  :
                  : "memory");
 }

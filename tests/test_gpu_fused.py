@@ -175,3 +175,28 @@ def test_every_limb_count(L0):
                 m.sync()
             out.append(c)
         assert torch.equal(out[0], out[1]), L
+
+
+@pytest.mark.parametrize("L0", [2, 16, 30, 44, 58, 90])
+def test_every_limb_count_of_the_separate_passes(L0):
+    """The separate decomposition and CRT read their accumulators in pairs of 16-column loads, the
+    second absent at the end of some: limb counts (and with them prime counts) of every remainder, an
+    explicit split, one tile and, past 128 primes, several."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    N, s = 512, torch.cuda.current_stream().cuda_stream
+    for L in range(L0, L0 + 14):
+        W = 32 * L - 13
+        q = orc.limbs_of(_q(N, W), L)
+        _, a = _operands(torch, N, W, 1, 3 * L, 0)
+        _, b = _operands(torch, N, W, 1, 3 * L + 1, 0)
+        c = [torch.full((1, N, L), -1, dtype=torch.int32, device="cuda") for _ in range(2)]
+        with polymult.Batch([(N, W, q, 1, a.data_ptr(), b.data_ptr(), c[0].data_ptr(), 5)]) as batch:
+            assert batch.class_info(0)["gemm"] == "tensor"
+            batch.run(s)
+            batch.sync()
+        with polymult.Multiplier(N, W, q, gemm="plain") as m:
+            m.multiply_device(a.data_ptr(), b.data_ptr(), c[1].data_ptr(), 1, s)
+            m.sync()
+        assert torch.equal(c[0], c[1]), L
