@@ -174,10 +174,11 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
                     __syncwarp();
                 }
             }
-            // MMAs and the image copy must land before this CTA's memory goes away
+            // MMAs and the image copy must land before this CTA's memory goes away, also where the
+            // epilogue, which waits for every MMA, has given up: whatever was issued, behind one more commit
             if (mine) {
                 if (!a_seen) mbar_wait_bounded(bar_a, 0, A.wait_clocks);
-                if (!ok && i > 0) {  // left early: whatever was issued, behind one more commit
+                if (i > 0) {
                     umma_commit(bar_a);
                     mbar_wait_bounded(bar_a, 1, A.wait_clocks);
                 }
