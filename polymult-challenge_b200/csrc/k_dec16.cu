@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
     const int kb = A.kb, q = A.q, qrun = A.qrun, L = A.L;
     const uint32_t op = blockIdx.x % A.nops, me = blockIdx.x / A.nops;
     const uint32_t mates = (gridDim.x - op + A.nops - 1) / A.nops;  // CTAs of this operand
-    const uint32_t* __restrict__ src = A.src[op];
+    const uint32_t* src = A.src[op];
     const uint32_t tiles_x = A.cw / 8;  // tiles per batch entry
     const uint32_t ntiles = tiles_x * A.nbatch;
     const uint32_t nsuper = (ntiles + qrun - 1) / qrun;
@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
                                 } else if constexpr (LV == 1) {
                                     v[u] = make_uint4(row[l], row[l + 1], row[l + 2], row[l + 3]);
                                 } else {
-                                    v[u] = make_uint4(__ldg(row + l), __ldg(row + min(l + 1, L - 1)),
-                                                      __ldg(row + min(l + 2, L - 1)), __ldg(row + min(l + 3, L - 1)));
+                                    v[u] = make_uint4(row[l], row[min(l + 1, L - 1)], row[min(l + 2, L - 1)],
+                                                      row[min(l + 3, L - 1)]);
                                 }
                             }
 #pragma unroll

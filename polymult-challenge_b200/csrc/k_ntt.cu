@@ -332,7 +332,7 @@ __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
 // PAIR: the residues lie in the pair layout (the 16-row split).
 template <int NB, int MODE, int W1, bool PAIR>
 __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)) k_ntt_rows(DevPlan P, uint32_t* __restrict__ R,
-                                                                           const uint32_t* __restrict__ RA,
+                                                                           const uint32_t* RA,
                                                                            const uint32_t* __restrict__ ra_sel) {
     using C = RowCfg<NB>;
     const int w1 = W1 >= 0 ? W1 : P.w1;

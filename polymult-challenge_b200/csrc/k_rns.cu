@@ -65,7 +65,7 @@ __device__ __forceinline__ void mac4x4(uint64_t (&acc)[4][4], uint4 a, uint4 b) 
 }  // namespace
 
 // smem: [raw TM x L][digits DP x TM][table DP x KP if tab_in_smem]
-__global__ void __launch_bounds__(256) k_rns_plain(DevPlan P, const uint32_t* __restrict__ src, ChunkMap C,
+__global__ void __launch_bounds__(256) k_rns_plain(DevPlan P, const uint32_t* src, ChunkMap C,
                                                    uint32_t npos, uint32_t* __restrict__ R, int tab_in_smem) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int TM = DEC_TM;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) k_rns_plain(DevPlan P, const uint32_t* __
             reinterpret_cast<uint4*>(tab_s)[idx] = __ldg(reinterpret_cast<const uint4*>(P.dec24) + idx);
     pdl_trigger();
     pdl_wait();
-    for (int w = threadIdx.x; w < cnt * L; w += blockDim.x) raw[w] = __ldg(s + w);  // contiguous
+    for (int w = threadIdx.x; w < cnt * L; w += blockDim.x) raw[w] = s[w];  // contiguous
     __syncthreads();
     stage_digits<TM>(raw, dig, L, DP, cnt);
     __syncthreads();
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) k_rns_plain(DevPlan P, const uint32_t* __
 }
 
 // smem: [y (K+1) x TM][S TM x DP (u64)][z TM x zs][table (K+1) x DP if tab_in_smem]
-__global__ void __launch_bounds__(256) k_crt_plain(DevPlan P, const uint32_t* __restrict__ R, ChunkMap C,
+__global__ void __launch_bounds__(256) k_crt_plain(DevPlan P, const uint32_t* R, ChunkMap C,
                                                    uint32_t npos, uint32_t* __restrict__ out, int tab_in_smem) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int TM = CRT_TM;

@@ -49,7 +49,7 @@ constexpr int DEC_EPI_THREADS = RNS_TC_THREADS - DEC_LOAD_THREADS;
 constexpr int DEC_SUBS = DEC_EPI_THREADS / TC_M;  // epilogue warps per TMEM lane quarter
 static_assert(DEC_EPI_THREADS % TC_M == 0, "whole warps per lane quarter");
 
-__global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const uint32_t* __restrict__ src, ChunkMap C,
+__global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const uint32_t* src, ChunkMap C,
                                                               uint32_t npos, uint32_t nbatch, uint32_t* __restrict__ R,
                                                               int use_bulk, int ring) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(RNS_TC_THREADS, 1) k_rns_tc(DevPlan P, const u
                 if (wait_or_abort(bar_raw + buf, (i / (uint32_t)ring) & 1, abort_f, P.wait_clocks) && threadIdx.x == 0)
                     raw_pending &= ~(1u << buf);
             } else {
-                for (int w = threadIdx.x; w < cnt * L; w += DEC_LOAD_THREADS) raw[w] = __ldg(s + w);
+                for (int w = threadIdx.x; w < cnt * L; w += DEC_LOAD_THREADS) raw[w] = s[w];
             }
             // the previous tile's MMAs must have read A (mma_done of its last half)
             if (i > 0) wait_or_abort(mma_done + (nhalves - 1), (i - 1) & 1, abort_f, P.wait_clocks);
@@ -329,7 +329,7 @@ __device__ __forceinline__ CrtSmem crt_smem(unsigned char* base, const DevPlan& 
 
 }  // namespace
 
-__global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const uint32_t* __restrict__ R, ChunkMap C,
+__global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tc(DevPlan P, const uint32_t* R, ChunkMap C,
                                                               uint32_t npos, uint32_t nbatch,
                                                               uint32_t* __restrict__ out, CrtPartial part,
                                                               CrtPrimeBlocks pbs) {
@@ -716,7 +716,7 @@ __device__ __forceinline__ CrtTmSmem crt_tm_smem(unsigned char* base, const DevP
 }
 }  // namespace
 
-__global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tm(DevPlan P, const uint32_t* __restrict__ R, ChunkMap C,
+__global__ void __launch_bounds__(CRT_TC_THREADS, 1) k_crt_tm(DevPlan P, const uint32_t* R, ChunkMap C,
                                                               uint32_t npos, uint32_t nbatch,
                                                               uint32_t* __restrict__ out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -976,8 +976,8 @@ size_t crt_tc_smem(const DevPlan& P, bool partial) {
 // partial sums of y_j / p_j) with the |x| < M/8 check, z = partial integer + v T_1, delta fold,
 // - q; 128 threads, one coefficient each, rows staged through shared memory so that loads and
 // stores are coalesced.
-__global__ void __launch_bounds__(TC_M) k_crt_finish(DevPlan P, const uint32_t* __restrict__ zp,
-                                                    const float* __restrict__ sp, uint32_t total,
+__global__ void __launch_bounds__(TC_M) k_crt_finish(DevPlan P, const uint32_t* zp,
+                                                    const float* sp, uint32_t total,
                                                     uint32_t* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = P.L, zl = crt_zl(L), zs = crt_zstride(L);

@@ -152,7 +152,10 @@ __device__ __forceinline__ void bfly_gs_sh(uint32_t& x, uint32_t& y, Tw2 w, uint
 // start while the kernel before it in the stream is still running.  pdl_wait() returns once
 // that kernel has completed and its memory operations are visible (at once after an ordinary
 // launch), so a kernel touches only shared memory, TMEM and the plan's constant tables before
-// it.  pdl_trigger() lets the next kernel's blocks launch, so that their prologues overlap this
+// it.  Data that earlier kernels wrote -- operands (a call's first launch is a programmatic one too),
+// residues, partial sums -- is read by plain loads: non-coherent ones (__ldg, or a const __restrict__
+// parameter) are for data that nothing writes while the kernel runs, and the wait is not documented to
+// refresh what they may find in L1.  pdl_trigger() lets the next kernel's blocks launch, so that their prologues overlap this
 // kernel's tail; it takes effect once every block of this grid has called it or exited.
 // Kernels that allocate TMEM call it only after their own allocation: a dependent block on the
 // same SM could otherwise hold the columns while it waits for this kernel to finish.

@@ -200,3 +200,101 @@ def test_every_limb_count_of_the_separate_passes(L0):
             m.multiply_device(a.data_ptr(), b.data_ptr(), c[1].data_ptr(), 1, s)
             m.sync()
         assert torch.equal(c[0], c[1]), L
+
+
+# aligned operands (bulk copies) and operands off the 16-byte boundary (plain loads), each form's
+# decomposition: with the column stages, in prime blocks, on the CUDA cores
+FORMS = [(512, 300, "tensor"), (512, 3000, "tensor"), (512, 300, "plain")]
+
+
+def _one_by_one(torch, m, a, b, s):
+    c = torch.zeros(a.shape, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, s)
+    m.sync()
+    return c
+
+
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("N,W,gemm", FORMS)
+def test_operands_of_the_kernel_before(N, W, gemm, off):
+    """Operands that the kernel before the call has just written, over older ones that calls have just
+    read, and products that are the next call's operand: those of calls run one by one."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L, s = (W + 31) // 32, torch.cuda.current_stream().cuda_stream
+    _, xs = _operands(torch, N, W, 5, 8, 0)
+    _, b = _operands(torch, N, W, 1, 9, off)
+    bufs = torch.zeros((7, N * L + 64), dtype=torch.int32, device="cuda")
+
+    def at(k):
+        return bufs[k, off:off + N * L].view(N, L)
+    with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L), gemm=gemm) as m:
+        want = [_one_by_one(torch, m, xs[i].clone(), b[0], s) for i in range(5)]
+        chain = want[0]
+        for _ in range(5):
+            c = torch.zeros(N * L + 1, dtype=torch.int32, device="cuda")[off:off + N * L].view(N, L)
+            c.copy_(chain)
+            chain = _one_by_one(torch, m, c, b[0], s)
+        a, got = at(0), []
+        for i in range(5):
+            torch.bitwise_or(xs[i], 0, out=a)
+            c = torch.zeros((N, L), dtype=torch.int32, device="cuda")
+            m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, s)
+            a.fill_(-1)
+            got.append(c)
+        torch.bitwise_or(xs[0], 0, out=a)
+        for k in range(6):
+            m.multiply_device(at(k).data_ptr(), b.data_ptr(), at(k + 1).data_ptr(), 1, s)
+        m.sync()
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)
+        assert torch.equal(at(6), chain)
+
+
+@pytest.mark.parametrize("graph", [None, True, False])
+@pytest.mark.parametrize("N,W,gemm", FORMS)
+def test_operands_of_another_stream(N, W, gemm, graph):
+    """Operands written on another stream and handed over by an event, overwritten there once the call
+    is done: a Multiplier's call, and a batch's run, whose streams wait for an event of their own."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    q = orc.limbs_of(_q(N, W), L)
+    _, xs = _operands(torch, N, W, 6, 8, 0)
+    _, b = _operands(torch, N, W, 1, 9, 0)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    a = torch.zeros((N, L), dtype=torch.int32, device="cuda")
+    c = torch.zeros_like(a)
+    got = [torch.zeros_like(a) for _ in range(6)]
+    with polymult.Multiplier(N, W, q, gemm=gemm) as m:
+        want = [_one_by_one(torch, m, xs[i].clone(), b[0], s1.cuda_stream) for i in range(6)]
+        batch = None
+        if graph is not None:
+            batch = polymult.Batch([(N, W, q, 1, a.data_ptr(), b.data_ptr(), c.data_ptr())], gemm=gemm, graph=graph)
+        torch.cuda.synchronize()
+        written, done = torch.cuda.Event(), torch.cuda.Event()
+        for i in range(6):
+            with torch.cuda.stream(s2):
+                if i:
+                    s2.wait_event(done)
+                a.fill_(-1)
+                torch.bitwise_or(xs[i], 0, out=a)
+                written.record(s2)
+            s1.wait_event(written)
+            if batch is None:
+                m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, s1.cuda_stream)
+            else:
+                batch.run(s1.cuda_stream)
+            with torch.cuda.stream(s1):
+                torch.bitwise_or(c, 0, out=got[i])
+                done.record(s1)
+        torch.cuda.synchronize()
+        if batch is not None:
+            batch.sync()
+            batch.close()
+        m.sync()
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
