@@ -665,13 +665,16 @@ def run_batched(torch, args, local):
     forms = {}
     for c in chosen:
         forms[c["gemm"]] = forms.get(c["gemm"], 0) + 1
+    # the splits that ran: classes whose column stages run inside the GEMM kernels have 16 rows
+    fused = [c["launches_per_multiply"] == 3 for c in chosen]
+    splits = sorted({(4, c["w1"] + c["w2"] - 4) if f else (c["w1"], c["w2"]) for c, f in zip(chosen, fused)})
     out.update({"value": round(total / (ms / 1000.0), 2), "unit": "mults/s", "ms_per_batch": round(ms, 4),
                 "untuned_value": round(total / (ms_default / 1000.0), 2),
                 "sequential_plain_value": round(total / (ms_seq / 1000.0), 2),
                 "speedup_vs_sequential_plain": round(ms_seq / ms, 3),
                 "graph_nodes": inf["graph_nodes"], "kernel_launches": inf["kernel_launches"],
                 "streams": inf["streams"], "scratch_gb": round(inf["scratch_bytes"] / 1e9, 3),
-                "gemm_forms_chosen": forms, "splits_chosen": sorted({(c["w1"], c["w2"]) for c in chosen}),
+                "gemm_forms_chosen": forms, "splits_chosen": splits, "three_launch_classes": sum(fused),
                 "variants_chosen": {"col_tma": sum(1 for c in chosen if c.get("col_tma")),
                                     "crt_a_in_tmem": sum(1 for c in chosen if c.get("crt_tm")),
                                     "launch_groups": sorted({int(c.get("launch_groups", 1)) for c in chosen})},

@@ -158,13 +158,16 @@ typedef struct pm_batch_info {
 } pm_batch_info;
 
 typedef struct pm_batch_class_info {
-    int32_t K, w1, w2;  /* split of separate column and row passes (a class whose column stages run
-                           inside the GEMM kernels: the square split's) */
+    int32_t K, w1, w2;  /* split of separate column and row passes: of a class whose column stages run
+                           inside the GEMM kernels (launches_per_multiply = 3, 16 rows) the one it does
+                           without them, 2^(logN / 2) rows */
     int32_t gemm_form;  /* PM_GEMM_PLAIN or PM_GEMM_TENSOR */
     double tuned_ms;    /* measured ms of the chosen configuration; 0 untuned, -1 from the cache */
-    int32_t col_tma;    /* 1: column passes by the TMA-pipelined kernel (256-row lines), 0: one tile per CTA */
+    int32_t col_tma;    /* 1: column passes by the TMA-pipelined kernel (256-row lines), 0: one tile per CTA, or
+                           none of their own */
     int32_t crt_tm;     /* 1: CRT GEMM with its A operand in tensor memory, 0: in shared memory (or plain) */
     uint32_t launch_groups; /* the class's multiplications run as this many launch groups */
+    int32_t launches_per_multiply; /* kernels of a launch group, as in pm_info */
 } pm_batch_class_info;
 
 int pm_batch_init(const pm_batch_class* classes, uint32_t nclasses, int gemm_form, int flags, int device,

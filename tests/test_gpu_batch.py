@@ -7,6 +7,7 @@ classes, with the C oracle.  Also: graph replays rewrite their outputs, every va
 point and every kernel variant and launch-group count the tuner chooses from gives the same
 bytes, the tuner's cache is written and read back, and line lengths up to
 2^10 (N = 2^18 .. 2^20, the three-phase and two-warp-row NTT forms) against the C oracle."""
+import ctypes
 import os
 
 import numpy as np
@@ -202,3 +203,33 @@ def test_long_lines_against_c_oracle(N, W):
     a = k["a"].cpu().numpy().view(np.uint32)[0]
     b = k["b"].cpu().numpy().view(np.uint32)[0]
     assert np.array_equal(got, c_oracle_mul(N, W, k["q"], a, b))
+
+
+def test_class_info_tells_the_form(tmp_path, monkeypatch):
+    """Three launches (column stages inside the GEMM kernels, which have neither a column pass nor the
+    CRT's operand in tensor memory) or the separate passes: as chosen by default, by an explicit
+    split, by a cache entry, and by the tuner, whose choice a second batch takes from the cache."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("POLYMULT_TUNE_CACHE", str(cache))
+    k = _class(torch, 65536, 1747, 2, seed=90)
+    assert ctypes.sizeof(polymult.PmBatchClassInfo) == 40  # as before the field: callers built then have its room
+
+    def form(w1=-1, **kw):
+        with polymult.Batch([_spec(k, w1)], **kw) as b:
+            ci = b.class_info(0)
+            assert b.info()["kernel_launches"] == ci["launches_per_multiply"] * ci["launch_groups"]
+            return ci["launches_per_multiply"], ci["col_tma"], ci["crt_tm"]
+    assert form() == (3, 0, 0)
+    assert form(8) == (7, 1, 1)
+    assert form(gemm="plain")[0] == 7
+    dev = torch.cuda.get_device_name(0).replace(" ", "_")
+    for w1, want in ((-1, (3, 0, 0)), (8, (7, 1, 1))):
+        cache.write_text("65536 1747 2 %s 0 %d 1.0 1 1 1\n" % (dev, w1))
+        assert form(tune=True) == want
+    cache.write_text("")
+    chosen = form(tune=True)
+    assert len(cache.read_text().splitlines()) == 1
+    assert form(tune=True) == chosen
