@@ -21,8 +21,8 @@
 // class's own operands, CUDA events around 3 repetitions after a warm-up, and keeps the
 // fastest; then, on that engine, the column-pass kernel (TMA pipeline / one tile per CTA), the
 // CRT GEMM's A placement (tensor / shared memory) and 1, 2 or 4 launch groups per class.
-// Results are cached per (N, W, count, device) in a text file ($POLYMULT_TUNE_CACHE, default
-// ~/.cache/polymult_b200/tune.txt).
+// Results are cached per (N, W, count, device, requested form) in a text file
+// ($POLYMULT_TUNE_CACHE, default ~/.cache/polymult_b200/tune.txt).
 #include "pm_batch.h"
 
 #include <algorithm>
@@ -98,13 +98,16 @@ void append_cache(const TuneKey& k, const Choice& c, double ms) {
 // multiplies per launch group when `count` runs in `groups` launch groups
 uint32_t per_group(uint32_t count, uint32_t groups) { return (count + groups - 1) / std::max<uint32_t>(1, groups); }
 
-std::string device_tag(int device) {
+// The device part of a cache key: its name, and the form where a batch asked for one, so that such a
+// batch neither takes nor leaves an entry of the free choice.
+std::string device_tag(int device, int gemm_request) {
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return "unknown";
     std::string s = prop.name;
     for (char& ch : s)
         if (ch == ' ') ch = '_';
-    return s;
+    const char* forms[] = {"", "/plain", "/tensor", "/mixed"};
+    return gemm_request > GEMM_AUTO && gemm_request <= GEMM_MIXED ? s + forms[gemm_request] : s;
 }
 
 }  // namespace
@@ -167,7 +170,7 @@ void Batch::release() {
 // of launch groups (second stage: switched on the chosen engine), and builds the class's
 // engine with them.
 void Batch::choose_configs(int gemm_request) {
-    const std::string dev = device_tag(device_);
+    const std::string dev = device_tag(device_, gemm_request);
     std::map<std::string, Choice> cache;
     if (flags_ & PM_BATCH_TUNE) cache = read_cache();
     // one probe scratch, sized for the largest class, while tuning
@@ -194,16 +197,15 @@ void Batch::choose_configs(int gemm_request) {
                 c.tuned_ms = -1.0;
                 continue;
             }
-            // candidates: splits around logN/2, both forms (tensor only where it fits)
+            // candidates: splits around logN/2, in the requested form or, with the choice left open, in
+            // both (tensor only where it fits)
             int logN = 0;
             while ((1u << logN) < s.N) ++logN;
             std::vector<std::pair<int, int>> cand;
             // AUTO resolves to the tensor-core form, or the mixed one where the CRT does not fit
-            const int forms[2] = {GEMM_AUTO, GEMM_PLAIN};
-            for (int f : forms) {
-                if (gemm_request != GEMM_AUTO && f != gemm_request) continue;
+            for (int f : gemm_request == GEMM_AUTO ? std::vector<int>{GEMM_AUTO, GEMM_PLAIN} : std::vector<int>{gemm_request}) {
                 // (-1: the engine's own choice, the fused 16-row split where it applies)
-                if (f == GEMM_AUTO) cand.push_back({f, -1});
+                if (f == GEMM_AUTO || f == GEMM_TENSOR) cand.push_back({f, -1});
                 for (int w1 = logN / 2 - 1; w1 <= logN / 2 + 1; ++w1)
                     if (w1 >= 0 && w1 <= 10 && logN - w1 >= (logN > 0 ? 1 : 0) && logN - w1 <= 10)
                         cand.push_back({f, w1});

@@ -233,3 +233,31 @@ def test_class_info_tells_the_form(tmp_path, monkeypatch):
     chosen = form(tune=True)
     assert len(cache.read_text().splitlines()) == 1
     assert form(tune=True) == chosen
+
+
+def test_a_requested_form_has_its_own_cache_entry(tmp_path, monkeypatch):
+    """A tuned batch of a requested form runs that form whatever the cache holds of the free choice,
+    finds its own entry again, and leaves the free choice's alone."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("POLYMULT_TUNE_CACHE", str(cache))
+    k = _class(torch, 1024, 300, 2, seed=91)
+    want = _single(torch, k)
+    dev = torch.cuda.get_device_name(0).replace(" ", "_")
+    cache.write_text("1024 300 2 %s 0 4 1.0 0 0 1\n" % dev)
+    for gemm in ("plain", "tensor"):
+        for ms in (0.0, -1.0):  # tuned, then from the cache
+            with polymult.Batch([_spec(k)], gemm=gemm, tune=True) as b:
+                ci = b.class_info(0)
+                assert ci["gemm"] == gemm and min(0.0, ci["tuned_ms"]) == ms
+                k["c"].zero_()
+                b.run(torch.cuda.current_stream().cuda_stream)
+                b.sync()
+            assert np.array_equal(k["c"].cpu().numpy().view(np.uint32), want)
+    lines = cache.read_text().splitlines()
+    assert len(lines) == 3 and all(len(ln.split()) == 10 for ln in lines)
+    with polymult.Batch([_spec(k)], tune=True) as b:
+        ci = b.class_info(0)
+        assert (ci["tuned_ms"], ci["w1"], ci["gemm"]) == (-1.0, 4, "tensor")
