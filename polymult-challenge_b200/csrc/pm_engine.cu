@@ -1205,12 +1205,6 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     ensure_scratch(1);
     const uint32_t nrows = plan_.nrows, ncols = plan_.ncols, L = plan_.L;
     const uint32_t* src[2] = {a, b};
-    // copy jobs of one column chunk: tasks of at least 64 KB of the chunk each (up to 64, one
-    // row at most), taken from the pool's word by whichever thread is free
-    auto tasks_for = [&](uint32_t cw) {
-        const size_t bytes = (size_t)nrows * cw * L * 4;
-        return (uint32_t)std::max<size_t>(1, std::min<size_t>({(size_t)nrows, 64, bytes >> 16}));
-    };
     // operands already in page-locked memory skip the host staging: each column chunk moves
     // with one strided DMA copy (rows of cw * L words at a pitch of ncols * L words); with all
     // three page-locked the call runs the direct-copy schedule
@@ -1253,13 +1247,13 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         uint32_t* dst = h_in_[P] + (size_t)ch.col0 * nrows * L;
         const uint32_t* s = src[P];
         const size_t seg = (size_t)ch.cw * L;
-        const uint32_t nt = tasks_for(ch.cw), rpt = (nrows + nt - 1) / nt;
+        const CopyTasks tasks(nrows, seg);
         job = [=](int t) {
-            const uint32_t r1 = std::min<uint32_t>(nrows, (uint32_t)(t + 1) * rpt);
-            for (uint32_t r = (uint32_t)t * rpt; r < r1; ++r)
-                stream_copy(dst + r * seg, s + ((size_t)r * ncols + ch.col0) * L, seg * 4, ntg);
+            tasks.each((uint32_t)t, [&](uint32_t r, size_t w, size_t n) {
+                stream_copy(dst + r * seg + w, s + ((size_t)r * ncols + ch.col0) * L + w, n * 4, ntg);
+            });
         };
-        pool_->start((int)nt, job);
+        pool_->start((int)tasks.count(), job);
         return true;
     };
     // opens the job that scatters output chunk oc from pinned memory into c
@@ -1267,13 +1261,13 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         const Chunk ch = cout[oc];
         const uint32_t* srcc = h_out_ + (size_t)ch.col0 * nrows * L;
         const size_t seg = (size_t)ch.cw * L;
-        const uint32_t nt = tasks_for(ch.cw), rpt = (nrows + nt - 1) / nt;
+        const CopyTasks tasks(nrows, seg);
         job = [=](int t) {
-            const uint32_t r1 = std::min<uint32_t>(nrows, (uint32_t)(t + 1) * rpt);
-            for (uint32_t r = (uint32_t)t * rpt; r < r1; ++r)
-                stream_copy(c + ((size_t)r * ncols + ch.col0) * L, srcc + r * seg, seg * 4);
+            tasks.each((uint32_t)t, [&](uint32_t r, size_t w, size_t n) {
+                stream_copy(c + ((size_t)r * ncols + ch.col0) * L + w, srcc + r * seg + w, n * 4);
+            });
         };
-        pool_->start((int)nt, job);
+        pool_->start((int)tasks.count(), job);
     };
     uint32_t* dR[2] = {d_ra_, d_rb_};
     using clk = std::chrono::steady_clock;

@@ -18,7 +18,9 @@
 // worker's fetch_add on a finished job's word only moves its ticket further past the count.
 #pragma once
 
+#include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstdint>
 #include <functional>
 #include <thread>
@@ -55,6 +57,29 @@ class HostPool {
     bool open_ = false;  // a job was started and not yet waited for
     uint32_t open_n_ = 0;
     int idle_us_;
+};
+
+// The tasks of a job that copies `rows` segments of `words` 32-bit words: at least 64 KB each and up
+// to 64 of them, whole rows, or parts of a row where the rows are fewer than the tasks wanted (the 16
+// rows of the fused form's chunks).  A task is what one preempted thread holds a job back by, and a
+// chunk's last tasks leave threads idle: a chunk of 3.6 MB is 48 tasks of 75 KB, not 16 of 225 KB.
+struct CopyTasks {
+    uint32_t rows, rows_per = 1, parts = 1;  // rows of a task; tasks of a row
+    size_t words;
+    CopyTasks(uint32_t nrows, size_t nwords) : rows(nrows), words(nwords) {
+        const size_t want = std::max<size_t>(1, std::min<size_t>(64, rows * words * 4 >> 16));
+        if (want < rows) rows_per = (uint32_t)((rows + want - 1) / want);
+        else parts = (uint32_t)(want / rows);
+    }
+    uint32_t count() const { return (rows + rows_per - 1) / rows_per * parts; }
+    // fn(row, first word, words) for every run of task t; parts begin on multiples of 32 bytes
+    template <class Fn>
+    void each(uint32_t t, const Fn& fn) const {
+        const uint32_t q = t % parts, r0 = t / parts * rows_per, r1 = std::min(rows, r0 + rows_per);
+        const size_t w0 = words * q / parts & ~(size_t)7;
+        const size_t w1 = q + 1 == parts ? words : words * (q + 1) / parts & ~(size_t)7;
+        for (uint32_t r = r0; r < r1; ++r) fn(r, w0, w1 - w0);
+    }
 };
 
 // Stress test of HostPool (pm_selftest_host_pool): task sets whose tasks did not each run

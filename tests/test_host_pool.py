@@ -7,9 +7,12 @@ function only after every task of the job has finished.  Four shapes are exercis
 pools (a first call each), long runs of task sets of varying size, task sets that find the
 workers parked on their futex and must wake them, and task sets opened on the workers alone
 (start) and joined by the caller after its own work (wait), as the staging pipeline does."""
+import os
+import subprocess
+
 import pytest
 
-from conftest import ensure_library
+from conftest import PKG, ensure_library
 
 
 def test_first_calls_of_fresh_pools():
@@ -44,3 +47,44 @@ def test_argument_check():
     ensure_library()
     with pytest.raises(polymult.PolymultError):
         polymult.host_pool_selftest(pools=1, runs=1, workers=100)
+
+
+def test_copy_tasks_cover_a_chunk_in_small_pieces(tmp_path):
+    """The tasks of a chunk's copy, whatever its rows: every word once, at least 64 KB and less than
+    twice a 64th of the chunk (or two rows' rounding) each, parts of a row on 32-byte boundaries."""
+    src = tmp_path / "tasks.cpp"
+    src.write_text(r"""
+#include "pm_hostpool.h"
+#include <cstdio>
+#include <cstdlib>
+int main() {
+    const uint32_t rows[] = {1, 2, 4, 16, 32, 64, 128, 256, 1024};
+    const size_t words[] = {1, 7, 8, 63, 1760, 2001, 7040, 28160, 56320, 65001, 225280};
+    for (uint32_t r : rows)
+        for (size_t w : words) {
+            const pm::CopyTasks T(r, w);
+            const size_t total = r * w;
+            std::vector<unsigned char> seen(total, 0);
+            bool ok = T.count() >= 1 && T.count() <= 64;
+            for (uint32_t t = 0; t < T.count(); ++t) {
+                size_t got = 0;
+                T.each(t, [&](uint32_t row, size_t first, size_t n) {
+                    ok = ok && row < r && first % 8 == 0 && first + n <= w;
+                    for (size_t k = 0; ok && k < n; ++k) ++seen[row * w + first + k];
+                    got += n;
+                });
+                ok = ok && (got * 4 + 32 >= 65536 || T.count() == 1 || t + 1 == T.count());
+                const size_t share = std::max<size_t>(total / 64, 16384);
+                ok = ok && got <= 2 * share + 2 * w * (T.parts == 1) + 8;
+            }
+            for (unsigned char x : seen) ok = ok && x == 1;
+            if (!ok) return std::printf("rows %u words %zu: %u tasks\n", r, w, T.count()), 1;
+        }
+    const pm::CopyTasks quarter(16, 56320);  // a quarter of 65536 coefficients of 55 words
+    return quarter.count() == 48 ? 0 : 2;
+}
+""")
+    exe = str(tmp_path / "tasks")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", os.path.join(PKG, "csrc"), str(src), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
