@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
             const int g = rd * CRT16_PROD_WARPS + warp;
             if (tile >= ntiles || g >= G) return;
             const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-            const uint32_t* s = A.R + residue_base(b, A.KP, 4 * g + jj, N) + residue_off(A.col0 + 8 * cx) + c;
+            const int j = min(4 * g + jj, A.K - 1);  // (lanes past the last prime read its residues)
+            const uint32_t* s = A.R + residue_base(b, A.K2, j, N) + residue_off(A.col0 + 8 * cx) + c;
 #pragma unroll
             for (int e = 0; e < 16; ++e) x[e] = s[e * step];
         };
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
             if ((rd == 0 || rd == nr0) && i > 0)  // the previous tile's MMAs have read this block
                 wait_or_abort(a_free + blk, (i - 1) & 1, abort_f, A.wait_clocks);
             if (g < G) {
-                // (primes K .. KP - 1: unset residues against zero B columns)
+                // (primes K .. KP - 1: whatever comes out, against zero B columns)
                 const uint2* tw = tw_s + 4 * g + jj;
                 const uint32_t p = tw[15 * A.KP].x;
                 auto stw = [&](int t) { return StrideTw<true>{tw + ((1 << t) - 1) * A.KP, A.KP, 1 << t}; };

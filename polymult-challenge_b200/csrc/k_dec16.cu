@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(DEC16_THREADS, 1) k_dec16(const __grid_constan
             }
             if (mine && tile < ntiles && *abort_f == 0) {
                 const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-                uint32_t* o = A.R[op] + residue_base(b, A.KP, j, N) + residue_off(A.col0 + 8 * cx);
+                uint32_t* o = A.R[op] + residue_base(b, A.K2, j, N) + residue_off(A.col0 + 8 * cx);
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const uint32_t w[8] = {lo[0][e], lo[1][e], lo[2][e], lo[3][e], hi[0][e], hi[1][e], hi[2][e], hi[3][e]};

@@ -365,7 +365,8 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
     const uint32_t p = P.p[j], pinv = P.pinv[j];
     size_t off;
     if constexpr (PAIR) {
-        auto qo = [&](size_t z) { return residue_base((uint32_t)z, P.KP, j, Nn) + (size_t)hic * (2u << NB); };
+        // (a lambda: written out, rows of 512 and 2048 points spill 8 to 36 bytes)
+        auto qo = [&](size_t z) { return residue_base((uint32_t)z, P.K2, j, Nn) + (size_t)hic * (2u << NB); };
         off = qo(zb);
     }
     else off = ((size_t)zb * P.K + j) * Nn + (size_t)hic * (1u << NB);
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
         uint32_t a[C::E];
         const size_t za = ra_sel ? (size_t)__ldg(ra_sel + zb) : (size_t)zb;
         size_t offa;
-        if constexpr (PAIR) offa = residue_base((uint32_t)za, P.KP, j, Nn) + (size_t)hic * (2u << NB);
+        if constexpr (PAIR) offa = residue_base((uint32_t)za, P.K2, j, Nn) + (size_t)hic * (2u << NB);
         else offa = (za * P.K + j) * Nn + (size_t)hic * (1u << NB);
         row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true, PAIR>(a, const_cast<uint32_t*>(RA + offa), r, active);
 #pragma unroll

@@ -29,6 +29,7 @@ struct DevPlan {
     int D, DP;                // 24-bit digits of a W-bit value (DP: rounded up to a multiple of 4)
     int fold_count;           // CRT folds z -> (z mod 2^W) + (z >> W) delta before the final -q
     int Kr;                   // primes of the residue arrays R[batch][Kr][N] (K except in a prime block)
+    int K2;                   // primes of a batch entry of the pair layout: pair_primes(K)
     uint64_t delta;
     const uint32_t* p;        // [KP]
     const uint32_t* pinv;     // [KP] p^-1 mod 2^32
@@ -73,15 +74,16 @@ struct CrtPrimeBlocks {
 
 // Pair layout of the residue arrays, used by the 16-row split: two primes share 128-byte lines,
 //   word (j, n) of a batch entry = (j / 2) 2N + (n / 16) 32 + (j % 2) 16 + n % 16,
-// KP primes' room per entry.  A kernel that holds a prime per lane (8 columns of one row each)
+// room for the primes rounded up to an even number per entry.  A kernel that holds a prime per lane (8 columns of one row each)
 // touches 16 lines a warp store instead of 32; a row kernel, one prime a block, reads 32
 // elements from 2 lines instead of 1.  With four primes a line the two prime-per-lane kernels were
 // faster (65536 x 1747 bits x 32: decomposition 23.6 against 25.5 us a multiply, CRT 17.4 against
 // 19.8) and the row pass slower (52.1 against 48.8); in sum the pairs gain 1 to 2 % (95.0 -> 93.9;
 // 32768 x 868 bits x 16: 23.4 -> 22.8) except at few large multiplies (x 4: 391 against 398 us).
-// Word of (prime j, coefficient 0) of batch entry b:
-__device__ __forceinline__ size_t residue_base(uint32_t b, int KP, int j, size_t N) {
-    return ((size_t)b * KP + (j & ~1)) * N + (size_t)(j & 1) * 16;
+__host__ __device__ constexpr int pair_primes(int K) { return (K + 1) & ~1; }
+// Word of (prime j, coefficient 0) of batch entry b, K2 = pair_primes(K):
+__device__ __forceinline__ size_t residue_base(uint32_t b, int K2, int j, size_t N) {
+    return ((size_t)b * K2 + (j & ~1)) * N + (size_t)(j & 1) * 16;
 }
 // offset of coefficient n from there; additive over disjoint bits, and a row of ncols >= 16 elements
 // takes 2 ncols words

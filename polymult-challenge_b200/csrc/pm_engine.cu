@@ -220,7 +220,7 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
         // amortise over the group.
         size_t group_words = size_t(256) << 20;
         if (const char* e = std::getenv("POLYMULT_GROUP_WORDS")) group_words = std::max<size_t>(1, std::strtoull(e, nullptr, 10));
-        const size_t per_mult = (size_t)plan_.K * plan_.N;
+        const size_t per_mult = residue_words();
         group_cap_ = (uint32_t)std::max<size_t>(1, std::min<size_t>(256, group_words / std::max<size_t>(1, per_mult)));
         if (crt_blocked_) reserve_crt_partials((size_t)group_cap_ * plan_.N);
         if (opt.host_pipeline) {
@@ -271,6 +271,7 @@ void Engine::upload_tables() {
     d.K = P.K;
     d.Kr = P.K;
     d.KP = P.KP;
+    d.K2 = pair_primes(P.K);
     d.L = (int)P.L;
     d.W = (int)P.W;
     d.D = P.D;
@@ -629,6 +630,7 @@ bool Engine::dec16_shape(Dec16Args& A) const {
     A.L = L;
     A.K = K;
     A.KP = plan_.KP;
+    A.K2 = pair_primes(K);
     A.q = K <= 32 ? 4 : K <= 64 ? 2 : 1;
     A.a_zero = 128 - 128 / A.q;
     A.a_rows = A.q > 1 ? A.a_zero + 128 : (K + 7) / 8 * 8;
@@ -690,6 +692,7 @@ bool Engine::crt16_shape(Crt16Args& A) const {
     A.W = (int)plan_.W;
     A.K = plan_.K;
     A.KP = plan_.KP;
+    A.K2 = pair_primes(plan_.K);
     A.nz = 4 * A.L + 4;
     A.nrows = (A.nz + 6 + 15) / 16 * 16;
     A.kb = (4 * plan_.KP + 31) / 32 * 32;

@@ -114,8 +114,8 @@ class Engine {
     // whether the column stages run inside the GEMM kernels (the 16-row split), and with it the
     // residues of whole operands lie in the pair layout
     bool fused() const { return fused_; }
-    // residue words of one operand's scratch (the pair layout rounds the primes up to fours)
-    size_t residue_words() const { return (size_t)(fused_ ? plan_.KP : plan_.K) * plan_.N; }
+    // residue words of one operand's scratch (the pair layout rounds the primes up to an even number)
+    size_t residue_words() const { return (size_t)(fused_ ? pair_primes(plan_.K) : plan_.K) * plan_.N; }
     bool col_tma_applies() const;
     bool crt_tm_applies() const { return crt_tm_ok_ && !fused_; }
     // the split of the separate column and row passes (a fused engine: the square split's)

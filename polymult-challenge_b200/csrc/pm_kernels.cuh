@@ -105,7 +105,7 @@ struct Dec16Args {
     int nb_buf, ring;             // operand buffers; raw pieces in flight
     int piece_octets, npo, segw;  // row octets a piece has room for and takes; word pitch of its rows
     uint32_t N, col0, cw, nbatch;
-    int K, KP;
+    int K, KP, K2;                // K2: pair_primes(K)
     const uint32_t* p;            // [KP]
     const uint32_t* wsh;          // [KP] floor(2^48 / p)
     const uint2* tw16;            // [15][KP] twiddles 1..15 of every prime
@@ -123,7 +123,7 @@ struct Crt16Args {
     uint32_t* out;
     const unsigned char* img;     // B image: rows = result bytes, then the bytes of sum y_j 2^53 / p_j
     int nrows, nz, kb;            // B rows; rows of result bytes (multiple of 4); K bytes
-    int K, KP, L, W;
+    int K, KP, K2, L, W;          // K2: pair_primes(K)
     uint32_t N, col0, cw, nbatch;
     int fold_count;
     uint64_t delta;

@@ -58,8 +58,8 @@ uint32_t* scratch_address(int device) {
 // The body of pm_run_device_static (pm_capi.cpp maps its exceptions to status codes and
 // restores the caller's current device).
 void run_device_static(Engine& e, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c, cudaStream_t stream) {
-    // (K N and not the pair layout's KP N: both are within the limit or neither, as N divides it by
-    // multiples of four primes)
+    // (K N and not the pair layout's, of an even number of primes: both are within the limit or
+    // neither, as it is an even multiple of N)
     const size_t words = (size_t)e.plan().K * e.plan().N;
     if (2 * words > kStaticScratchWords)
         throw InvalidPoint("pm_run_device_static: K*N = " + std::to_string(words) +

@@ -298,3 +298,32 @@ def test_operands_of_another_stream(N, W, gemm, graph):
         m.sync()
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("N,W", [(2048, 64), (4096, 256), (2048, 868), (2048, 1001)])
+def test_scratch_of_the_pair_layout(monkeypatch, N, W):
+    """Residue scratch: the primes of a multiply, rounded up to an even number, and launch groups that
+    stay within POLYMULT_GROUP_WORDS; the last multiplies of a group hold the same products."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L, count = (W + 31) // 32, 7
+    q = orc.limbs_of(_q(N, W), L)
+    _, a = _operands(torch, N, W, count, 1, 0)
+    _, b = _operands(torch, N, W, count, 2, 0)
+    s = torch.cuda.current_stream().cuda_stream
+    with polymult.Multiplier(N, W, q, gemm="plain") as m:
+        want = torch.zeros_like(a)
+        m.multiply_device(a.data_ptr(), b.data_ptr(), want.data_ptr(), count, s)
+        m.sync()
+        K = m.info()["K"]
+    words = 5 * (K + K % 2) * N + 1
+    monkeypatch.setenv("POLYMULT_GROUP_WORDS", str(words))
+    with polymult.Multiplier(N, W, q) as m:
+        assert m.info()["launches_per_multiply"] == 3
+        assert m.info()["scratch_bytes"] == 2 * 4 * (K + K % 2) * N
+        c = torch.zeros_like(a)
+        m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), count, s)
+        m.sync()
+        assert m.info()["group"] == 5 and m.info()["scratch_bytes"] <= 2 * 4 * words
+    assert torch.equal(c, want)
