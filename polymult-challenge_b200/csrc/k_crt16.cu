@@ -101,12 +101,16 @@ __global__ void __launch_bounds__(CRT16_THREADS, 1) k_crt16(const __grid_constan
         const int c = lane & 7, jj = lane >> 3;
         const size_t N = LN >= 0 ? (size_t)16 << (LN >= 0 ? LN : 0) : A.N;
         const size_t step = N / 16 * 2;  // words between rows
+        // the lane's prime in a group, and in the last one, where lanes past the last pair of primes read
+        // that pair's residues
+        const size_t lane_off = residue_base(0, 4, jj, N) + c;
+        const size_t last_off = residue_base(0, 4, A.K2 % 4 ? jj & 1 : jj, N) + c;
         auto load = [&](uint32_t tile, int rd, uint32_t (&x)[16]) {
             const int g = rd * CRT16_PROD_WARPS + warp;
             if (tile >= ntiles || g >= G) return;
             const uint32_t b = tile / tiles_x, cx = tile - b * tiles_x;
-            const int j = min(4 * g + jj, A.K - 1);  // (lanes past the last prime read its residues)
-            const uint32_t* s = A.R + residue_base(b, A.K2, j, N) + residue_off(A.col0 + 8 * cx) + c;
+            const uint32_t* s = A.R + residue_base(b, A.K2, 4 * g, N) + (g + 1 < G ? lane_off : last_off) +
+                                residue_off(A.col0 + 8 * cx);
 #pragma unroll
             for (int e = 0; e < 16; ++e) x[e] = s[e * step];
         };
