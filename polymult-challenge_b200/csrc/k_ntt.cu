@@ -179,13 +179,16 @@ __device__ __forceinline__ void row_global(uint32_t (&v)[RowCfg<NB>::E], uint32_
     }
 }
 
-// Last-phase twiddles of a row of the 16-row split, from a copy of the table laid out by thread
-// (build_row_twiddles): a stage's 2^t twiddles of thread r are 16-byte pairs at [pair][r], so that
-// a warp reads consecutive pairs, 4 lines a load -- the table's own runs of 2^t entries per thread
-// take up to 16 lines a load.  w[m]: entry m of thread `r` (REV: 2^t - 1 - m).
-template <int LPR, bool REV>
+// Last-phase twiddles of a row of the 16-row split, whose part of the table is laid out by thread
+// (arrange_row_twiddles): a stage's 2^t twiddles of thread r are 16-byte pairs at [pair][r], so that
+// a warp reads consecutive pairs, 4 lines a load -- runs of 2^t entries per thread take up to 16
+// lines a load.  The phase does the stages from T0 on; they hold the same (16 - 2^T0) LPR entries
+// per row in either order.  w[m]: entry m of thread `r` (REV: 2^t - 1 - m).
+template <int LPR, int T0, bool REV>
 struct RowTw {
-    const uint4* base;  // the row's [7][LPR] pairs (stages t = 1, 2, 3), then [LPR] entries of t = 0
+    static constexpr int STRIDE = (16 - (1 << T0)) * LPR / 2;  // uint4 words of a row
+    static constexpr int FIRST = T0 > 0 ? 1 << (T0 - 1) : 1;   // pairs of the stages before the first of pairs, + 1
+    const uint4* base;  // the row's pairs of stages max(T0, 1) .. 3, then (T0 = 0) LPR entries of stage 0
     int r, n;
     __device__ __forceinline__ Tw2 operator[](int m) const {
         if (n == 1) {
@@ -193,16 +196,14 @@ struct RowTw {
             return Tw2{u.x, u.y};
         }
         const int e = REV ? n - 1 - m : m;
-        const uint4 u = __ldg(base + (n / 2 - 1 + (e >> 1)) * LPR + r);
+        const uint4 u = __ldg(base + (n / 2 - FIRST + (e >> 1)) * LPR + r);
         return (e & 1) ? Tw2{u.z, u.w} : Tw2{u.x, u.y};
     }
 };
-// uint4 words of a row's table
-__host__ __device__ constexpr int row_tw_stride(int lpr) { return 7 * lpr + lpr / 2; }
 
 // Forward phases K..NPH-1 of a row (registers in the layout of phase K on entry, of phase
 // NPH-1 on exit).  Stage ls of row hi, group gi uses tw[2^(w1+ls) + hi 2^ls + gi].
-template <int NB, int K, bool PAIR>
+template <int NB, int K, bool TWL>
 __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
                                             const uint2* twj, const uint4* twl, int w1, uint32_t hi, uint32_t p) {
     using C = RowCfg<NB>;
@@ -215,8 +216,9 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        if constexpr (PAIR && K == C::NPH - 1) {
-            auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
+        if constexpr (TWL && K == C::NPH - 1) {
+            using Tw = RowTw<C::LPR, C::t0(K), false>;
+            auto ltw = [&](int t) { return Tw{twl + (size_t)hi * Tw::STRIDE, r, 1 << t}; };
             radix_fwd<C::RB, C::t0(K)>(v, ltw, p);
         } else {
             radix_fwd<C::RB, C::t0(K)>(v, stw, p);
@@ -226,14 +228,14 @@ __device__ __forceinline__ void row_forward(uint32_t (&v)[RowCfg<NB>::E], uint32
             region_sync<NB, K>();
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             __syncwarp();
-            row_forward<NB, K + 1, PAIR>(v, region, rho, r, twj, twl, w1, hi, p);
+            row_forward<NB, K + 1, TWL>(v, region, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
 
 // row_forward on two operands' rows of the same prime and row index (b in v, a in u), each in
 // its own shared-memory region for the exchanges.
-template <int NB, int K, bool PAIR>
+template <int NB, int K, bool TWL>
 __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint32_t (&u)[RowCfg<NB>::E],
                                              uint32_t* region, uint32_t* region_u, int rho, int r, const uint2* twj,
                                              const uint4* twl, int w1, uint32_t hi, uint32_t p) {
@@ -245,8 +247,9 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             const int ls = C::ls(K, t);
             return RunTw<false>{twj + (1u << (w1 + ls)) + (hi << ls) + (hip << t), 1 << t};
         };
-        if constexpr (PAIR && K == C::NPH - 1) {
-            auto ltw = [&](int t) { return RowTw<C::LPR, false>{twl + (size_t)hi * row_tw_stride(C::LPR), r, 1 << t}; };
+        if constexpr (TWL && K == C::NPH - 1) {
+            using Tw = RowTw<C::LPR, C::t0(K), false>;
+            auto ltw = [&](int t) { return Tw{twl + (size_t)hi * Tw::STRIDE, r, 1 << t}; };
             radix_fwd2<C::RB, C::t0(K)>(v, u, ltw, p);
         } else {
             radix_fwd2<C::RB, C::t0(K)>(v, u, stw, p);
@@ -258,7 +261,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
             row_xchg<NB, K + 1, false>(v, region, rho, r);
             row_xchg<NB, K + 1, false>(u, region_u, rho, r);
             __syncwarp();
-            row_forward2<NB, K + 1, PAIR>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
+            row_forward2<NB, K + 1, TWL>(v, u, region, region_u, rho, r, twj, twl, w1, hi, p);
         }
     }
 }
@@ -266,7 +269,7 @@ __device__ __forceinline__ void row_forward2(uint32_t (&v)[RowCfg<NB>::E], uint3
 // Inverse phases K down to 0 (registers in the layout of phase K on entry, phase 0 on exit).
 // The inverse twiddle of (ls, hi, gi) is the forward entry of the mirrored row nrows-1-hi at
 // 2^ls - 1 - gi.
-template <int NB, int K, bool PAIR>
+template <int NB, int K, bool TWL>
 __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32_t* region, int rho, int r,
                                             const uint2* twj, const uint4* twl, int w1, uint32_t hi_m, uint32_t p) {
     using C = RowCfg<NB>;
@@ -279,10 +282,9 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
             const int ls = C::ls(K, t);
             return RunTw<true>{twj + (1u << (w1 + ls)) + (hi_m << ls) + (1u << ls) - ((hip + 1u) << t), 1 << t};
         };
-        if constexpr (PAIR && K == C::NPH - 1) {  // thread LPR - 1 - r's entries of the mirrored row, reversed
-            auto ltw = [&](int t) {
-                return RowTw<C::LPR, true>{twl + (size_t)hi_m * row_tw_stride(C::LPR), C::LPR - 1 - r, 1 << t};
-            };
+        if constexpr (TWL && K == C::NPH - 1) {  // thread LPR - 1 - r's entries of the mirrored row, reversed
+            using Tw = RowTw<C::LPR, C::t0(K), true>;
+            auto ltw = [&](int t) { return Tw{twl + (size_t)hi_m * Tw::STRIDE, C::LPR - 1 - r, 1 << t}; };
             radix_inv<C::RB, C::t0(K)>(v, ltw, p);
         } else {
             radix_inv<C::RB, C::t0(K)>(v, stw, p);
@@ -292,7 +294,7 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
             region_sync<NB, K - 1>();
             row_xchg<NB, K - 1, false>(v, region, rho, r);
             __syncwarp();
-            row_inverse<NB, K - 1, PAIR>(v, region, rho, r, twj, twl, w1, hi_m, p);
+            row_inverse<NB, K - 1, TWL>(v, region, rho, r, twj, twl, w1, hi_m, p);
         }
     }
 }
@@ -329,8 +331,9 @@ __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
 #ifndef POLYMULT_ROW_STATIC
 #define POLYMULT_ROW_STATIC 1
 #endif
-// PAIR: the residues lie in the pair layout (the 16-row split).
-template <int NB, int MODE, int W1, bool PAIR>
+// TWL: the plan's last-phase twiddles lie by thread (an engine of the fused form's 16-row split); PAIR:
+// the residues lie in the pair layout (that form's whole operands and chunks of whole tiles).
+template <int NB, int MODE, int W1, bool TWL, bool PAIR>
 __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)) k_ntt_rows(DevPlan P, uint32_t* __restrict__ R,
                                                                            const uint32_t* RA,
                                                                            const uint32_t* __restrict__ ra_sel) {
@@ -371,9 +374,15 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
     }
     else off = ((size_t)zb * P.K + j) * Nn + (size_t)hic * (1u << NB);
     uint32_t* row = R + off;
-    const uint2* twj = P.tw + (size_t)j * Nn;
+    // The compiler's schedule of the whole kernel follows the shape of these two products (registers and
+    // spills hardly do): with 64-bit ones throughout, rows of 65536 x 1747 bits x 32 take 49.3 us a
+    // multiply, with the table's pointer from a field 48.8, as here 46.8 (16384 x 1747 bits x 8: 12.8
+    // and 12.1); rows of 128 to 512 and of 2048 points are the same in all forms.
+    auto table = [&](uint32_t st) { return P.tw + (size_t)j * st; };
+    // (TWL: the table's entries up to the last phase's)
+    const uint2* twj = table(TWL ? Nn >> (4 - C::t0(C::NPH > 0 ? C::NPH - 1 : 0)) : Nn);
     const uint4* twl = nullptr;
-    if constexpr (PAIR) twl = P.twl + (size_t)j * nrows * row_tw_stride(C::LPR);
+    if constexpr (TWL) twl = P.twl + (size_t)(j * nrows) * RowTw<C::LPR, C::t0(C::NPH - 1), false>::STRIDE;
 
     uint32_t v[C::E];
     pdl_trigger();
@@ -382,13 +391,13 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
     if constexpr (MODE == ROWS_BOTH) {
         uint32_t a[C::E];
         row_global<NB, 0, true, PAIR>(a, const_cast<uint32_t*>(RA + off), r, active);
-        row_forward2<NB, 0, PAIR>(v, a, region, region + REGION_WORDS, rho, r, twj, twl, w1, hic, p);
+        row_forward2<NB, 0, TWL>(v, a, region, region + REGION_WORDS, rho, r, twj, twl, w1, hic, p);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1, PAIR>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_inverse<NB, C::NPH - 1, TWL>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
         row_global<NB, 0, false, PAIR>(v, row, r, active);
     } else if constexpr (MODE == ROWS_FUSED) {
-        row_forward<NB, 0, PAIR>(v, region, rho, r, twj, twl, w1, hic, p);
+        row_forward<NB, 0, TWL>(v, region, rho, r, twj, twl, w1, hic, p);
         uint32_t a[C::E];
         const size_t za = ra_sel ? (size_t)__ldg(ra_sel + zb) : (size_t)zb;
         size_t offa;
@@ -397,10 +406,10 @@ __global__ void __launch_bounds__(RowCfg<NB>::THREADS, rows_min_blocks(NB, MODE)
         row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), true, PAIR>(a, const_cast<uint32_t*>(RA + offa), r, active);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = mont_mul(red_once(red_once(a[e], 2 * p), p), v[e], p, pinv);
-        row_inverse<NB, C::NPH - 1, PAIR>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
+        row_inverse<NB, C::NPH - 1, TWL>(v, region, rho, r, twj, twl, w1, nrows - 1 - hic, p);
         row_global<NB, 0, false, PAIR>(v, row, r, active);
     } else {
-        row_forward<NB, 0, PAIR>(v, region, rho, r, twj, twl, w1, hic, p);
+        row_forward<NB, 0, TWL>(v, region, rho, r, twj, twl, w1, hic, p);
         row_global<NB, (C::NPH > 0 ? C::NPH - 1 : 0), false, PAIR>(v, row, r, active);
     }
 }
@@ -556,7 +565,7 @@ __global__ void __launch_bounds__(256, 3) k_ntt_cols2(DevPlan P, uint32_t* __res
     const int j = (int)blockIdx.y;
     const uint32_t p = P.p[j];
     uint32_t* base = R + ((size_t)blockIdx.z * P.K + j) * P.N + col0 + (blockIdx.x * COL2_TC);
-    const uint2* tw = P.tw + (size_t)j * P.N;
+    const uint2* tw = P.tw + (size_t)j * P.tw_stride;
     pdl_trigger();
     for (int k = threadIdx.x; k < NR; k += blockDim.x) {
         const uint2 w = __ldg(tw + k);
@@ -697,7 +706,7 @@ __global__ void __launch_bounds__(ColtCfg<NB>::THREADS, ColtCfg<NB>::MIN_BLOCKS)
                 unsigned char* slot = smem_raw + 128 + (size_t)s * G::SLOT_BYTES;
                 mbar_arrive_expect_tx(full + s, G::SLOT_BYTES);
                 tma_load_2d(slot, &tmap, (int)(col0 + tx * G::TC), (int)(unit << NB), full + s);
-                bulk_g2s(slot + G::TILE_BYTES, P.tw + (size_t)j * P.N, G::NR * 8, full + s);
+                bulk_g2s(slot + G::TILE_BYTES, P.tw + (size_t)j * P.tw_stride, G::NR * 8, full + s);
             }
             // every copy issued into a slot lands before the CTA exits (the latest per slot)
             for (uint32_t q = k > G::STAGES ? k - G::STAGES : 0; q < k; ++q)
@@ -734,7 +743,7 @@ __global__ void __launch_bounds__(256, 3) k_ntt_cols16(DevPlan P, uint32_t* __re
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = (int)blockIdx.y;
     const uint32_t p = P.p[j];
-    const uint2* tw = P.tw + (size_t)j * P.N;
+    const uint2* tw = P.tw + (size_t)j * P.tw_stride;
     const size_t step = P.ncols / 2;
     uint2* g = reinterpret_cast<uint2*>(R + ((size_t)blockIdx.z * P.K + j) * P.N + col0) + x;
     pdl_trigger();
@@ -764,7 +773,7 @@ __global__ void __launch_bounds__(256, NB >= 5 ? 4 : 1) k_ntt_cols(DevPlan P, ui
     const int j = (int)blockIdx.y;
     const uint32_t p = P.p[j];
     uint32_t* base = R + ((size_t)blockIdx.z * P.K + j) * P.N + col0 + ((uint32_t)blockIdx.x << ltc);
-    const uint2* tw = P.tw + (size_t)j * P.N;
+    const uint2* tw = P.tw + (size_t)j * P.tw_stride;
     pdl_trigger();
     for (int k = threadIdx.x; k < NR; k += blockDim.x) {
         const uint2 u = __ldg(tw + k);
@@ -776,30 +785,35 @@ __global__ void __launch_bounds__(256, NB >= 5 ? 4 : 1) k_ntt_cols(DevPlan P, ui
     else col_phases<NB, INV, 0, -1>(tile, tws, base, P.ncols, ltc, p);
 }
 
-// The rows' last-phase twiddles by thread (RowTw), from the plan's table: thread r of row hi takes
-// entries (r << t) .. (r << t) + 2^t - 1 of the row's part of stage logN - 4 + t.
-__global__ void k_build_row_tw(const uint2* __restrict__ tw, uint2* __restrict__ twl, uint32_t N, int lpr, uint32_t total) {
+// The rows' last-phase twiddles by thread (RowTw) from their order in the plan's table: thread r of
+// row hi takes entries (r << t) .. (r << t) + 2^t - 1 of the row's part of stage logN - 4 + t, t from
+// t0 on.
+__global__ void k_arrange_row_tw(const uint2* src, uint2* dst, uint32_t N, int lpr, int t0, uint32_t total) {
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;  // (prime, row, thread)
     if (x >= total) return;
-    const uint32_t r = x % lpr, hi = x / lpr % 16, j = x / lpr / 16;
-    const uint2* src = tw + (size_t)j * N;
-    uint2* dst = twl + (size_t)(x / lpr) * (2 * row_tw_stride(lpr));
-    for (int t = 0; t < 4; ++t)
+    const uint32_t r = x % lpr, hi = x / lpr % 16;
+    src += (size_t)(x / lpr / 16) * N;
+    dst += (size_t)(x / lpr) * (16 - (1 << t0)) * lpr;
+    const int first = t0 > 0 ? 1 << (t0 - 1) : 1;
+    for (int t = t0; t < 4; ++t)
         for (int m = 0; m < (1 << t); ++m) {
             const uint2 w = src[(N >> (4 - t)) + ((hi * lpr) << t) + (r << t) + m];
             if (t == 0) dst[14 * lpr + r] = w;
-            else dst[2 * (((1 << (t - 1)) - 1 + (m >> 1)) * lpr + r) + (m & 1)] = w;
+            else dst[2 * (((1 << (t - 1)) - first + (m >> 1)) * lpr + r) + (m & 1)] = w;
         }
 }
 
-size_t row_tw_words(const DevPlan& P) { return P.w2 >= 5 ? (size_t)P.K * 16 * row_tw_stride(1 << (P.w2 - 4)) : 0; }
+uint32_t row_tw_low(const DevPlan& P) { return P.N >> (4 - (4 - P.w2 % 4) % 4); }
 
-void build_row_twiddles(const DevPlan& P, uint4* twl, cudaStream_t s) {
-    const int lpr = 1 << (P.w2 - 4);
-    const uint32_t total = (uint32_t)P.K * 16 * lpr;
-    const cudaError_t e = launch_kernel(k_build_row_tw, dim3((total + 255) / 256), dim3(256), 0, s, false, P.tw,
-                                        reinterpret_cast<uint2*>(twl), P.N, lpr, total);
-    if (e != cudaSuccess) throw_cuda(e, "launch k_build_row_tw");
+void arrange_row_twiddles(const DevPlan& P, const uint2* src, uint2* low, uint2* by_thread, int primes, cudaStream_t s) {
+    const int lpr = 1 << (P.w2 - 4), t0 = (4 - P.w2 % 4) % 4;
+    const size_t n_low = row_tw_low(P);
+    cudaError_t e = cudaMemcpy2DAsync(low, n_low * sizeof(uint2), src, (size_t)P.N * sizeof(uint2), n_low * sizeof(uint2),
+                                      (size_t)primes, cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) throw_cuda(e, "copy of the twiddles");
+    const uint32_t total = (uint32_t)primes * 16 * lpr;
+    e = launch_kernel(k_arrange_row_tw, dim3((total + 255) / 256), dim3(256), 0, s, false, src, by_thread, P.N, lpr, t0, total);
+    if (e != cudaSuccess) throw_cuda(e, "launch k_arrange_row_tw");
 }
 
 namespace {
@@ -919,17 +933,18 @@ void launch_cols_nb(bool inv, dim3 grid, size_t smem, cudaStream_t s, const DevP
 // the row kernel of a mode for line length 2^NB and the plan's w1: a compile-time w1 for the
 // splits of N = 4096 .. 65536 that the batches and the engine use, else w1 from the plan
 template <int NB, int MODE>
-auto row_kernel(int w1, bool pair) {
-    if constexpr (NB >= 5) {
-        if (pair) return k_ntt_rows<NB, MODE, 4, true>;  // the 16-row split
+auto row_kernel(const DevPlan& P, bool pair) {
+    if constexpr (NB >= 5) {  // the 16-row split of the fused form
+        if (pair) return k_ntt_rows<NB, MODE, 4, true, true>;
+        if constexpr (MODE != ROWS_BOTH) {  // (whole operands are in the pair layout)
+            if (P.twl) return k_ntt_rows<NB, MODE, 4, true, false>;
+        }
     }
-    (void)pair;
     if constexpr (POLYMULT_ROW_STATIC && NB >= 6 && NB <= 8) {
-        if (w1 == NB) return k_ntt_rows<NB, MODE, NB, false>;
-        if (w1 == NB - 1) return k_ntt_rows<NB, MODE, NB - 1, false>;
+        if (P.w1 == NB) return k_ntt_rows<NB, MODE, NB, false, false>;
+        if (P.w1 == NB - 1) return k_ntt_rows<NB, MODE, NB - 1, false, false>;
     }
-    (void)w1;
-    return k_ntt_rows<NB, MODE, -1, false>;
+    return k_ntt_rows<NB, MODE, -1, false, false>;
 }
 
 template <int NB>
@@ -937,9 +952,9 @@ void launch_rows_nb(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint3
                     const uint32_t* ra_sel, bool pdl, bool pair) {
     // grid comes as (row blocks, primes, batch); the static form takes it as (batch, row blocks, primes)
     const dim3 g = POLYMULT_ROW_STATIC ? dim3(grid.z, grid.x, grid.y) : grid;
-    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P.w1, pair)
-                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P.w1, pair)
-                                                             : row_kernel<NB, ROWS_FWD>(P.w1, pair),
+    const cudaError_t e = launch_kernel(mode == ROWS_BOTH    ? row_kernel<NB, ROWS_BOTH>(P, pair)
+                                        : mode == ROWS_FUSED ? row_kernel<NB, ROWS_FUSED>(P, pair)
+                                                             : row_kernel<NB, ROWS_FWD>(P, pair),
                                         g, dim3(RowCfg<NB>::THREADS), 0, s, pdl, P, R, RA, ra_sel);
     if (e != cudaSuccess)
         throw_cuda(e, mode == ROWS_BOTH    ? "launch k_ntt_rows<both operands>"
@@ -1042,9 +1057,10 @@ struct ColProbeF {
 template <int NB>
 struct RowProbeF {
     template <int MODE>
-    static void probe(int w1) {
+    static void probe(const DevPlan& P) {
         for (const bool pair : {false, true}) {
-            const void* f = (const void*)row_kernel<NB, MODE>(w1, pair);
+            if (pair && !P.twl) break;
+            const void* f = (const void*)row_kernel<NB, MODE>(P, pair);
             cudaFuncAttributes fa{};
             cudaError_t e = cudaFuncGetAttributes(&fa, f);
             if (e == cudaSuccess) {
@@ -1054,10 +1070,10 @@ struct RowProbeF {
             if (e != cudaSuccess) throw_cuda(e, "NTT kernel image");
         }
     }
-    static void run(int w1) {
-        probe<ROWS_FWD>(w1);
-        probe<ROWS_FUSED>(w1);
-        probe<ROWS_BOTH>(w1);
+    static void run(const DevPlan& P) {
+        probe<ROWS_FWD>(P);
+        probe<ROWS_FUSED>(P);
+        probe<ROWS_BOTH>(P);
     }
 };
 template <int NB>
@@ -1088,9 +1104,9 @@ void ntt_set_smem_limit(int bytes, int w1, int w2) {
     if (w1 > 0) dispatch_nb<ColAttrF>(w1, bytes, w2);
 }
 
-void ntt_probe_images(int w1, int w2) {
-    if (w1 > 0) dispatch_nb<ColProbeF>(w1, w2);
-    dispatch_rows<RowProbeF>(w2, w1);
+void ntt_probe_images(const DevPlan& P) {
+    if (P.w1 > 0) dispatch_nb<ColProbeF>(P.w1, P.w2);
+    dispatch_rows<RowProbeF>(P.w2, P);
 }
 
 size_t ntt_cols_smem(const DevPlan& P, int ltc) {

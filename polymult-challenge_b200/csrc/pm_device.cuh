@@ -36,8 +36,10 @@ struct DevPlan {
     const uint32_t* crt_c;    // [KP]
     const uint32_t* crt_cc;   // [KP]
     const float* rcp;         // [KP]
-    const uint2* tw;          // [K][N] {psi^bitrev(k), floor(psi^bitrev(k) 2^32 / p)} (Shoup form)
-    const uint4* twl;         // the 16-row split's last row stages in thread order (RowTw, k_ntt.cu)
+    const uint2* tw;          // [K][tw_stride] {psi^bitrev(k), floor(psi^bitrev(k) 2^32 / p)} (Shoup form), k < N
+    const uint4* twl;         // the fused form: the entries of the row passes' last phase, by thread (RowTw,
+                              // k_ntt.cu), tw holding those before them; else null, and tw all N
+    uint32_t tw_stride;
     const uint32_t* dec24;    // [DP][KP] 2^(24 d) R mod p_j
     const uint32_t* crt24;    // [K+1][DP] 24-bit digits of Q_j = (M/p_j) mod q; row K: of T_1
     const uint32_t* t1;       // [L] T_1 = (-M) mod q

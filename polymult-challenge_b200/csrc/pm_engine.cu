@@ -183,8 +183,10 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
     const bool try16 = opt.w1 < 0 && (gemm_request == GEMM_AUTO || gemm_request == GEMM_TENSOR) && plan_.logN >= 9 &&
                        plan_.logN <= 16 && dec16_shape(dec16_) && crt16_shape(crt16_);
     if (try16) set_split16(plan_);
+    fused_ = try16;
     try {
         upload_tables();
+        if (fused_) make_fused();
         setup_launch_shapes();
         // The tensor-core decomposition runs in prime blocks of at most 128 primes (TMEM holds
         // 4 byte columns per prime) whose B image fits shared memory; the tensor-core CRT needs
@@ -212,7 +214,6 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
         crt_tm_ok_ = crt_tc_ && plan_.KP <= 128 && dp_.crt_nrows <= 256 && dp_.crt_kbytes <= 512 &&
                      crt_tm_smem(dp_) <= smem_optin_;
         crt_tm_ = POLYMULT_CRT_TM && crt_tm_ok_;
-        if (try16) make_fused();
         // multiplies per launch group of run_device: up to POLYMULT_GROUP_WORDS residue words
         // per operand (default 256 Mi: 32 multiplies at N = 65536, W = 1747, 2 GB of residue
         // scratch), at most 256.  Measured there: 8 per group 9081 mults/s, 16 9435, 32 9646 --
@@ -284,7 +285,9 @@ void Engine::upload_tables() {
     d.crt_c = dev_upload(dev_allocs_, P.crt_c, tb);
     d.crt_cc = dev_upload(dev_allocs_, P.crt_cc, tb);
     d.rcp = dev_upload(dev_allocs_, P.rcp, tb);
-    d.tw = reinterpret_cast<const uint2*>(dev_upload(dev_allocs_, P.tw, tb));
+    d.tw_stride = P.N;
+    if (fused_) upload_row_twiddles();
+    else d.tw = reinterpret_cast<const uint2*>(dev_upload(dev_allocs_, P.tw, tb));
     d.dec24 = dev_upload(dev_allocs_, P.dec24, tb);
     d.crt24 = dev_upload(dev_allocs_, P.crt24, tb);
     d.t1 = dev_upload(dev_allocs_, P.t1, tb);
@@ -303,6 +306,33 @@ void Engine::upload_tables() {
     d.wait_clocks = kWaitClocks;
     // POLYMULT_COL_TMA=0: the column passes keep the one-tile-per-CTA kernels
     d.col_tma = !(std::getenv("POLYMULT_COL_TMA") && std::getenv("POLYMULT_COL_TMA")[0] == '0');
+}
+
+// The twiddles of the 16-row split: one table of K N entries, as elsewhere, but in two parts (DevPlan);
+// through a buffer of a few primes' (16 MB).
+void Engine::upload_row_twiddles() {
+    const size_t N = plan_.N;
+    const int step = std::min(plan_.K, std::max(1, (int)((2u << 20) / N)));
+    uint2* t = dev_alloc<uint2>(dev_allocs_, (size_t)plan_.K * N, &table_bytes_);
+    dp_.tw = t;
+    dp_.tw_stride = row_tw_low(dp_);
+    uint2* by_thread = t + (size_t)plan_.K * dp_.tw_stride;
+    dp_.twl = reinterpret_cast<const uint4*>(by_thread);
+    uint2* src = nullptr;
+    cuda_check(cudaMalloc(&src, step * N * sizeof(uint2)), "cudaMalloc");
+    try {
+        for (int j = 0; j < plan_.K; j += step) {
+            const int n = std::min(step, plan_.K - j);
+            cuda_check(cudaMemcpy(src, plan_.tw.data() + (size_t)j * N * 2, n * N * sizeof(uint2), cudaMemcpyHostToDevice),
+                       "upload");
+            arrange_row_twiddles(dp_, src, t + (size_t)j * dp_.tw_stride, by_thread + j * (N - dp_.tw_stride), n, nullptr);
+        }
+        cuda_check(cudaStreamSynchronize(nullptr), "row twiddles");
+    } catch (...) {
+        cudaFree(src);
+        throw;
+    }
+    cudaFree(src);
 }
 
 void Engine::set_status_for_test(uint32_t bits) {
@@ -342,7 +372,7 @@ void Engine::setup_launch_shapes() {
     // Every kernel may use up to the device's opt-in maximum: contexts for different points
     // share these kernels, so a per-point limit set by one context could fail another's launch.
     const int mx = (int)smem_optin_;
-    ntt_probe_images(plan_.w1, plan_.w2);
+    ntt_probe_images(dp_);
     struct Probe {
         const void* fn;
         const char* name;
@@ -677,11 +707,6 @@ void Engine::make_fused() {
     C.tw16 = D.tw16;
     C.status = dp_.status;
     C.wait_clocks = dp_.wait_clocks;
-    uint4* twl = dev_alloc<uint4>(dev_allocs_, row_tw_words(dp_), &table_bytes_);
-    build_row_twiddles(dp_, twl, nullptr);
-    cuda_check(cudaStreamSynchronize(nullptr), "row twiddles");
-    dp_.twl = twl;
-    fused_ = true;
 }
 
 // Shape of the fused CRT: every prime in one tile, the result bytes and the quotient's 6 in at most

@@ -171,6 +171,7 @@ class Engine {
     bool dec16_shape(Dec16Args& A) const;
     bool crt16_shape(Crt16Args& A) const;
     void make_fused();
+    void upload_row_twiddles();
     void launch_dec16_ops(Dec16Args A, Chunk ch, uint32_t nb, cudaStream_t s, bool pdl) const;
     bool pair_chunks(const std::vector<Chunk>& v) const;
     // (prime block, result-byte block) launches of a CRT too large for one tile

@@ -44,14 +44,15 @@ void launch_ntt_cols(bool inv, dim3 grid, size_t smem, cudaStream_t s, const Dev
 // pointwise, inverse stages into R
 void launch_ntt_rows(int mode, dim3 grid, cudaStream_t s, const DevPlan& P, uint32_t* R, const uint32_t* RA,
                      const uint32_t* ra_sel = nullptr, bool pdl = false, bool pair = false);
-// the row passes' last-phase twiddles in thread order (pair layout only): 16-byte words, and their build
-size_t row_tw_words(const DevPlan& P);
-void build_row_twiddles(const DevPlan& P, uint4* twl, cudaStream_t s);
+// The 16-row split's twiddles of `primes` primes, from src [primes][N]: the row_tw_low entries a prime
+// before the row passes' last phase to low, those of that phase, by thread, to by_thread.
+uint32_t row_tw_low(const DevPlan& P);
+void arrange_row_twiddles(const DevPlan& P, const uint2* src, uint2* low, uint2* by_thread, int primes, cudaStream_t s);
 // rows of 2^w2 words per row-pass CTA (grid.x = ceil(nrows / this))
 int ntt_rows_per_cta(int w2);
 // line lengths 2^w1 (columns) and 2^w2 (rows) select the compile-time specialisations
 void ntt_set_smem_limit(int bytes, int w1, int w2);  // max dynamic shared memory of their kernels
-void ntt_probe_images(int w1, int w2);              // throws CudaError if an image cannot load
+void ntt_probe_images(const DevPlan& P);              // throws CudaError if an image cannot load
 size_t ntt_cols_smem(const DevPlan& P, int ltc);
 
 // ---- plain (CUDA-core) RNS decomposition and CRT (k_rns.cu)

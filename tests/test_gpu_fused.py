@@ -327,3 +327,40 @@ def test_scratch_of_the_pair_layout(monkeypatch, N, W):
         m.sync()
         assert m.info()["group"] == 5 and m.info()["scratch_bytes"] <= 2 * 4 * words
     assert torch.equal(c, want)
+
+
+@pytest.mark.parametrize("N,W,body", [(512, 300, 16), (1024, 300, 32), (2048, 300, 32), (4096, 300, 64), (8192, 868, 128)])
+def test_narrow_host_chunks(N, W, body):
+    """The separate passes of an engine whose rows' twiddles lie by thread: host schedules with chunks
+    below a tile's 8 columns, at each row length they reach."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    xa, a = _operands(torch, N, W, 1, 5, 0)
+    xb, b = _operands(torch, N, W, 1, 6, 0)
+    c = torch.zeros((1, N, L), dtype=torch.int32, device="cuda")
+    with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L)) as m:
+        assert m.info()["launches_per_multiply"] == 3 and N // 16 // body < 8
+        m.multiply_device(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, torch.cuda.current_stream().cuda_stream)
+        m.sync()
+        m.set_pipeline(body, body)
+        got = m.multiply(xa[0], xb[0])
+    assert np.array_equal(got, c.cpu().numpy().view(np.uint32)[0])
+
+
+@pytest.mark.parametrize("N,W", [(512, 64), (4096, 868), (65536, 1747)])
+def test_tables_of_the_fused_form(N, W):
+    """The fused form's tables beside the separate passes': its constant images, no second copy of the
+    twiddles."""
+    _torch()
+    import polymult
+    ensure_library()
+    got = []
+    for gemm in ("tensor", "plain"):
+        with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), (W + 31) // 32), gemm=gemm) as m:
+            got.append(m.info())
+    assert got[0]["launches_per_multiply"] == 3
+    # 4 constant bytes x at most 256 rows x at most 256 K bytes for each operand, 256 x 512 for the CRT,
+    # 15 twiddles, p and floor(2^48 / p) of up to 128 primes
+    assert got[0]["table_bytes"] - got[1]["table_bytes"] <= 2 * 4 * 256 * 256 + 256 * 512 + 128 * (15 * 8 + 4)
