@@ -188,7 +188,8 @@ void pm_batch_free(pm_batch* batch);
  * pm_server_host_alloc let the copies run asynchronously).  Continuous batching: whenever one of
  * the server's `streams` slots is free, it takes every queued request up to its capacity,
  * whatever their resident operand, and runs them as one batch while other slots' batches are on
- * the GPU.  Admission: each request in flight holds 8NL + 4KN bytes of device memory; with the
+ * the GPU.  Admission: each request in flight holds 8NL + 4KN bytes of device memory (K rounded up to
+ * an even number where a request runs as three kernels, unless the budget is too small for that); with the
  * resident transforms and tables, the total stays within hbm_budget bytes.  Each result is
  * bit-identical to the same multiplication run alone.  Synchronous; fills latency[i] (seconds,
  * completion - arrival) and *stats. */

@@ -7,11 +7,11 @@
 // forward transform a multiply otherwise recomputes per call: k_row_fwd's output,
 // solve.cu:341-355).  A request multiplies a fresh operand a by one of them, so it costs one
 // decomposition, one forward column pass, the fused row pass (forward a, pointwise with the
-// resident b_k, inverse), the inverse column pass and the CRT -- five kernels instead of
-// eight -- plus its own H2D and D2H copy.
+// resident b_k, inverse), the inverse column pass and the CRT -- five kernels, or three where the
+// GEMM kernels run the column passes -- plus its own H2D and D2H copy.
 //
 // Admission: every in-flight request holds its input, residue and output buffers
-// (8NL + 4KN bytes); the budget minus the resident transforms and the tables bounds the
+// (8NL + 4KN bytes, K rounded up to an even number in the form of three kernels); the budget minus the resident transforms and the tables bounds the
 // requests in flight (max_inflight).  Device memory is carved at start-up into `streams`
 // slots of cap = min(max_batch, max_inflight / streams) requests each.
 //
@@ -49,11 +49,19 @@ Server::Server(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, const uint
     EngineOptions opt;
     opt.host_pipeline = false;
     eng_.reset(new Engine(N, W, L, q, gemm_request, device, opt));
+    auto fixed_bytes = [&] { return (uint64_t)nres_ * eng_->residue_words() * 4 + eng_->table_bytes(); };
+    auto request_bytes = [&] { return (uint64_t)(2 * eng_->plan().coeff_words() + eng_->residue_words()) * 4; };
+    // the fused form's constant images and its even number of primes take a little more than the separate
+    // form, which serves a budget that ends between the two
+    if (eng_->fused() && hbm_budget <= fixed_bytes() + request_bytes()) {
+        opt.w1 = eng_->split_w1();
+        eng_.reset();
+        eng_.reset(new Engine(N, W, L, q, gemm_request, device, opt));
+    }
     try {
         const Plan& P = eng_->plan();
         const size_t cw = P.coeff_words(), rw = eng_->residue_words();
-        const uint64_t fixed = (uint64_t)nres_ * rw * 4 + eng_->table_bytes();
-        const uint64_t per_req = (uint64_t)(2 * cw + rw) * 4;
+        const uint64_t fixed = fixed_bytes(), per_req = request_bytes();
         if (hbm_budget <= fixed + per_req)
             throw InvalidPoint("HBM budget too small: resident operands and tables need " + std::to_string(fixed) +
                                " bytes and one request " + std::to_string(per_req));

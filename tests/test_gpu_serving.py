@@ -155,3 +155,28 @@ def test_batches_in_pieces_equal_alone(N, W, nreq, pinned):
             assert np.array_equal(np.array(c), want[order])
             for i in range(nreq):
                 assert int(dig[i]) == polymult.digest_host(np.array(c[i]))
+
+
+@pytest.mark.parametrize("N,W", [(2048, 64), (4096, 868), (8192, 256)])
+def test_least_budget(N, W):
+    """The least budget: the resident operands, the tables and one request of the separate passes, which
+    serve it where the form of three kernels takes more; a byte less is refused."""
+    torch = _torch()
+    import polymult
+    import workload
+    ensure_library()
+    q = (1 << W) - 2 * N + 1
+    L = (W + 31) // 32
+    ops = workload.uniform_operands(N, W, q, 5, seed=W)
+    res, reqs, sel = ops[:2], ops[2:], np.array([1, 0, 1], dtype=np.uint32)
+    want = _alone(torch, N, W, q, L, res, reqs, sel)
+    with polymult.Multiplier(N, W, orc.limbs_of(q, L), gemm="plain") as m:
+        inf = m.info()
+    need = 2 * inf["K"] * N * 4 + inf["table_bytes"] + (2 * N * L + inf["K"] * N) * 4
+    with polymult.Server(N, W, orc.limbs_of(q, L), res, hbm_budget=need + 1, max_batch=4, streams=2) as srv:
+        got, _, st = _serve(srv, reqs, sel, np.zeros(len(reqs)))
+        assert st["max_inflight"] == st["peak_inflight"] == 1
+        assert np.array_equal(got, want)
+    with pytest.raises(polymult.PolymultError) as ei:
+        polymult.Server(N, W, orc.limbs_of(q, L), res, hbm_budget=need)
+    assert ei.value.code == polymult.PM_ERR_INVALID
