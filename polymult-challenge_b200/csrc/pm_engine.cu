@@ -1256,6 +1256,15 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     for (const Chunk& ch : cin_[kind]) items.push_back({1, ch});
     const int nin = (int)items.size();
 
+    // A small call, one chunk each way, in one stream: both operands copied, then the three launches of
+    // the device-resident call, then the result's copy.  There a's own kernels outlast b's copy, and each
+    // hand-over between streams costs microseconds.  Medians in us, against a's decomposition and rows
+    // under b's copy: page-locked operands of 0.02 MB (2048 x 64 bits) 71.5 -> 56, 0.13 MB (4096 x 256)
+    // 73.6 -> 66.6, 0.23 MB (2048 x 868) 75.5 -> 74, 0.26 MB (4096 x 500) 75.6 -> 76 to 80; pageable
+    // 0.13 MB 83.7 -> 76.9, 0.23 MB 86 -> 81, 0.26 MB 84.1 -> 85.2 and (8192 x 256) 84.4 -> 97.
+    const bool small_call = pair && nin == 2 && nout == 1 && opbytes < (size_t)256 << 10;
+    cudaStream_t h2d = small_call ? s_comp_[0] : s_h2d_, d2h = small_call ? s_comp_[0] : s_d2h_;
+
     // The pool's open copy job.  The workers copy chunk i + 1 (or scatter output chunk oc)
     // while this thread issues chunk i's copies and kernels (12-20 us of API calls per chunk),
     // then joins in with wait(); the guard, declared after the job, waits for it before the
@@ -1311,7 +1320,7 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         cuda_check(cudaEventRecord(trace_ev_[marks.size()], st), "record");
         marks.emplace_back(name, trace_ev_[marks.size()]);
     };
-    mark("start", s_h2d_);
+    mark("start", h2d);
     if (stage_start(0)) pool_->wait();
     t_stage0 = clk::now();
     // the kernels of input item k, once its copy is issued (the copy's event: ev_in_[hi])
@@ -1323,6 +1332,10 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         // that its kernels, the fused row pass and the first output chunk's follow each other
         // in one stream (each launch overlapping the previous kernel's tail)
         const bool last = k + 1 == nin;
+        if (small_call) {
+            if (last) launch_fwd2(d_in_[0], d_in_[1], 1, d_ra_, d_rb_, s_comp_[0], false);
+            return;
+        }
         cudaStream_t sc = last ? s_comp_[0] : s_comp_[k % 3];
         if (last)
             for (int q = na; q < k; ++q) cuda_check(cudaStreamWaitEvent(sc, ev_done_in_[q], 0), "wait");
@@ -1367,13 +1380,12 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
             for (int k = pend; k <= i; ++k) words += (size_t)items[k].second.cw * nrows * L;
             if (direct_in[P])
                 cuda_check(cudaMemcpy2DAsync(d_in_[P] + off, (size_t)c0.cw * L * 4, src[P] + (size_t)c0.col0 * L, pitch,
-                                             (size_t)c0.cw * L * 4, nrows, cudaMemcpyHostToDevice, s_h2d_),
+                                             (size_t)c0.cw * L * 4, nrows, cudaMemcpyHostToDevice, h2d),
                            "H2D");
             else
-                cuda_check(cudaMemcpyAsync(d_in_[P] + off, h_in_[P] + off, words * 4, cudaMemcpyHostToDevice, s_h2d_),
-                           "H2D");
-            cuda_check(cudaEventRecord(ev_in_[i], s_h2d_), "record");
-            mark("h2d" + std::to_string(i), s_h2d_);
+                cuda_check(cudaMemcpyAsync(d_in_[P] + off, h_in_[P] + off, words * 4, cudaMemcpyHostToDevice, h2d), "H2D");
+            if (!small_call) cuda_check(cudaEventRecord(ev_in_[i], h2d), "record");
+            mark("h2d" + std::to_string(i), h2d);
             for (int k = pend; k <= i; ++k) issue_compute(k, i);
             fl_prev = fl_last;
             fl_last = i;
@@ -1385,7 +1397,8 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     }
     // stream 0 has run a's row pass and b's last chunk after the others
     cudaStream_t s0 = s_comp_[0];
-    launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true, pair);
+    if (small_call) launch_rows_both(d_rb_, d_ra_, 1, s0, true, true);
+    else launch_rows(true, d_rb_, d_ra_, 1, s0, nullptr, true, pair);
     if (kind == 0) cuda_check(cudaEventRecord(ev_fused_, s0), "record");
     mark("fused", s0);
     auto issue_out = [&](size_t oc) {
@@ -1399,23 +1412,24 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         if (si != 0) cuda_check(cudaStreamWaitEvent(sc, ev_fused_, 0), "wait");
         // output chunks run on three streams: each gets its own region of the partial buffers
         launch_inv(d_rb_, ch, 1, d_out_ + off, sc, (size_t)ch.col0 * nrows, si == 0, pair);
-        cuda_check(cudaEventRecord(ev_crt_[oc], sc), "record");
         mark("crt" + std::to_string(oc), sc);
-        cuda_check(cudaStreamWaitEvent(s_d2h_, ev_crt_[oc], 0), "wait");
+        if (!small_call) {
+            cuda_check(cudaEventRecord(ev_crt_[oc], sc), "record");
+            cuda_check(cudaStreamWaitEvent(d2h, ev_crt_[oc], 0), "wait");
+        }
         if (direct_out)
             cuda_check(cudaMemcpy2DAsync(c + (size_t)ch.col0 * L, pitch, d_out_ + off, (size_t)ch.cw * L * 4,
-                                         (size_t)ch.cw * L * 4, nrows, cudaMemcpyDeviceToHost, s_d2h_),
+                                         (size_t)ch.cw * L * 4, nrows, cudaMemcpyDeviceToHost, d2h),
                        "D2H");
         else
-            cuda_check(cudaMemcpyAsync(h_out_ + off, d_out_ + off, words * 4, cudaMemcpyDeviceToHost, s_d2h_),
-                       "D2H");
-        cuda_check(cudaEventRecord(ev_out_[oc], s_d2h_), "record");
-        mark("d2h" + std::to_string(oc), s_d2h_);
+            cuda_check(cudaMemcpyAsync(h_out_ + off, d_out_ + off, words * 4, cudaMemcpyDeviceToHost, d2h), "D2H");
+        cuda_check(cudaEventRecord(ev_out_[oc], d2h), "record");
+        mark("d2h" + std::to_string(oc), d2h);
         if (oc + 1 == nout) {
             // device status word -> pinned memory behind the last D2H (s_d2h has waited on every CRT)
-            cuda_check(cudaMemcpyAsync(h_status_, dp_.status, 4, cudaMemcpyDeviceToHost, s_d2h_), "status D2H");
-            cuda_check(cudaMemsetAsync(dp_.status, 0, 4, s_d2h_), "status clear");
-            cuda_check(cudaEventRecord(ev_out_[oc], s_d2h_), "record");  // re-recorded: the host waits on it
+            cuda_check(cudaMemcpyAsync(h_status_, dp_.status, 4, cudaMemcpyDeviceToHost, d2h), "status D2H");
+            cuda_check(cudaMemsetAsync(dp_.status, 0, 4, d2h), "status clear");
+            cuda_check(cudaEventRecord(ev_out_[oc], d2h), "record");  // re-recorded: the host waits on it
         }
     };
     // Output chunks issued before the host waits on the first: all of them when nothing is

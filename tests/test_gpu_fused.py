@@ -364,3 +364,28 @@ def test_tables_of_the_fused_form(N, W):
     # 4 constant bytes x at most 256 rows x at most 256 K bytes for each operand, 256 x 512 for the CRT,
     # 15 twiddles, p and floor(2^48 / p) of up to 128 primes
     assert got[0]["table_bytes"] - got[1]["table_bytes"] <= 2 * 4 * 256 * 256 + 256 * 512 + 128 * (15 * 8 + 4)
+
+
+@pytest.mark.parametrize("N,W", [(512, 64), (4096, 256), (8192, 200), (8192, 250), (4096, 520)])
+def test_small_host_calls(N, W):
+    """Host calls around the size below which a call runs in one stream (operands of 256 KB), one after
+    another, from pageable and page-locked buffers and with one of the three page-locked."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    L = (W + 31) // 32
+    xs, ds = _operands(torch, N, W, 4, 11, 0)
+    want = torch.zeros((3, N, L), dtype=torch.int32, device="cuda")
+    pinned = [torch.from_numpy(x.view(np.int32).copy()).pin_memory().numpy().view(np.uint32) for x in xs]
+    with polymult.Multiplier(N, W, orc.limbs_of(_q(N, W), L)) as m:
+        for i in range(3):
+            m.multiply_device(ds[i].data_ptr(), ds[i + 1].data_ptr(), want[i].data_ptr(), 1,
+                              torch.cuda.current_stream().cuda_stream)
+        m.sync()
+        want = want.cpu().numpy().view(np.uint32)
+        for pa, pb, pc in [(0, 0, 0), (1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)]:
+            for i in range(3):
+                out = torch.zeros((N, L), dtype=torch.int32)
+                out = (out.pin_memory() if pc else out).numpy().view(np.uint32)
+                m.multiply((pinned if pa else xs)[i], (pinned if pb else xs)[i + 1], out=out)
+                assert np.array_equal(out, want[i]), (pa, pb, pc, i)
