@@ -50,8 +50,9 @@ def test_argument_check():
 
 
 def test_copy_tasks_cover_a_chunk_in_small_pieces(tmp_path):
-    """The tasks of a chunk's copy, whatever its rows: every word once, at least 64 KB and less than
-    twice a 64th of the chunk (or two rows' rounding) each, parts of a row on 32-byte boundaries."""
+    """The tasks of a chunk's copy, whatever its rows: every word once, at least 32 KB each and at most
+    128 KB or a 32nd of the chunk (a row more where a task has several), parts of a row on 32-byte
+    boundaries."""
     src = tmp_path / "tasks.cpp"
     src.write_text(r"""
 #include "pm_hostpool.h"
@@ -65,7 +66,7 @@ int main() {
             const pm::CopyTasks T(r, w);
             const size_t total = r * w;
             std::vector<unsigned char> seen(total, 0);
-            bool ok = T.count() >= 1 && T.count() <= 64;
+            bool ok = T.count() >= 1 && T.count() <= 128;
             for (uint32_t t = 0; t < T.count(); ++t) {
                 size_t got = 0;
                 T.each(t, [&](uint32_t row, size_t first, size_t n) {
@@ -73,15 +74,15 @@ int main() {
                     for (size_t k = 0; ok && k < n; ++k) ++seen[row * w + first + k];
                     got += n;
                 });
-                ok = ok && (got * 4 + 32 >= 65536 || T.count() == 1 || t + 1 == T.count());
+                ok = ok && (got * 4 + 32 >= 32768 || T.count() == 1 || t + 1 == T.count());
                 const size_t share = std::max<size_t>(total / 64, 16384);
-                ok = ok && got <= 2 * share + 2 * w * (T.parts == 1) + 8;
+                ok = ok && got <= 2 * share + (T.rows_per > 1 ? w : 8);
             }
             for (unsigned char x : seen) ok = ok && x == 1;
             if (!ok) return std::printf("rows %u words %zu: %u tasks\n", r, w, T.count()), 1;
         }
-    const pm::CopyTasks quarter(16, 56320);  // a quarter of 65536 coefficients of 55 words
-    return quarter.count() == 48 ? 0 : 2;
+    // quarters of 65536 coefficients of 55 words and of 32768 of 28
+    return pm::CopyTasks(16, 56320).count() == 48 && pm::CopyTasks(16, 14336).count() == 16 ? 0 : 2;
 }
 """)
     exe = str(tmp_path / "tasks")
