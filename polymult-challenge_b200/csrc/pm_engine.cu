@@ -1426,9 +1426,9 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
         cuda_check(cudaEventRecord(ev_out_[oc], d2h), "record");
         mark("d2h" + std::to_string(oc), d2h);
         if (oc + 1 == nout) {
-            // device status word -> pinned memory behind the last D2H (s_d2h has waited on every CRT)
+            // device status word -> pinned memory behind the last D2H (d2h has waited on every CRT); it is
+            // cleared only where a check has failed
             cuda_check(cudaMemcpyAsync(h_status_, dp_.status, 4, cudaMemcpyDeviceToHost, d2h), "status D2H");
-            cuda_check(cudaMemsetAsync(dp_.status, 0, 4, d2h), "status clear");
             cuda_check(cudaEventRecord(ev_out_[oc], d2h), "record");  // re-recorded: the host waits on it
         }
     };
@@ -1480,6 +1480,8 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     const uint32_t st = *h_status_;
     if (st) {
         *h_status_ = 0;
+        cuda_check(cudaMemsetAsync(dp_.status, 0, 4, d2h), "status clear");
+        cuda_check(cudaStreamSynchronize(d2h), "status clear");
         std::string what = "device-side check failed:";
         if (st & DEV_ERR_CRT_BOUND) what += " CRT estimate outside its exactness bound;";
         if (st & DEV_ERR_FOLD) what += " CRT value outside its bound after folding;";
