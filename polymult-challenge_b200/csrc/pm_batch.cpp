@@ -351,6 +351,9 @@ void Batch::alloc_scratch() {
     scratch_words_.assign(ns, 0);
     for (size_t s = 0; s < ns; ++s) {
         if (!need[s]) continue;
+        // both halves 256-byte aligned for every class of the stream: the largest may hold any number of
+        // words (N = 1), and another's kernels move up to 32 bytes at a time
+        need[s] = (need[s] + 63) / 64 * 64;
         cuda_check(cudaMalloc(&scratch_[s], 2 * need[s] * 4), "cudaMalloc batch scratch");
         scratch_words_[s] = need[s];
     }

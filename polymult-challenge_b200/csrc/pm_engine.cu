@@ -1259,9 +1259,9 @@ void Engine::run_host(const uint32_t* a, const uint32_t* b, uint32_t* c) {
     // A small call, one chunk each way, in one stream: both operands copied, then the three launches of
     // the device-resident call, then the result's copy.  There a's own kernels outlast b's copy, and each
     // hand-over between streams costs microseconds.  Medians in us, against a's decomposition and rows
-    // under b's copy: page-locked operands of 0.02 MB (2048 x 64 bits) 71.5 -> 56, 0.13 MB (4096 x 256)
-    // 73.6 -> 66.6, 0.23 MB (2048 x 868) 75.5 -> 74, 0.26 MB (4096 x 500) 75.6 -> 76 to 80; pageable
-    // 0.13 MB 83.7 -> 76.9, 0.23 MB 86 -> 81, 0.26 MB 84.1 -> 85.2 and (8192 x 256) 84.4 -> 97.
+    // under b's copy: page-locked operands of 0.02 MB (2048 x 64 bits) 60.3 -> 53, 0.13 MB (4096 x 256)
+    // 62.4 -> 58 to 62; pageable 0.02 MB 65.3 -> 55, 0.13 MB 74.3 -> 72, 0.23 MB (2048 x 868) 79.8 -> 76.7,
+    // 0.26 MB 79.7 -> 76.8 (4096 x 500) and 79.1 -> 79.4 (8192 x 256), 0.46 MB (4096 x 868) 89.5 -> 90.6.
     const bool small_call = pair && nin == 2 && nout == 1 && opbytes < (size_t)256 << 10;
     cudaStream_t h2d = small_call ? s_comp_[0] : s_h2d_, d2h = small_call ? s_comp_[0] : s_d2h_;
 

@@ -261,3 +261,21 @@ def test_a_requested_form_has_its_own_cache_entry(tmp_path, monkeypatch):
     with polymult.Batch([_spec(k)], tune=True) as b:
         ci = b.class_info(0)
         assert (ci["tuned_ms"], ci["w1"], ci["gemm"]) == (-1.0, 4, "tensor")
+
+
+@pytest.mark.parametrize("N0,W0,count0", [(1, 64, 3001), (2, 100, 1461), (4, 40, 1501)])
+def test_scratch_shared_with_a_class_of_any_word_count(N0, W0, count0):
+    """Nine classes on eight streams: the last shares its stream, and its second residue array begins
+    behind the largest class's, whose words are no multiple of what its kernels move at a time."""
+    torch = _torch()
+    import polymult
+    ensure_library()
+    points = [(512, 64, 8)] * 7 + [(N0, W0, count0), (512, 64, 1)]
+    ks = [_class(torch, N, W, c, seed=200 + i) for i, (N, W, c) in enumerate(points)]
+    want = [_single(torch, k) for k in ks]
+    with polymult.Batch([_spec(k) for k in ks]) as b:
+        assert b.info()["streams"] == 8
+        b.run(torch.cuda.current_stream().cuda_stream)
+        b.sync()
+    for k, w in zip(ks, want):
+        assert np.array_equal(k["c"].cpu().numpy().view(np.uint32), w), (k["N"], k["count"])

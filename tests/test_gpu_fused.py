@@ -152,7 +152,7 @@ def test_call_between_other_kernels_of_its_stream(N, W):
         assert torch.equal(g, w)
 
 
-@pytest.mark.parametrize("L0", [2, 10, 18, 26, 34, 42, 50])
+@pytest.mark.parametrize("L0", [1, 9, 17, 25, 33, 41, 49])
 def test_every_limb_count(L0):
     """The CRT's epilogue takes a coefficient's limbs in halves, pairs of four-limb steps, a step left
     over and up to three limbs behind it: every limb count of the fused form, so that each of these
