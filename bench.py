@@ -233,6 +233,9 @@ def pct(sorted_ms, p):
 # ------------------------------------------------------------------------------------------
 # CPU legs: the reference's own implementation (oracle/_ref), else the C restatement
 # ------------------------------------------------------------------------------------------
+REFERENCE_SO = os.path.join(ORACLE, "_ref", "libref_emu.so")
+
+
 class ReferenceCPU:
     """The reference's solve.cu in CPU-emulator form (oracle/_ref/libref_emu.so, its own
     fherma_run behind a C shim), else the C restatement of its RNS method."""
@@ -241,7 +244,7 @@ class ReferenceCPU:
         import numpy as np
         self.N, self.W, self.L = N, W, (W + 31) // 32
         self.qv = np.frombuffer(int(q).to_bytes(4 * self.L, "little"), dtype="<u4").copy()
-        so = os.path.join(ORACLE, "_ref", "libref_emu.so")
+        so = REFERENCE_SO
         self.err = ctypes.create_string_buffer(256)
         if os.path.exists(so):
             lib = ctypes.CDLL(so)
@@ -312,6 +315,10 @@ def reference_cpu(N, W, q, a, b, calls, warm):
 def run_reference(args):
     world, rank, _ = dist_init()
     if rank != 0:
+        return
+    if not os.path.exists(REFERENCE_SO):  # (the C restatement of its method is not the reference)
+        print(json.dumps({"impl": "reference", "unavailable": "the build of the reference's own sources is missing "
+                                                              "(oracle/_ref) and the sources are not here"}), flush=True)
         return
     import numpy as np
     import workload
