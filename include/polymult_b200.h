@@ -49,14 +49,16 @@ enum pm_gemm_form {
 typedef struct pm_info {
     uint32_t N, W, L;
     int32_t K;             /* RNS primes */
-    int32_t logN, w1, w2;  /* 4-step split: nrows = 2^w1, ncols = 2^w2 (w1 = 4 where the column stages run
-                              inside the GEMM kernels: tensor form, K <= 128, 2^9 <= N <= 2^16) */
+    int32_t logN, w1, w2;  /* 4-step split: nrows = 2^w1, ncols = 2^w2.  Where the column stages run inside the
+                              GEMM kernels (launches_per_multiply = 3) w1 = 4: tensor form, 2^9 <= N <= 2^16
+                              and both kernels' tables within shared memory, up to about 120 primes */
     int32_t gemm_form;     /* resolved form: PM_GEMM_PLAIN, PM_GEMM_TENSOR or PM_GEMM_MIXED */
     int32_t device;
     uint64_t delta;        /* 2^W - q */
     uint64_t table_bytes;  /* device memory of the per-point tables */
     uint64_t scratch_bytes;/* device memory of the residue scratch */
-    int32_t launches_per_multiply; /* kernels launched per device-resident multiply group */
+    int32_t launches_per_multiply; /* kernels launched per device-resident multiply group: 3 where the column
+                                      stages run inside the GEMM kernels, elsewhere more */
     int32_t group;         /* multiplies per launch group of pm_run_device (its scratch grows to this on use) */
 } pm_info;
 
@@ -76,7 +78,7 @@ int pm_run_device(pm_context* ctx, const uint32_t* d_a, const uint32_t* d_b, uin
                   void* stream);
 
 /* Kernels of one device-resident multiply group, in launch order (pm_time_stages).  Where the column
- * stages run inside the GEMM kernels (pm_info.w1 = 4), PM_STAGE_DEC_A is the one kernel that takes
+ * stages run inside the GEMM kernels (pm_info.launches_per_multiply = 3), PM_STAGE_DEC_A is the one kernel that takes
  * both operands through decomposition and column pass and PM_STAGE_CRT the inverse column pass and
  * CRT; PM_STAGE_COLS_A, _DEC_B, _COLS_B and _COLS_INV then read as the bare time between two event
  * records. */

@@ -17,9 +17,9 @@
 //
 // What bounds it: per tile and SM sub-partition the integer multiply-add pipe (236 butterflies and
 // 14 x 5 wide products per thread pair, ~3300 clocks at K = 118, L = 55) beside the HBM time of
-// the tile's bytes (~3800 clocks); producers and epilogue run on different tiles.  Measured: 10,900
-// clocks a tile, 19.8 us a multiply at N = 65536, W = 1747 in launches of 32 (an inverse column pass and
-// a CRT of their own: 26); the multiply-add pipe at 50%, issue slots at 53%.
+// the tile's bytes (~3800 clocks); producers and epilogue run on different tiles.  Measured: 11,000
+// clocks a tile, 20.0 us a multiply at N = 65536, W = 1747 in launches of 32 (an inverse column pass and
+// a CRT of their own: 26); the multiply-add pipe at 49%, issue slots at 51%.
 #include "pm_crt.cuh"
 #include "pm_ntt.cuh"
 #include "pm_tc.cuh"

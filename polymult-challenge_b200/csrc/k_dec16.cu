@@ -52,14 +52,13 @@ __device__ __forceinline__ uint32_t dec_reduce(uint32_t r0, uint32_t r1, uint32_
 //   warp 9 keeps a ring of raw pieces filled: the row segments of `npo` row octets of the super-tile
 //     (8 columns x L limbs each, contiguous in the operand), one bulk copy per row;
 //   warps 10-11 re-lay each piece out as the K-major operand, in one of `nb_buf` buffers.
-// The four hand work to one another through mbarriers only.  One thread doing all of it (and forming
-// every descriptor and address anew) took 19,000 clocks a tile at L = 55, K = 118, against the
-// epilogue's 5,500; the re-layout by branches 6,400 (its warps get the issue slots and the
-// instruction cache that the epilogue leaves); 4-byte cp.async straight into the operand 15,000.
-// Measured 25.5 us for both operands of a multiply at N = 65536, W = 1747 in launches of 32 (separate
+// The four hand work to one another through mbarriers only, and the helpers' roles are apart because
+// their warps get the issue slots and the instruction cache that the epilogue leaves.
+// Measured 25.8 us for both operands of a multiply at N = 65536, W = 1747 in launches of 32 (separate
 // decompositions and column passes: 48): the epilogue is the limit, two warps an SM sub-partition with
-// 224 registers, which cannot cover one another's waits (issue 51%, multiply-add pipe 57%).  Three
-// groups of 152 registers would store 16 bytes at a time: 44.5 us, half sectors do not merge in L2.
+// 224 registers, which cannot cover one another's waits (issue 51%, multiply-add pipe 56%).  It stays
+// at two groups because three, with 152 registers each, can hold half a row's 8 columns and would
+// store half sectors, which do not merge in L2: 44.5 us.
 // A CTA works for one operand (blockIdx.x mod nops), so that its constant image is loaded once and
 // both operands of a multiply share a launch.
 // Few primes (K <= 32 or 64): q = 4 or 2 tiles share an accumulator.  Lanes are split into q groups

@@ -28,18 +28,19 @@ namespace pm {
 // ----------------------------------------------------------------------------------------
 // Decomposition.  Persistent, warp-specialised, 640 threads; tiles of 128 positions over
 // (batch, npos).
-//   loader group (warps 0-7, two threads a tile row: with four warps and sixteen epilogue warps
-//     65536 x 4000 bits took 84.5 us an operand, now 81.6; with eight and sixteen 83.3): thread 0 keeps a ring of raw coefficient tiles filled by
-//     bulk copies (contiguous cnt*L words each, prefetched two tiles ahead); the group
-//     re-lays the tile out as the K-major A operand once the previous tile's MMAs have read
-//     A; warp 0 then issues the MMAs of the two prime halves -- half h once the epilogue
+//   loader group (warps 0-7, two threads a tile row): thread 0 keeps a ring of raw coefficient
+//     tiles filled by bulk copies (contiguous cnt*L words each, prefetched two tiles ahead); the
+//     group re-lays the tile out as the K-major A operand once the previous tile's MMAs have
+//     read A; warp 0 then issues the MMAs of the two prime halves -- half h once the epilogue
 //     has released TMEM half h -- with one commit per half (mma_done[h]);
 //   epilogue group (warps 8-19): warp w reads TMEM lane quarter w % 4, the 16-column chunks
 //     congruent to (w - 8) / 4 mod 3, of prime half 0 and then of half 1, and turns four byte
 //     columns into one sum, one REDC and a residue store; all 384 threads arrive on
 //     acc_empty[h] once they have read half h, so the next tile's half-0 MMA runs while they
 //     read half 1.
-// So tile i's epilogue (the long phase) overlaps tile i+1's copy, relayout and MMAs.  Bounded
+// So tile i's epilogue (the long phase) overlaps tile i+1's copy, relayout and MMAs.  Eight loader and
+// twelve epilogue warps share the SM best: 81.6 us an operand at 65536 x 4000 bits, against 84.5 with
+// four and sixteen and 83.3 with eight and sixteen.  Bounded
 // waits with a shared abort flag as in the CRT kernel.
 // smem: [B image][A tile][raw ring 2 x 128*L words][bars: B, raw 2, mma_done 2, acc_empty 2]
 //       [slot][abort][{p, p^-1 mod 2^32} x KP]

@@ -7,7 +7,7 @@
 // solve.cu:85-87, 917-918, 1403-1419).  Here a batch is a list of CLASSES -- one point and
 // `count` multiplications of it whose operands lie contiguously in device memory -- and:
 //   * every class runs as one launch per kernel covering all of its multiplications
-//     (grid.z / the persistent tile range spans the class's batch), so the 8 kernels of a
+//     (grid.z / the persistent tile range spans the class's batch), so the kernels of a
 //     class see count x the work of one multiply -- or as 2 or 4 such launch groups in a row
 //     where the tuner measured that faster;
 //   * classes are spread over a few streams (largest work first, each class to the stream
@@ -17,9 +17,9 @@
 //   * residue scratch is allocated once at init: per stream, the largest class on it (the
 //     classes of one stream run one after the other and reuse it).
 // The autotuner (PM_BATCH_TUNE) times, per class, the fused 16-row form (where it applies), every
-// split w1 in logN/2 - 1 .. logN/2 + 1 that the kernels support and both GEMM forms (where the tensor-core form fits) on the
-// class's own operands, CUDA events around 3 repetitions after a warm-up, and keeps the
-// fastest; then, on that engine, the column-pass kernel (TMA pipeline / one tile per CTA), the
+// split w1 in logN/2 - 1 .. logN/2 + 1 that the kernels support and both GEMM forms (where the
+// tensor-core form fits) on the class's own operands, CUDA events around 3 repetitions after a
+// warm-up, and keeps the fastest; then, on that engine, the column-pass kernel (TMA pipeline / one tile per CTA), the
 // CRT GEMM's A placement (tensor / shared memory) and 1, 2 or 4 launch groups per class.
 // Results are cached per (N, W, count, device, requested form) in a text file
 // ($POLYMULT_TUNE_CACHE, default ~/.cache/polymult_b200/tune.txt).

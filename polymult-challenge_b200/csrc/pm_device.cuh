@@ -76,12 +76,12 @@ struct CrtPrimeBlocks {
 
 // Pair layout of the residue arrays, used by the 16-row split: two primes share 128-byte lines,
 //   word (j, n) of a batch entry = (j / 2) 2N + (n / 16) 32 + (j % 2) 16 + n % 16,
-// room for the primes rounded up to an even number per entry.  A kernel that holds a prime per lane (8 columns of one row each)
-// touches 16 lines a warp store instead of 32; a row kernel, one prime a block, reads 32
-// elements from 2 lines instead of 1.  With four primes a line the two prime-per-lane kernels were
-// faster (65536 x 1747 bits x 32: decomposition 23.6 against 25.5 us a multiply, CRT 17.4 against
-// 19.8) and the row pass slower (52.1 against 48.8); in sum the pairs gain 1 to 2 % (95.0 -> 93.9;
-// 32768 x 868 bits x 16: 23.4 -> 22.8) except at few large multiplies (x 4: 391 against 398 us).
+// room for the primes rounded up to an even number per entry.  A kernel that holds a prime per lane
+// (8 columns of one row each) touches 16 lines a warp store instead of 32; a row kernel, one prime a
+// block, reads 32 elements from 2 lines instead of 1.  With four primes a line the two prime-per-lane
+// kernels are faster and the row pass slower; calls take, quads against pairs, us: 65536 x 1747 bits
+// x 1 109.6 / 109.1, x 32 3103 / 3038; 32768 x 868 x 1 39.0 / 38.4, x 16 373 / 370; 8192 x 1001 x 5
+// 52.3 / 51.7; 4096 x 256 x 64 86.4 / 85.1; quads also round the room up to four primes.
 __host__ __device__ constexpr int pair_primes(int K) { return (K + 1) & ~1; }
 // Word of (prime j, coefficient 0) of batch entry b, K2 = pair_primes(K):
 __device__ __forceinline__ size_t residue_base(uint32_t b, int K2, int j, size_t N) {

@@ -176,8 +176,8 @@ Engine::Engine(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int gemm_r
                                             std::to_string(prop.major * 10 + prop.minor));
     num_sms_ = prop.multiProcessorCount;
     smem_optin_ = prop.sharedMemPerBlockOptin;
-    // The 16-row split where both of its GEMM kernels take the point; else the square one.  Points
-    // of more than 128 primes keep the square split: a 4096-point row pass costs them more (92
+    // The 16-row split where both of its GEMM kernels take the point (about 120 primes); else the square
+    // one.  Points beyond keep the square split: a 4096-point row pass costs them more (92
     // against 55 us a multiply at N = 65536, W = 3000) than the decomposition in prime blocks saves
     // by taking the column pass along (137 against 139 us).
     const bool try16 = opt.w1 < 0 && (gemm_request == GEMM_AUTO || gemm_request == GEMM_TENSOR) && plan_.logN >= 9 &&

@@ -58,7 +58,8 @@ struct Chunk {
 struct EngineOptions {
     bool host_pipeline = true;  // pinned staging + streams for run_host (not needed by batches)
     // 4-step split nrows = 2^w1; -1: 16 rows with the column stages inside the GEMM kernels where
-    // those apply (tensor-core forms, at most 128 primes, 2^9 <= N <= 2^16), else logN / 2
+    // those apply (tensor-core forms, 2^9 <= N <= 2^16, both kernels' tables within shared memory: up to
+    // about 120 primes), else logN / 2
     int w1 = -1;
 };
 

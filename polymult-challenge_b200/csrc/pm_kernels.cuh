@@ -92,7 +92,8 @@ __global__ void k_crt_tm(DevPlan P, const uint32_t* R, ChunkMap C, uint32_t npos
 size_t crt_tm_smem(const DevPlan& P);
 
 // ---- GEMM kernels fused with the 16-row column pass (nrows = 16, ncols = N / 16)
-// Decomposition + forward column pass (k_dec16.cu): points of at most 128 primes.  A launch covers
+// Decomposition + forward column pass (k_dec16.cu): points of at most 128 primes (a TMEM lane each)
+// whose constant image leaves room for an operand tile and two raw pieces.  A launch covers
 // one or both operands of its multiplies.
 struct Dec16Args {
     const uint32_t* src[2];
@@ -118,7 +119,8 @@ constexpr int DEC16_MAX_RING = 8;
 size_t dec16_smem(const Dec16Args& A);
 void launch_dec16(const Dec16Args& A, uint32_t grid, size_t smem, cudaStream_t s, bool pdl);
 void dec16_set_smem_limit(int bytes);
-// Inverse column pass + CRT (k_crt16.cu): points of at most 128 primes.
+// Inverse column pass + CRT (k_crt16.cu): points whose operand tile, constants and result rows fit shared
+// memory, about 120 primes.
 struct Crt16Args {
     const uint32_t* R;
     uint32_t* out;

@@ -170,12 +170,6 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Arrives on `bar` once all of this thread's cp.async so far have landed (the barrier's count
-// includes it).
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // One thread: expect and issue a copy of `bytes` (multiple of 16) in pieces of <= 32 KB.
 __device__ __forceinline__ void bulk_g2s_all(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     mbar_arrive_expect_tx(bar, bytes);
