@@ -81,8 +81,9 @@ int main() {
             for (unsigned char x : seen) ok = ok && x == 1;
             if (!ok) return std::printf("rows %u words %zu: %u tasks\n", r, w, T.count()), 1;
         }
-    // quarters of 65536 coefficients of 55 words and of 32768 of 28
-    return pm::CopyTasks(16, 56320).count() == 48 && pm::CopyTasks(16, 14336).count() == 16 ? 0 : 2;
+    // quarters of 65536 coefficients of 55 words, of 32768 of 38 and of 28
+    return pm::CopyTasks(16, 56320).count() == 64 && pm::CopyTasks(16, 19456).count() == 32 &&
+                   pm::CopyTasks(16, 14336).count() == 16 ? 0 : 2;
 }
 """)
     exe = str(tmp_path / "tasks")
