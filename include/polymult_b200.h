@@ -297,7 +297,7 @@ uint64_t pm_digest_host(const uint32_t* words, uint64_t n);
  * failed device-side check would; the next pm_sync or pm_run then reports PM_ERR_DEVICE and
  * clears the word.  Waits for the context's device work first. */
 int pm_test_set_status(pm_context* ctx, uint32_t bits);
-#define PM_DEVICE_CRT_BOUND 1u /* fp32 CRT estimate not within 1/4 of an integer (|x| < M/8 violated) */
+#define PM_DEVICE_CRT_BOUND 1u /* CRT quotient estimate not within 1/4 of an integer (|x| < M/8 violated) */
 #define PM_DEVICE_FOLD 2u      /* CRT value above its bound after the folds */
 #define PM_DEVICE_WAIT 4u      /* an mbarrier wait of a tensor-core kernel ran out */
 

@@ -16,7 +16,7 @@ namespace pm {
 
 // Device status word bits (read back by the host after a run).
 enum : uint32_t {
-    DEV_ERR_CRT_BOUND = 1u,   // fp32 CRT estimate not within 1/4 of an integer (|x| < M/8 violated)
+    DEV_ERR_CRT_BOUND = 1u,   // CRT quotient estimate not within 1/4 of an integer (|x| < M/8 violated)
     DEV_ERR_FOLD = 2u,        // the CRT value had bits above 2^W after its folds (outside its bound)
     DEV_ERR_WAIT = 4u,        // an mbarrier wait hit its iteration limit
 };
