@@ -318,9 +318,10 @@ __device__ __forceinline__ void row_inverse(uint32_t (&v)[RowCfg<NB>::E], uint32
 // fused form (host pipeline, server) keeps a 4-byte stack slot at 7 (8 bytes at 6).
 enum : int { ROWS_FWD = 0, ROWS_FUSED = 1, ROWS_BOTH = 2 };
 __host__ __device__ constexpr int rows_min_blocks(int nb, int mode) {
-    if (nb == 12) return 3;                      // 256 threads, 80 registers (4 at 64: 52.7 -> 54.5 us at N = 65536, W = 1747)
-    if (nb == 11) return 7;                      // 72 registers (12.1 -> 11.6 us at N = 32768, W = 868)
-    if (nb == 10) return 6;                      // 80 registers (7 spill: 13.3 -> 14.2 us at N = 16384, W = 1747)
+    if (nb == 12) return 3;                      // 256 threads, 80 registers (4 at 64, 65536 x 1747 bits: alone 58.0 -> 59.6
+                                                 // us, in launches of 32 46.8 -> 46.4, the calls the same)
+    if (nb == 11) return 7;                      // 72 registers (6 at 80: 11.0 -> 11.6 us at N = 32768, W = 868)
+    if (nb == 10) return 6;                      // 80 registers (7 spill: 12.1 -> 13.0 us at N = 16384, W = 1747)
     return nb >= 9 ? (mode == ROWS_FWD ? 5 : 4) : (mode == ROWS_FWD ? 8 : 7);
 }
 // POLYMULT_ROW_STATIC: the row kernels take the column-stage count w1 (and with it nrows and N)
